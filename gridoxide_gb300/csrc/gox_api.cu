@@ -23,8 +23,10 @@
 
 #include "../../include/gridoxide_gb300.h"
 #include "gox_engine.hpp"
+#include "gox_dot.hpp"
 #include "gox_stream.hpp"
 #include "gox_kernels.cuh"
+#include "gox_dot.cuh"
 #include "gox_pivot.cuh"
 
 namespace gox {
@@ -314,8 +316,45 @@ struct DevSchedule {
   int st_wl[2] = {0, 0}, st_wp[2] = {0, 0};  // levels / phases the wide kernels run
   int st_wr[2] = {0, 0};                      // their stage rows per warp
   std::vector<int32_t> lev_ptr_h;  // host copy: columns per refactor level
-  // launches of one refactor (with both substitutions when the stream has them)
-  int refactor_launches(int i) const { return 1 + st_wl[i] + st_wp[i]; }
+  // a dot-product program in place of the streams, per precision (on: used)
+  struct DotPlanDev {
+    bool on = false, with_subst = false;
+    int top_warps = 0, bins = 0;
+    DevMem words, bottom, prep, top, back;
+    DotDev d{};
+  } dot[2];
+  // the plan's substitutions are part of its refactor
+  bool has_bwd(int i) const { return dot[i].on ? dot[i].with_subst : st_bwd[i]; }
+  // launches of one refactor (with both substitutions when the plan has them)
+  int refactor_launches(int i) const {
+    if (dot[i].on)
+      return 1 + (dot[i].d.n_bottom > 0) + (dot[i].d.n_prep > 0) + (dot[i].d.n_back > 0);
+    return 1 + st_wl[i] + st_wp[i];
+  }
+
+  // (null: the streams)
+  void load_dot(int i, const DotProgram* p) {
+    DotPlanDev& x = dot[i];
+    x.on = p != nullptr;
+    if (!p) return;
+    x.with_subst = p->with_subst;
+    x.top_warps = (int)p->top.size();
+    x.bins = p->plan.bins;
+    upload(x.words, p->words);
+    upload(x.bottom, p->bottom);
+    upload(x.prep, p->prep);
+    upload(x.top, p->top);
+    upload(x.back, p->back);
+    x.d.words = x.words.as<uint4>();
+    x.d.bottom = x.bottom.as<int32_t>();
+    x.d.prep = x.prep.as<int32_t>();
+    x.d.top = x.top.as<int32_t>();
+    x.d.back = x.back.as<int32_t>();
+    x.d.n_bottom = (int)p->bottom.size();
+    x.d.n_prep = (int)p->prep.size();
+    x.d.n_top = (int)p->top.size();
+    x.d.n_back = (int)p->back.size();
+  }
 
   void load_streams(const Stream& s32, const Stream& s64) {
     const Stream* ss[2] = {&s32, &s64};
@@ -548,6 +587,18 @@ static void make_streams(const Schedule& sc, Stream& s32, Stream& s64) {
   }
 }
 
+// A program through the checking host interpreter, as every stream: indices,
+// order of each sum, no value read before it is final.
+static std::shared_ptr<const DotProgram> make_dot(const Schedule& sc, const DotPlan& plan) {
+  auto p = std::make_shared<DotProgram>();
+  build_dot(sc, plan, *p);
+  std::vector<double> lu(sc.n_slots, 1.0), rhs(sc.n_u, 0.0), X;
+  bool sing = false;
+  const std::string e = run_dot_host(sc, *p, lu, rhs, X, sing);
+  if (!e.empty()) throw std::runtime_error("dot program check: " + e);
+  return p;
+}
+
 struct Timing {
   bool on = false;
   double iters = 0, total = 0, k1 = 0, k2 = 0, k3 = 0, k4 = 0;
@@ -586,6 +637,10 @@ struct Iter {
   }
   static void refactor(const DevSchedule& ds, const BatchDev& D, cudaStream_t st) {
     const int i = sizeof(T) == 4 ? 0 : 1;
+    if (ds.dot[i].on) {
+      dot(ds.dot[i].d, ds.d, D, D.G, st);
+      return;
+    }
     refactor_with(ds, ds.st[i], ds.st_nw[i], ds.st_smem[i], ds.st_wl[i], ds.st_wp[i], ds.st_wr[i], D,
                   D.G, st);
   }
@@ -608,6 +663,37 @@ struct Iter {
       wide_attr();
       k_refactor_wide<T><<<blocks, 32 * kWideWarps, wide_smem(wr), st>>>(ds.d, D, L, groups, wr);
     }
+  }
+  // The dot kernels keep 20 % of the SM's 228 KB as shared memory (their
+  // windows need 8 to 48 KB per SM): the L1 is where the values of earlier
+  // sums are found again.  Measured on the 2,000-bus grid, 128 groups FP32 /
+  // 47 groups FP64, ms per refactor: the driver's own choice 1.77 / 2.35, 15-25 %
+  // 1.71 / 2.29, 50 % 1.77 / 2.36, 10 % (fewer CTAs fit) 2.33 / 2.37.
+  static void dot_attr() {
+    static std::once_flag once[64];
+    int dev = 0;
+    GOX_CK(cudaGetDevice(&dev));
+    std::call_once(once[dev & 63], [] {
+      const cudaFuncAttribute a = cudaFuncAttributePreferredSharedMemoryCarveout;
+      GOX_CK(cudaFuncSetAttribute(k_dot_bins<T>, a, 20));
+      GOX_CK(cudaFuncSetAttribute(k_dot_top<T, 16>, a, 20));
+      if constexpr (sizeof(T) == 4) GOX_CK(cudaFuncSetAttribute(k_dot_top<T, 32>, a, 20));
+    });
+  }
+  static void dot_bins(const DotDev& P, const SchedDev& S, const BatchDev& D, int which, int n, int groups,
+                       cudaStream_t st) {
+    if (n == 0) return;
+    k_dot_bins<T><<<dim3((n + kDotBinWarps - 1) / kDotBinWarps, groups), 32 * kDotBinWarps, 0, st>>>(P, S, D, which);
+  }
+  static void dot(const DotDev& P, const SchedDev& S, const BatchDev& D, int groups, cudaStream_t st) {
+    dot_attr();
+    dot_bins(P, S, D, DOT_BOTTOM, P.n_bottom, groups, st);
+    dot_bins(P, S, D, DOT_PREP, P.n_prep, groups, st);
+    if constexpr (sizeof(T) == 4) {
+      if (P.n_top == 32) k_dot_top<T, 32><<<groups, 1024, 0, st>>>(P, S, D);
+    }
+    if (P.n_top == 16) k_dot_top<T, 16><<<groups, 512, 0, st>>>(P, S, D);
+    dot_bins(P, S, D, DOT_BACK, P.n_back, groups, st);
   }
   // shared memory of a wide-kernel CTA whose warps stage `rows` rows
   static size_t wide_smem(int rows) { return (size_t)kWideWarps * rows * 32 * sizeof(T); }
@@ -649,7 +735,7 @@ struct Iter {
   // the substitutions the refactor's stream did not run (none when it ran
   // the backward substitution too); returns the launches
   static int solve_rest(const DevSchedule& ds, const BatchDev& D, cudaStream_t st) {
-    if (ds.st_bwd[sizeof(T) == 4 ? 0 : 1]) return 0;
+    if (ds.has_bwd(sizeof(T) == 4 ? 0 : 1)) return 0;
     solve(ds.d, D, st);
     return 1;
   }
@@ -732,6 +818,8 @@ struct gox_topo {
   Numeric num;
   Schedule sc;
   Stream s32, s64;
+  // the dot program used in place of the streams, per precision (null: the streams)
+  std::shared_ptr<const DotProgram> dot[2];
   DevSchedule dsched;
   DevBatch batch;
   // re-packing: the smaller batch the running scenarios move to, and their
@@ -927,6 +1015,8 @@ static int fix_pivots(gox_topo* t, int B, const double* p_spec, const double* q_
       t->num = std::move(N);
       build_schedule(&t->jac, t->csc, t->sym, t->num, t->sc);
       make_streams(t->sc, t->s32, t->s64);
+      t->dot[0].reset();
+      t->dot[1].reset();
       t->factored = true;
       t->uploaded = false;
       (void)nu;
@@ -935,6 +1025,14 @@ static int fix_pivots(gox_topo* t, int B, const double* p_spec, const double* q_
     first_singular.push_back(s);
   }
   return -1;
+}
+
+// The schedule and the refactor plans to the device
+static void upload_plans(gox_topo* t) {
+  t->dsched.load(t->sc, t->yp, t->yi, t->yre, t->yim);
+  t->dsched.load_streams(t->s32, t->s64);
+  for (int i = 0; i < 2; i++) t->dsched.load_dot(i, t->dot[i].get());
+  t->uploaded = true;
 }
 
 static constexpr int kGraphMinGroups = 64;  // batches of >= 2,048 scenarios
@@ -1031,6 +1129,7 @@ static std::vector<unsigned char> loop_key(const gox_topo* t, const BatchDev& D,
   put(&t->dsched.st_smem[i], sizeof(size_t)); put(&t->dsched.st_bwd[i], sizeof(bool));
   put(&t->dsched.st_wl[i], sizeof(int)); put(&t->dsched.st_wp[i], sizeof(int));
   put(&t->dsched.st_wr[i], sizeof(int));
+  put(&t->dsched.dot[i].on, sizeof(bool)); put(&t->dsched.dot[i].d, sizeof(DotDev));
   return key;
 }
 
@@ -1183,13 +1282,16 @@ static void tune_cache_load() {
   std::fclose(f);
 }
 
-static void tune_cache_store(const std::array<int, 4>& k, const StreamPlan& p) {
-  const int nw = p.nw, cw = p.chunk_words, sy = p.sync, wd = p.wide_levels > 0 ? p.wide_min : 0;
-  g_tune[k] = {nw, cw, sy, wd};
+// A dot program's entry: its top's warps, the words of its streams' chunks
+// (no stream plan has chunks that short), 0, its bins.
+static constexpr int kDotChunkWords = 4 * kDotChunk;
+
+static void tune_cache_store(const std::array<int, 4>& k, const std::array<int, 4>& v) {
+  g_tune[k] = v;
   const char* path = std::getenv("GOX_TUNE_CACHE");
   if (!path || !*path) return;
   if (FILE* f = std::fopen(path, "a")) {
-    std::fprintf(f, "gox-tune-3 %d %d %d %d %d %d %d %d\n", k[0], k[1], k[2], k[3], nw, cw, sy, wd);
+    std::fprintf(f, "gox-tune-3 %d %d %d %d %d %d %d %d\n", k[0], k[1], k[2], k[3], v[0], v[1], v[2], v[3]);
     std::fclose(f);
   }
 }
@@ -1221,7 +1323,16 @@ static void drop_loops(gox_topo* t, int i) {
   t->loop_graphs = std::move(keep);
 }
 
+static void install_dot(gox_topo* t, int i, std::shared_ptr<const DotProgram> p) {
+  for (gox_topo* x = t; x; x = x->twin.get()) {  // and the split solves' twins
+    x->dot[i] = p;
+    if (x->uploaded) x->dsched.load_dot(i, p.get());
+    drop_loops(x, i);
+  }
+}
+
 static void install_stream(gox_topo* t, int i, Stream&& s) {
+  install_dot(t, i, nullptr);
   (i == 0 ? t->s32 : t->s64) = std::move(s);
   t->dsched.load_streams(t->s32, t->s64);
   drop_loops(t, i);
@@ -1247,8 +1358,20 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st) {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     tune_cache_load();
     auto it = g_tune.find(key);
-    if (it == g_tune.end() && t->tune_cache_only) return;
-    if (it != g_tune.end()) {
+    if (it == g_tune.end() && t->tune_cache_only) {
+      // not timed: the program the measured rule gives
+      install_dot(t, i, make_dot(sc, dot_default(sc, elem, D.G)));
+      return;
+    }
+    if (it != g_tune.end() && it->second[1] == kDotChunkWords) {
+      for (const DotPlan& p : dot_candidates(sc, elem))
+        if (p.top_warps == it->second[0] && p.bins == it->second[3]) {
+          install_dot(t, i, make_dot(sc, p));
+          TU.source = 2;
+          return;
+        }
+      if (t->tune_cache_only) return;
+    } else if (it != g_tune.end()) {
       const Stream& cur = i == 0 ? t->s32 : t->s64;
       auto same = [&](const StreamPlan& p) {
         return p.nw == it->second[0] && p.chunk_words == it->second[1] && p.sync == it->second[2] &&
@@ -1278,13 +1401,24 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st) {
   std::vector<StreamPlan> cand = candidate_plans(sc, elem, kRefactorSmem);
   std::vector<Stream> built(cand.size());
   std::vector<char> ok(cand.size(), 0);
+  const std::vector<DotPlan> dcand = dot_candidates(sc, elem);
+  std::vector<std::shared_ptr<const DotProgram>> dbuilt(dcand.size());
   {
     std::vector<std::thread> th;
     std::atomic<size_t> next{0};
     const unsigned nt = std::max(1u, std::min(8u, std::thread::hardware_concurrency()));
     for (unsigned w = 0; w < nt; w++)
       th.emplace_back([&] {
-        for (size_t c; (c = next++) < cand.size();) ok[c] = compile_checked(sc, cand[c], built[c]);
+        for (size_t c; (c = next++) < cand.size() + dcand.size();) {
+          if (c < cand.size()) {
+            ok[c] = compile_checked(sc, cand[c], built[c]);
+          } else {
+            try {
+              dbuilt[c - cand.size()] = make_dot(sc, dcand[c - cand.size()]);
+            } catch (const std::exception&) {  // not a candidate
+            }
+          }
+        }
       });
     for (auto& x : th) x.join();
   }
@@ -1299,7 +1433,44 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st) {
   double best_ms = 1e30;
   int best = -1;
   TU.table.clear();
-  for (size_t c = 0; c < cand.size(); c++) {
+  // two runs of `launch` on the image; the second one's time, or a negative
+  // number when a bounded wait gave up
+  auto time_plan = [&](auto&& launch) -> float {
+    float ms = 0.0f;
+    for (int rep = 0; rep < 2; rep++) {
+      GOX_CK(cudaMemcpyAsync(D.lu, bak.p, img_bytes, cudaMemcpyDeviceToDevice, st));
+      GOX_CK(cudaEventRecord(e0, st));
+      launch();
+      GOX_CK(cudaEventRecord(e1, st));
+      GOX_CK(cudaEventSynchronize(e1));
+      GOX_CK(cudaEventElapsedTime(&ms, e0, e1));
+    }
+    GOX_CK(cudaGetLastError());
+    int32_t herr[2] = {0, 0};
+    GOX_CK(cudaMemcpyAsync(herr, D.err - 1, 8, cudaMemcpyDeviceToHost, st));
+    GOX_CK(cudaStreamSynchronize(st));
+    if (!herr[1]) return ms;
+    const int32_t z[2] = {0, 0};
+    GOX_CK(cudaMemcpyAsync(D.err - 1, z, 8, cudaMemcpyHostToDevice, st));
+    return -1.0f;
+  };
+  for (size_t c = 0; c < cand.size() + dcand.size(); c++) {
+    if (c >= cand.size()) {
+      const DotProgram* p = dbuilt[c - cand.size()].get();
+      if (!p) continue;
+      DevSchedule::DotPlanDev& x = t->dsched.dot[i];
+      t->dsched.load_dot(i, p);
+      x.on = false;  // until one is installed
+      const float ms = time_plan([&] { Iter<T>::dot(x.d, t->dsched.d, D, Gt, st); });
+      if (ms < 0.0f) continue;
+      TU.table.push_back({(double)p->plan.top_warps, (double)kDotChunkWords, 0.0, (double)ms, 0.0,
+                          (double)p->plan.bins, (double)p->plan.bins});
+      if (ms < best_ms) {
+        best_ms = ms;
+        best = (int)c;
+      }
+      continue;
+    }
     if (!ok[c]) continue;
     const Stream& s = built[c];
     upload(words, s.words);
@@ -1314,25 +1485,11 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st) {
     P.chunk_words = s.plan.chunk_words;
     P.n_bars = s.n_bars;
     P.sync = s.plan.sync;
-    float ms = 0.0f;
-    for (int rep = 0; rep < 2; rep++) {
-      GOX_CK(cudaMemcpyAsync(D.lu, bak.p, img_bytes, cudaMemcpyDeviceToDevice, st));
-      GOX_CK(cudaEventRecord(e0, st));
+    const float ms = time_plan([&] {
       Iter<T>::refactor_with(t->dsched, P, s.plan.nw, stream_smem_bytes(s.plan), s.plan.wide_levels,
                              s.plan.wide_phases, s.plan.wide_rows, D, Gt, st);
-      GOX_CK(cudaEventRecord(e1, st));
-      GOX_CK(cudaEventSynchronize(e1));
-      GOX_CK(cudaEventElapsedTime(&ms, e0, e1));
-    }
-    GOX_CK(cudaGetLastError());
-    int32_t herr[2] = {0, 0};
-    GOX_CK(cudaMemcpyAsync(herr, D.err - 1, 8, cudaMemcpyDeviceToHost, st));
-    GOX_CK(cudaStreamSynchronize(st));
-    if (herr[1]) {  // a bounded wait gave up under this plan: not a candidate
-      const int32_t z[2] = {0, 0};
-      GOX_CK(cudaMemcpyAsync(D.err - 1, z, 8, cudaMemcpyHostToDevice, st));
-      continue;
-    }
+    });
+    if (ms < 0.0f) continue;  // a bounded wait gave up under this plan: not a candidate
     TU.table.push_back({(double)s.plan.nw, (double)s.plan.chunk_words, (double)s.plan.ring_rows,
                         (double)ms, (double)s.plan.sync, (double)s.plan.wide_levels,
                         (double)s.plan.wide_phases});
@@ -1347,11 +1504,19 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st) {
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (best < 0) return;
-  const StreamPlan bestp = cand[best];
-  install_stream(t, i, std::move(built[best]));
+  std::array<int, 4> entry;
+  if (best >= (int)cand.size()) {
+    const std::shared_ptr<const DotProgram> p = dbuilt[best - (int)cand.size()];
+    entry = {p->plan.top_warps, kDotChunkWords, 0, p->plan.bins};
+    install_dot(t, i, p);
+  } else {
+    const StreamPlan& p = cand[best];
+    entry = {p.nw, p.chunk_words, p.sync, p.wide_levels > 0 ? p.wide_min : 0};
+    install_stream(t, i, std::move(built[best]));
+  }
   TU.source = 1;
   std::lock_guard<std::mutex> lk(g_tune_mu);
-  tune_cache_store(key, bestp);
+  tune_cache_store(key, entry);
 }
 
 // Re-packing of the running scenarios (host-driven loop).  After an
@@ -1470,7 +1635,7 @@ static void run_iterations(gox_topo* t, BatchDev D, int max_iter, bool outage, c
     GOX_CK(cudaStreamSynchronize(st));
     const int its = h[1], ran_out = (h[0] > 0 && its >= max_iter) ? 1 : 0;
     const int fills = h[0] > 0 ? its : its - 1;
-    const int ns = t->dsched.st_bwd[sizeof(T) == 4 ? 0 : 1] ? 0 : 1;
+    const int ns = t->dsched.has_bwd(sizeof(T) == 4 ? 0 : 1) ? 0 : 1;
     const int nr = t->dsched.refactor_launches(sizeof(T) == 4 ? 0 : 1);
     t->launches += (int64_t)its * 4 + (int64_t)fills * (1 + nr + ns) + ran_out * 2;
     return;
@@ -1638,6 +1803,7 @@ static void guess_build(gox_topo* t, const double* p0, const double* q0) {
   std::vector<double> dummy_x;
   G.dsched.load(G.sc, dummy_p, dummy_i, dummy_x, dummy_x);
   G.dsched.load_streams(G.s32, G.s64);
+  G.dsched.load_dot(1, make_dot(G.sc, dot_default(G.sc, 8, 128)).get());
   // value recipe per LU slot, then per off-diagonal entry
   const int ns = G.sc.n_slots, no = G.sc.n_off;
   std::vector<int32_t> rec((size_t)(ns + no) * 4);
@@ -1872,9 +2038,7 @@ static int batch_prepare(gox_topo* t, int B, const double* p_spec, const double*
   const bool outage = o_slot != nullptr;
   const bool want_hist = hist != nullptr;
   if (!t->uploaded) {
-    t->dsched.load(t->sc, t->yp, t->yi, t->yre, t->yim);
-    t->dsched.load_streams(t->s32, t->s64);
-    t->uploaded = true;
+    upload_plans(t);
   }
   const SchedDev& S = t->dsched.d;
   DevBatch& DB = t->batch;
@@ -2084,6 +2248,7 @@ struct MultiLists {
   struct L { size_t off = 0, job = 0; int n = 0, ctas = 0; };
   L upd, inj, dec, fill, rf;
   std::vector<L> wide;  // per wide level
+  L dbins[3], dtop[2];  // dot programs: bottom, prep, back; the top with 16 and 32 warps
   MultiList view(const L& l) const {
     MultiList m;
     m.off = dev.as<int32_t>() + l.off;
@@ -2124,14 +2289,34 @@ static void build_lists(const std::vector<gox_topo*>& ts, const std::vector<Batc
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
     return (i == 0 ? ts[a]->s32 : ts[a]->s64).est_cycles > (i == 0 ? ts[b]->s32 : ts[b]->s64).est_cycles;
   });
-  M.rf = add(order, [&](int j) { return G(j); });
+  // jobs whose plan is a dot program: a list per launch, the top's by its warps
+  // (longest first too); the others run their streams
+  std::vector<int> dots, streams, top[2];
+  for (int j : order) {
+    const auto& x = ts[j]->dsched.dot[i];
+    (x.on ? dots : streams).push_back(j);
+    if (x.on) top[x.top_warps == 32].push_back(j);
+  }
+  for (int w = 0; w < 2; w++) M.dtop[w] = add(top[w], [&](int j) { return G(j); });
+  for (int w : {DOT_BOTTOM, DOT_PREP, DOT_BACK}) {
+    auto n = [&](int j) {
+      const DotDev& d = ts[j]->dsched.dot[i].d;
+      return w == DOT_BOTTOM ? d.n_bottom : w == DOT_PREP ? d.n_prep : d.n_back;
+    };
+    std::vector<int> jl;
+    for (int j : dots)
+      if (n(j) > 0) jl.push_back(j);
+    M.dbins[w] = add(jl, [&](int j) { return dot_blocks(n(j)) * G(j); });
+  }
+  M.rf = add(streams, [&](int j) { return G(j); });
+  auto levels = [&](int j) { return ts[j]->dsched.dot[i].on ? 0 : ts[j]->dsched.st_wl[i]; };
   int maxl = 0;
-  for (int j : act) maxl = std::max(maxl, ts[j]->dsched.st_wl[i]);
+  for (int j : act) maxl = std::max(maxl, levels(j));
   M.wide.clear();
   for (int L = 0; L < maxl; L++) {
     std::vector<int> jl;
     for (int j : act)
-      if (ts[j]->dsched.st_wl[i] > L) jl.push_back(j);
+      if (levels(j) > L) jl.push_back(j);
     M.wide.push_back(add(jl, [&](int j) {
       const std::vector<int32_t>& lp = ts[j]->dsched.lev_ptr_h;
       const long long tasks = (long long)(lp[L + 1] - lp[L]) * G(j);
@@ -2152,6 +2337,7 @@ static void upload_jobs(const std::vector<gox_topo*>& ts, const std::vector<Batc
     jobs[j].S = ts[j]->dsched.d;
     jobs[j].D = runs[j].D;
     jobs[j].P = ts[j]->dsched.st[i];
+    jobs[j].dot = ts[j]->dsched.dot[i].d;
     jobs[j].nw = ts[j]->dsched.st_nw[i];
   }
   dev.ensure(jobs.size() * sizeof(MultiJob));
@@ -2179,6 +2365,7 @@ static void run_multi(const std::vector<gox_topo*>& ts, std::vector<BatchRun>& r
     nw_max = 1;
     smem_max = 0;
     for (gox_topo* t : ts) {
+      if (t->dsched.dot[i].on) continue;
       nw_max = std::max(nw_max, t->dsched.st_nw[i]);
       smem_max = std::max(smem_max, t->dsched.st_smem[i]);
     }
@@ -2194,6 +2381,10 @@ static void run_multi(const std::vector<gox_topo*>& ts, std::vector<BatchRun>& r
       GOX_CK(cudaFuncSetAttribute(k_refactor_wide_multi<T>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)Iter<T>::kWideSmem));
+      const cudaFuncAttribute a = cudaFuncAttributePreferredSharedMemoryCarveout;  // as the single kernels
+      GOX_CK(cudaFuncSetAttribute(k_dot_bins_multi<T>, a, 20));
+      GOX_CK(cudaFuncSetAttribute(k_dot_top_multi<T, 16>, a, 20));
+      if constexpr (sizeof(T) == 4) GOX_CK(cudaFuncSetAttribute(k_dot_top_multi<T, 32>, a, 20));
     });
   }
   const MultiJob* J = nullptr;
@@ -2268,6 +2459,17 @@ static void run_multi(const std::vector<gox_topo*>& ts, std::vector<BatchRun>& r
     launch(M.rf, [&](unsigned c, MultiList l) {
       k_refactor_multi<T><<<c, 32 * nw_max, smem_max, st>>>(J, l);
     });
+    auto bins = [&](int w) {
+      launch(M.dbins[w], [&](unsigned c, MultiList l) {
+        k_dot_bins_multi<T><<<c, 32 * kDotBinWarps, 0, st>>>(J, l, w);
+      });
+    };
+    bins(DOT_BOTTOM);
+    bins(DOT_PREP);
+    if constexpr (sizeof(T) == 4)
+      launch(M.dtop[1], [&](unsigned c, MultiList l) { k_dot_top_multi<T, 32><<<c, 1024, 0, st>>>(J, l); });
+    launch(M.dtop[0], [&](unsigned c, MultiList l) { k_dot_top_multi<T, 16><<<c, 512, 0, st>>>(J, l); });
+    bins(DOT_BACK);
     rec();
     for (size_t L = M.wide.size(); L-- > 0;)
       launch(M.wide[L], [&](unsigned c, MultiList l) {
@@ -2726,6 +2928,7 @@ static std::unique_ptr<gox_topo> clone_factored(const gox_topo* t) {
   v->yp = t->yp; v->yi = t->yi; v->yre = t->yre; v->yim = t->yim; v->bus_type = t->bus_type;
   v->jac = t->jac; v->csc = t->csc; v->sym = t->sym; v->num = t->num; v->sc = t->sc;
   v->s32 = t->s32; v->s64 = t->s64;
+  v->dot[0] = t->dot[0]; v->dot[1] = t->dot[1];
   v->factored = true;
   v->uploaded = false;
   v->device = t->device;
@@ -2955,6 +3158,8 @@ int gox_topo_reset(gox_topo* t) {
   t->uploaded = false;
   t->num = Numeric();
   t->sc = Schedule();
+  t->dot[0].reset();
+  t->dot[1].reset();
   t->tune[0] = gox_topo::Tuning();
   t->tune[1] = gox_topo::Tuning();
   return GOX_OK;
@@ -3512,6 +3717,22 @@ int gox_topo_emulate_step(const gox_topo* t, const double* jac_vals, const doubl
     for (int x = 0; x < sc.n_slots; x++)
       if (!(lu[x] == lu64[x]) && !(std::isnan(lu[x]) && std::isnan(lu64[x])))
         throw std::runtime_error("the two refactor streams disagree");
+    // ... and the dot programs of both precisions, the same factor again
+    for (int elem : {4, 8}) {
+      DotProgram p;
+      build_dot(sc, dot_default(sc, elem, 1), p);
+      std::vector<double> lud(sc.n_slots, 0.0), Xd;
+      for (int x = 0; x < sc.n_slots; x++)
+        lud[x] = sc.slot_a[x] >= 0 ? packed[sc.a_csc[sc.slot_a[x]]] : 0.0;
+      bool singd = false;
+      const std::string ed = run_dot_host(sc, p, lud, b, Xd, singd);
+      if (!ed.empty()) throw std::runtime_error("dot program: " + ed);
+      auto differ = [](double x, double y) { return !(x == y) && !(std::isnan(x) && std::isnan(y)); };
+      for (int x = 0; x < sc.n_slots; x++)
+        if (differ(lu[x], lud[x])) throw std::runtime_error("the dot program's factor differs from the streams'");
+      for (int x = 0; x < n && t->s32.has_bwd && p.with_subst; x++)
+        if (differ(X[x], Xd[x])) throw std::runtime_error("the dot program's solution differs from the streams'");
+    }
     bad = sing32;
     if (t->s32.has_bwd != t->s64.has_bwd) throw std::runtime_error("stream plans disagree");
     for (int x = 0; x < n && t->s32.has_bwd; x++)
@@ -3605,9 +3826,7 @@ int gox_topo_factor_values(gox_topo* t, int32_t B, const double* p_spec, const d
     AllocStreamScope alloc_scope(st);
     const int n = t->n_bus, G = (B + 31) / 32;
     if (!t->uploaded) {
-      t->dsched.load(t->sc, t->yp, t->yi, t->yre, t->yim);
-      t->dsched.load_streams(t->s32, t->s64);
-      t->uploaded = true;
+      upload_plans(t);
     }
     t->dsched.d.zip = t->zip.empty() ? nullptr : t->dzip.as<double>();
     const SchedDev& S = t->dsched.d;
@@ -3649,9 +3868,7 @@ int gox_topo_pivot_solve(gox_topo* t, const double* jac_vals, const double* rhs,
     const Schedule& sc = t->sc;
     const int n = sc.n_u;
     if (!t->uploaded) {
-      t->dsched.load(t->sc, t->yp, t->yi, t->yre, t->yim);
-      t->dsched.load_streams(t->s32, t->s64);
-      t->uploaded = true;
+      upload_plans(t);
     }
     const SchedDev& S = t->dsched.d;
     DevBatch& DB = t->batch;
@@ -3745,6 +3962,13 @@ int gox_topo_tuning(const gox_topo* t, int32_t precision, int64_t* plan, double*
   plan[6] = s.plan.sync;
   plan[7] = s.plan.wide_levels;
   plan[8] = s.plan.wide_phases;
+  if (const DotProgram* p = t->dot[i].get()) {
+    plan[0] = p->plan.top_warps;
+    plan[1] = plan[2] = 0;
+    plan[3] = kDotChunkWords;
+    plan[6] = 0;
+    plan[7] = plan[8] = p->plan.bins;
+  }
   int rows = 0;
   for (const auto& r : TU.table) {
     if (!table || rows >= max_rows) break;
@@ -3949,6 +4173,7 @@ int gox_ls_create(int32_t n, int32_t nnz, const int32_t* rows, const int32_t* co
     std::vector<double> dummy_x;
     h->dsched.load(h->sc, dummy_p, dummy_i, dummy_x, dummy_x);
     h->dsched.load_streams(h->s32, h->s64);
+    h->dsched.load_dot(1, make_dot(h->sc, dot_default(h->sc, 8, 1)).get());
     const SchedDev& S = h->dsched.d;
     h->jbuf.ensure((size_t)S.n_a * 32 * 8 + 8);
     h->lu.ensure((size_t)S.n_slots * 32 * 8 + 8);

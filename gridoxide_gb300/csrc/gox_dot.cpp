@@ -1,0 +1,853 @@
+// Compiler and checking interpreter of the dot-product programs.
+#include "gox_dot.hpp"
+
+#include <algorithm>
+#include <cmath>
+#include <numeric>
+#include <queue>
+#include <stdexcept>
+
+namespace gox {
+
+namespace {
+
+// The sums of a schedule: per value its ordered terms.  Values are numbered
+// LU slots first, then y (row k at n_slots + k).
+struct Sums {
+  std::vector<int32_t> ptr, a, b;  // value -> terms
+  std::vector<int32_t> col;        // LU slot -> column
+};
+
+Sums make_sums(const Schedule& sc) {
+  Sums s;
+  const int n = sc.n_u, ns = sc.n_slots;
+  s.ptr.assign((size_t)ns + n + 1, 0);
+  s.col.assign(ns, 0);
+  for (int k = 0; k < n; k++) {
+    const int base = sc.c_base[k];
+    for (int d = 0; d < sc.c_ulen[k] + 1 + sc.c_llen[k]; d++) s.col[base + d] = k;
+    for (int e = sc.cu_ptr[k]; e < sc.cu_ptr[k + 1]; e++)
+      for (int t = sc.cu_dptr[e]; t < sc.cu_dptr[e + 1]; t++) s.ptr[base + sc.cu_dst[t] + 1]++;
+    if (sc.fuse_fwd) s.ptr[ns + k + 1] += sc.fw_ptr[k + 1] - sc.fw_ptr[k];
+  }
+  for (size_t v = 0; v + 1 < s.ptr.size(); v++) s.ptr[v + 1] += s.ptr[v];
+  s.a.assign(s.ptr.back(), 0);
+  s.b.assign(s.ptr.back(), 0);
+  std::vector<int32_t> at(s.ptr.begin(), s.ptr.end() - 1);
+  for (int k = 0; k < n; k++) {
+    const int base = sc.c_base[k];
+    for (int e = sc.cu_ptr[k]; e < sc.cu_ptr[k + 1]; e++) {
+      const int j = sc.cu_j[e], l0 = sc.c_base[j] + sc.c_ulen[j] + 1;
+      for (int t = sc.cu_dptr[e]; t < sc.cu_dptr[e + 1]; t++) {
+        const int v = base + sc.cu_dst[t];
+        s.a[at[v]] = l0 + (t - sc.cu_dptr[e]);
+        s.b[at[v]++] = base + (e - sc.cu_ptr[k]);
+      }
+    }
+    if (sc.fuse_fwd)
+      for (int t = sc.fw_ptr[k]; t < sc.fw_ptr[k + 1]; t++) {
+        s.a[at[ns + k]] = sc.fw_slot[t];
+        s.b[at[ns + k]++] = sc.fw_col[t];
+      }
+  }
+  return s;
+}
+
+// Rough cycles of n products on one warp (only their proportions matter:
+// they balance bins and warps)
+double sum_cost(int n) { return 60.0 + 25.0 * n; }
+
+struct Writer {
+  std::vector<uint32_t> w;
+  size_t last = (size_t)-1;  // word index of the header a barrier can go with
+  int idle = 0;              // barriers to take without work
+  void raw(uint32_t x, uint32_t y, uint32_t z, uint32_t v) { w.insert(w.end(), {x, y, z, v}); }
+  // room for n quads in the chunk (and for the quad that leaves it)
+  void room(int n) {
+    const int used = (int)(w.size() / 4) % kDotChunk;
+    if (used + n + 1 <= kDotChunk) return;
+    raw(DOT_SKIP, 0u, 0u, 0u);
+    while (w.size() % (4 * kDotChunk)) w.push_back(0);
+  }
+  void flush() {
+    if (!idle) return;
+    room(1);
+    raw(DOT_BAR, (uint32_t)idle, 0u, 0u);
+    idle = 0;
+  }
+  // a sum's products [0, n) as units of up to 8
+  int sum(uint32_t op, uint32_t y, uint32_t z, const int32_t* a, const int32_t* b, int n) {
+    flush();
+    int units = 0;
+    bool cin = false;
+    do {
+      const int m = std::min(n, kDotTerms);
+      room(1 + (m + 1) / 2);
+      last = w.size();
+      raw(op | (cin ? DOT_CIN : 0u) | (m < n ? DOT_COUT : 0u) | ((uint32_t)m << 12), y, z, 0u);
+      for (int t = 0; t < m; t += 2) {
+        const int u = t + 1 < m ? t + 1 : t;
+        raw((uint32_t)a[t], (uint32_t)b[t], (uint32_t)a[u], (uint32_t)b[u]);
+      }
+      a += m;
+      b += m;
+      n -= m;
+      cin = true;
+      units++;
+    } while (n > 0);
+    return units;
+  }
+  // LU slots and rows, up to 40 of each
+  void touch(const std::vector<int32_t>& lu, const std::vector<int32_t>& x) {
+    if (lu.empty() && x.empty()) return;
+    flush();
+    const int ql = ((int)lu.size() + 3) / 4, qx = ((int)x.size() + 3) / 4;
+    room(1 + ql + qx);
+    raw(DOT_TOUCH, (uint32_t)ql, (uint32_t)qx, 0u);
+    for (const std::vector<int32_t>* l : {&lu, &x})
+      for (size_t i = 0; i < l->size(); i += 4) {
+        auto at = [&](size_t q) { return (uint32_t)(*l)[std::min(q, l->size() - 1)]; };
+        raw(at(i), at(i + 1), at(i + 2), at(i + 3));
+      }
+  }
+  void bar() {
+    if (idle == 0 && last != (size_t)-1) w[last] |= DOT_BARF;
+    else idle++;
+    last = (size_t)-1;
+  }
+  void end() {
+    flush();
+    room(1);
+    raw(DOT_END, 0u, 0u, 0u);
+    // a warp loads up to three chunks past the one it is in
+    while (w.size() % (4 * kDotChunk)) w.push_back(0);
+    w.insert(w.end(), 4 * kDotChunk * 3, 0u);
+  }
+};
+
+void append(DotProgram& P, std::vector<int32_t>& starts, Writer& W) {
+  W.end();
+  starts.push_back((int32_t)(P.words.size() / 4));
+  P.words.insert(P.words.end(), W.w.begin(), W.w.end());
+}
+
+}  // namespace
+
+// 16 warps in FP64: more of them only queue for the FP64 pipe (2 lanes a
+// cycle), and 32 leave too few registers for 8 products in flight.
+static int top_warps(int elem) { return elem == 4 ? 32 : 16; }
+
+// Bins: the more there are, the more of the chip the bottom fills but the more
+// columns are left to the top's ticks (measured, ms per refactor with 32 / 64 /
+// 128 / 256 / 512 / 1024 bins: 2,000 buses, 128 groups FP32 - / 1.93 / 1.79 /
+// 1.77 / 1.78 / -; one group - / - / 1.13 / 1.07 / 1.12 / -; 10,000 buses, 128
+// groups - / 7.4 / 6.4 / 6.1 / 6.0 / -; 20,000 buses, one group - / - / 5.1 /
+// 4.4 / 4.3 / 4.7).  Below 400 unknowns the launches around the top cost what
+// the bottom saves (118 buses FP64, one group: no bins 0.221, 32 bins 0.219).
+DotPlan dot_default(const Schedule& sc, int elem, int groups) {
+  DotPlan p;
+  p.top_warps = top_warps(elem);
+  const int per = groups >= 32 ? 32 : 16;  // unknowns per bin
+  while (sc.n_u >= 400 && p.bins < 512 && p.bins * per < sc.n_u) p.bins = p.bins ? 2 * p.bins : 32;
+  return p;
+}
+
+std::vector<DotPlan> dot_candidates(const Schedule& sc, int elem) {
+  std::vector<DotPlan> out;
+  for (int bins : {0, 32, 64, 128, 256, 512, 1024}) {
+    if (bins > 0 && (bins * 4 > sc.n_u || bins * 400 < sc.n_u)) continue;
+    if (bins == 0 && sc.n_u > 1500) continue;
+    for (int w : {32, 16}) {
+      if (w > top_warps(elem)) continue;
+      DotPlan p;
+      p.bins = bins;
+      p.top_warps = w;
+      out.push_back(p);
+    }
+  }
+  return out;
+}
+
+void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
+  P = DotProgram();
+  P.plan = plan;
+  const int n = sc.n_u, ns = sc.n_slots;
+  const bool subst = sc.fuse_fwd;
+  P.with_subst = subst;
+  const Sums S = make_sums(sc);
+  auto nt = [&](int v) { return S.ptr[v + 1] - S.ptr[v]; };
+  auto len = [&](int k) { return sc.c_ulen[k] + 1 + sc.c_llen[k]; };
+  std::vector<int32_t> taken(ns + n, 0);  // products already in the program, per value
+
+  // ---- bottom: parts of the elimination forest of at most cap * (total /
+  // bins) cost, grown column by column (a column joins when everything it
+  // depends on is in the bottom and the part it makes stays small enough)
+  std::vector<double> ccost(n, 0.0);
+  double total = 0;
+  for (int k = 0; k < n; k++) {
+    ccost[k] = 300.0 + 12.0 * len(k);
+    for (int e = sc.cu_ptr[k]; e < sc.cu_ptr[k + 1]; e++) ccost[k] += 40.0 + 8.0 * (sc.cu_dptr[e + 1] - sc.cu_dptr[e]);
+    if (subst) ccost[k] += 8.0 * nt(ns + k);
+    total += ccost[k];
+  }
+  std::vector<int32_t> part(n, -1);  // union-find parent of bottom columns, -1: top
+  std::vector<double> pcost(n, 0.0);
+  auto find = [&](int k) {
+    while (part[k] != k) k = part[k] = part[part[k]];
+    return k;
+  };
+  if (plan.bins > 0) {
+    const double cap = plan.cap * total / plan.bins;
+    std::vector<int32_t> roots;
+    for (int k = 0; k < n; k++) {
+      bool ok = true;
+      roots.clear();
+      double c = ccost[k];
+      auto dep = [&](int j) {
+        if (part[j] < 0) { ok = false; return; }
+        const int r = find(j);
+        if (std::find(roots.begin(), roots.end(), r) == roots.end()) {
+          roots.push_back(r);
+          c += pcost[r];
+        }
+      };
+      for (int e = sc.cu_ptr[k]; ok && e < sc.cu_ptr[k + 1]; e++) dep(sc.cu_j[e]);
+      if (subst)
+        for (int t = sc.fw_ptr[k]; ok && t < sc.fw_ptr[k + 1]; t++) dep(sc.fw_col[t]);
+      if (!ok || c > cap) continue;
+      part[k] = k;
+      for (int r : roots) part[r] = k;
+      pcost[k] = c;
+    }
+  }
+  // parts to bins, largest first onto the least loaded bin
+  std::vector<std::vector<int32_t>> members(n);
+  std::vector<int32_t> parts;
+  for (int k = 0; k < n; k++)
+    if (part[k] >= 0) {
+      const int r = find(k);
+      members[r].push_back(k);
+      if (r == k) parts.push_back(k);
+      P.bottom_cols++;
+    }
+  std::stable_sort(parts.begin(), parts.end(), [&](int x, int y) { return pcost[x] > pcost[y]; });
+  std::vector<std::vector<int32_t>> bin(plan.bins);
+  {
+    std::priority_queue<std::pair<double, int>, std::vector<std::pair<double, int>>, std::greater<>> q;
+    for (int b = 0; b < plan.bins; b++) q.push({0.0, b});
+    for (int r : parts) {
+      auto [c, b] = q.top();
+      q.pop();
+      bin[b].insert(bin[b].end(), members[r].begin(), members[r].end());
+      q.push({c + pcost[r], b});
+    }
+  }
+  auto emit_sum = [&](Writer& W, uint32_t op, int v, uint32_t z, int t0, int t1) {
+    const bool y = v >= ns;
+    P.units += W.sum(op | (y && t0 == S.ptr[v] ? DOT_FIRST : 0u), (uint32_t)(y ? v - ns : v), z, S.a.data() + t0,
+                     S.b.data() + t0, t1 - t0);
+  };
+  for (int b = 0; b < plan.bins; b++) {
+    if (bin[b].empty()) continue;
+    Writer W;
+    for (int k : bin[b]) {
+      const int base = sc.c_base[k], ul = sc.c_ulen[k];
+      for (int d = 0; d < len(k); d++) {
+        const int v = base + d;
+        if (d < ul && nt(v) == 0) continue;
+        emit_sum(W, d < ul ? DOT_U : d == ul ? DOT_D : DOT_L, v, 0, S.ptr[v], S.ptr[v + 1]);
+        taken[v] = nt(v);
+      }
+      if (subst) {
+        emit_sum(W, DOT_Y, ns + k, 0, S.ptr[ns + k], S.ptr[ns + k + 1]);
+        taken[ns + k] = nt(ns + k);
+      }
+    }
+    append(P, P.bottom, W);
+  }
+  // ---- prep: per top column, the leading products of each sum whose values
+  // the bottom (or the prep of this same column) finishes
+  if (P.bottom_cols > 0) {
+    for (int k = 0; k < n; k++) {
+      if (part[k] >= 0) continue;
+      Writer W;
+      const int base = sc.c_base[k];
+      auto prefix = [&](int v) {
+        int t = S.ptr[v];
+        for (; t < S.ptr[v + 1]; t++) {
+          if (part[S.col[S.a[t]]] < 0) break;  // an L value of a top column
+          if (v >= ns ? part[S.b[t]] < 0 : taken[S.b[t]] != nt(S.b[t])) break;
+        }
+        if (t == S.ptr[v]) return;
+        emit_sum(W, v >= ns ? DOT_Y : DOT_U, v, 0, S.ptr[v], t);
+        taken[v] = t - S.ptr[v];
+        P.prep_terms += taken[v];
+      };
+      for (int d = 0; d < len(k); d++) prefix(base + d);
+      if (subst) prefix(ns + k);
+      if (!W.w.empty()) append(P, P.prep, W);
+    }
+  }
+
+  // ---- top: nodes (a leading part of a sum, a U entry, a column's pivot and
+  // L entries, a y), each in a tick after the ticks of what it reads
+  struct Node {
+    int32_t kind;    // 0 part, 1 U, 2 column, 3 y
+    int32_t v;       // value, or the column
+    int32_t t0, t1;  // products (kinds 0, 1, 3)
+    int32_t tick;    // as soon as possible
+    int32_t late;    // as late as possible
+    double cost;
+  };
+  std::vector<Node> nodes;
+  std::vector<std::pair<int32_t, int32_t>> edges;
+  std::vector<int32_t> node_of(ns + n, -1);  // value -> the node that finishes it (-1: before the top)
+  std::vector<int32_t> done(ns + n, -1);     // value -> tick it is final after
+  std::vector<int32_t> from(ns + n, 0);      // first product left for the node that finishes it
+  const int NT = plan.top_warps;
+  int makespan = 0;
+  std::vector<int32_t> preds;
+  auto add_node = [&](Node nd) {
+    std::sort(preds.begin(), preds.end());
+    preds.erase(std::unique(preds.begin(), preds.end()), preds.end());
+    const int id = (int)nodes.size();
+    for (int p : preds)
+      if (p >= 0) edges.push_back({p, id});
+    nodes.push_back(nd);
+    makespan = std::max(makespan, nd.tick + 1);
+    return id;
+  };
+  auto second = [&](int v, int t) { return v >= ns ? ns + S.b[t] : S.b[t]; };
+  auto ready = [&](int v, int t0, int t1) {
+    int r = -1;
+    for (int t = t0; t < t1; t++) r = std::max({r, done[S.a[t]], done[second(v, t)]});
+    return r + 1;
+  };
+  auto take_preds = [&](int v, int t0, int t1) {
+    for (int t = t0; t < t1; t++) {
+      preds.push_back(node_of[S.a[t]]);
+      preds.push_back(node_of[second(v, t)]);
+    }
+  };
+  // a long sum whose last products come late: its leading ones run as parts in
+  // earlier ticks, so the tick that finishes it has few left
+  constexpr int kPartMin = 5, kPartMax = 16;
+  auto split = [&](int v, int final_tick) {
+    int t = S.ptr[v] + taken[v];
+    const int t1 = S.ptr[v + 1];
+    int prev = -1, prev_tick = -1;
+    while (t1 - t >= kPartMin) {
+      int q = t, r = std::max(0, prev_tick + 1);
+      while (q < t1 && q - t < kPartMax) {
+        const int rq = std::max(r, ready(v, q, q + 1));
+        if (rq > final_tick - 1) break;
+        r = rq;
+        q++;
+      }
+      if (q - t < kPartMin) break;
+      preds.clear();
+      take_preds(v, t, q);
+      preds.push_back(prev);
+      prev = add_node({0, v, t, q, r, 0, sum_cost(q - t)});
+      prev_tick = r;
+      t = q;
+      P.parts++;
+    }
+    from[v] = t;
+    return prev;
+  };
+  auto left = [&](int v) { return S.ptr[v + 1] - from[v]; };
+  for (int k = 0; k < n; k++) {
+    if (part[k] >= 0) continue;
+    const int base = sc.c_base[k], ul = sc.c_ulen[k];
+    for (int v = base; v < base + ul; v++) {
+      if (nt(v) == taken[v]) continue;
+      const int r = ready(v, S.ptr[v] + taken[v], S.ptr[v + 1]);
+      const int p = split(v, r);
+      preds.clear();
+      take_preds(v, from[v], S.ptr[v + 1]);
+      preds.push_back(p);
+      node_of[v] = add_node({1, v, from[v], S.ptr[v + 1], r, 0, sum_cost(left(v))});
+      done[v] = r;
+    }
+    int r = 0;
+    for (int v = base + ul; v < base + len(k); v++) r = std::max(r, ready(v, S.ptr[v] + taken[v], S.ptr[v + 1]));
+    std::vector<int32_t> cp;
+    double cost = 0;
+    for (int v = base + ul; v < base + len(k); v++) {
+      cp.push_back(split(v, r));
+      cost += sum_cost(left(v));
+    }
+    preds = cp;
+    for (int v = base + ul; v < base + len(k); v++) take_preds(v, from[v], S.ptr[v + 1]);
+    const int id = add_node({2, k, 0, 0, r, 0, cost});
+    for (int v = base + ul; v < base + len(k); v++) {
+      node_of[v] = id;
+      done[v] = r;
+    }
+    if (subst && (taken[ns + k] < nt(ns + k) || taken[ns + k] == 0)) {
+      const int v = ns + k;
+      const int ry = ready(v, S.ptr[v] + taken[v], S.ptr[v + 1]);
+      const int p = split(v, ry);
+      preds.clear();
+      take_preds(v, from[v], S.ptr[v + 1]);
+      preds.push_back(p);
+      node_of[v] = add_node({3, v, from[v], S.ptr[v + 1], ry, 0, sum_cost(left(v))});
+      done[v] = ry;
+    }
+  }
+  // as late as possible
+  const int nn = (int)nodes.size();
+  for (auto& x : nodes) x.late = makespan - 1;
+  std::vector<int32_t> sptr(nn + 1, 0), succ(edges.size()), npred(nn, 0);
+  for (auto& e : edges) {
+    sptr[e.first + 1]++;
+    npred[e.second]++;
+  }
+  for (int i = 0; i < nn; i++) sptr[i + 1] += sptr[i];
+  {
+    std::vector<int32_t> at(sptr.begin(), sptr.end() - 1);
+    for (auto& e : edges) succ[at[e.first]++] = e.second;
+  }
+  for (int i = nn - 1; i >= 0; i--)
+    for (int q = sptr[i]; q < sptr[i + 1]; q++) nodes[i].late = std::min(nodes[i].late, nodes[succ[q]].late - 1);
+
+  // what each tick's warps do (the backward rows' ticks included)
+  struct Do { int32_t w; uint32_t op; int32_t v; uint32_t z; int32_t t0, t1; };
+  std::vector<std::vector<Do>> plan_of;
+  std::vector<std::vector<double>> load_of;
+  int tick = 0;
+  auto emit = [&](int w, uint32_t op, int v, uint32_t z, int t0, int t1) {
+    P.top_terms += t1 - t0;
+    plan_of.back().push_back({w, op, v, z, t0, t1});
+  };
+
+  // ticks: what cannot wait, then ready nodes (the most urgent first) while
+  // the warps have room beside it
+  {
+    using Item = std::pair<int32_t, int32_t>;  // late, node
+    std::priority_queue<Item, std::vector<Item>, std::greater<>> q;
+    for (int i = 0; i < nn; i++)
+      if (npred[i] == 0) q.push({nodes[i].late, i});
+    int todo = nn;
+    std::vector<int32_t> now;
+    std::vector<double> load(NT);
+    while (todo > 0) {
+      now.clear();
+      double room = 0, sum = 0, ready_cost = 0;
+      std::vector<Item> rest;
+      while (!q.empty()) {
+        Item it = q.top();
+        q.pop();
+        ready_cost += nodes[it.second].cost;
+        if (it.first <= tick) {
+          now.push_back(it.second);
+          sum += nodes[it.second].cost;
+          room = std::max(room, nodes[it.second].kind == 2 ? 250.0 : nodes[it.second].cost);
+        } else {
+          rest.push_back(it);
+        }
+      }
+      room = std::max({room, 250.0, std::min(ready_cost / NT, 6000.0)});
+      for (Item& it : rest) {
+        if (sum + nodes[it.second].cost <= 0.8 * room * NT) {
+          now.push_back(it.second);
+          sum += nodes[it.second].cost;
+        } else {
+          q.push(it);
+        }
+      }
+      // warps: columns first (split over warps while there are warps for all
+      // their entries), then the other sums onto the least loaded warp
+      std::fill(load.begin(), load.end(), 0.0);
+      plan_of.emplace_back();
+      std::vector<int32_t> cols, others, whole;
+      for (int i : now) (nodes[i].kind == 2 ? cols : others).push_back(i);
+      std::stable_sort(cols.begin(), cols.end(), [&](int x, int y) { return nodes[x].late < nodes[y].late; });
+      int used = 0, mids = 0;
+      const int shift = (tick * 7) % NT;
+      auto least = [&]() { return (int)(std::min_element(load.begin(), load.end()) - load.begin()); };
+      for (int i : cols) {
+        const int k = nodes[i].v, ul = sc.c_ulen[k], ll = sc.c_llen[k], base = sc.c_base[k];
+        if (ll > 0 && used + 1 + ll <= NT && mids < kDotMaxMid) {
+          const uint32_t z = (uint32_t)(32 * (1 + ll)) | ((uint32_t)mids << 16), id = (uint32_t)(mids + 1) << 8;
+          mids++;
+          for (int e = 0; e <= ll; e++) {
+            const int v = base + ul + e, w = (used++ + shift) % NT;
+            emit(w, (e ? DOT_LH : DOT_D) | id, v, z, from[v], S.ptr[v + 1]);
+            load[w] += sum_cost(left(v)) + (e ? 60 : 0);
+          }
+        } else {
+          whole.push_back(i);
+        }
+      }
+      for (int i : whole) {
+        const int k = nodes[i].v, ul = sc.c_ulen[k], ll = sc.c_llen[k], base = sc.c_base[k];
+        const int w = least();
+        for (int e = 0; e <= ll; e++) {
+          const int v = base + ul + e;
+          emit(w, e ? DOT_L : DOT_D, v, 0, from[v], S.ptr[v + 1]);
+          load[w] += sum_cost(left(v));
+        }
+      }
+      std::stable_sort(others.begin(), others.end(), [&](int x, int y) { return nodes[x].cost > nodes[y].cost; });
+      for (int i : others) {
+        const Node& nd = nodes[i];
+        const int w = least();
+        const bool y = nd.v >= ns;
+        emit(w, y ? DOT_Y : DOT_U, nd.v, 0, nd.t0, nd.t1);
+        load[w] += nd.cost;
+      }
+      load_of.push_back(load);
+      todo -= (int)now.size();
+      tick++;
+      for (int i : now)
+        for (int s = sptr[i]; s < sptr[i + 1]; s++)
+          if (--npred[succ[s]] == 0) q.push({nodes[succ[s]].late, succ[s]});
+    }
+  }
+  P.ticks = tick;
+  auto row = [&](Writer& w, int k) {
+    P.units += w.sum(DOT_B, (uint32_t)k, (uint32_t)sc.diag_slot[k], sc.bw_slot.data() + sc.bw_ptr[k],
+                     sc.bw_col.data() + sc.bw_ptr[k], sc.bw_ptr[k + 1] - sc.bw_ptr[k]);
+  };
+  // ---- backward rows of the top columns, level by level, then the bottom's
+  if (subst) {
+    std::vector<int32_t> lev(n, 0);
+    std::vector<std::vector<int32_t>> bylev;
+    for (int k = n - 1; k >= 0; k--) {
+      if (part[k] >= 0) continue;
+      int l = 0;
+      for (int t = sc.bw_ptr[k]; t < sc.bw_ptr[k + 1]; t++) {
+        if (part[sc.bw_col[t]] >= 0) throw std::runtime_error("a top row reads a bottom row");
+        l = std::max(l, lev[sc.bw_col[t]] + 1);
+      }
+      lev[k] = l;
+      if ((int)bylev.size() <= l) bylev.resize(l + 1);
+      bylev[l].push_back(k);
+    }
+    P.back_ticks = (int)bylev.size();
+    int turn = 0;
+    for (auto& rows : bylev) {
+      std::vector<double> load(NT, 0.0);
+      plan_of.emplace_back();
+      for (int k : rows) {
+        const int w = rows.size() <= (size_t)NT ? turn++ % NT
+                                                : (int)(std::min_element(load.begin(), load.end()) - load.begin());
+        load[w] += sum_cost(sc.bw_ptr[k + 1] - sc.bw_ptr[k]);
+        plan_of.back().push_back({w, DOT_B, ns + k, 0u, 0, 0});
+      }
+      load_of.push_back(load);
+    }
+    for (int b = 0; b < plan.bins; b++) {
+      if (bin[b].empty()) continue;
+      Writer w;
+      for (size_t i = bin[b].size(); i-- > 0;) row(w, bin[b][i]);
+      append(P, P.back, w);
+    }
+  }
+  // the top's streams; a value whose last use lies too far back to be still in
+  // the L1 is touched `ahead` ticks before the tick that needs it, by the
+  // warps with the least to do there (not for ticks that fill all warps: they
+  // hide their loads behind each other)
+  {
+    const int nticks = (int)plan_of.size();
+    std::vector<std::vector<std::pair<std::vector<int32_t>, std::vector<int32_t>>>> touch(nticks);  // per tick and warp
+    if (plan.ahead > 0) {
+      std::vector<int64_t> last(ns + n, -(int64_t)1 << 40);
+      int64_t now = 0;
+      std::vector<int32_t> need;
+      for (int t = 0; t < nticks; t++) {
+        need.clear();
+        auto use = [&](int v) {
+          if (now - last[v] > plan.keep) need.push_back(v);
+          last[v] = now++;
+        };
+        for (const Do& d : plan_of[t]) {
+          use(d.v);
+          if (d.op == DOT_B) {
+            const int k = d.v - ns;
+            use(sc.diag_slot[k]);
+            for (int e = sc.bw_ptr[k]; e < sc.bw_ptr[k + 1]; e++) {
+              use(sc.bw_slot[e]);
+              use(ns + sc.bw_col[e]);
+            }
+          } else {
+            for (int e = d.t0; e < d.t1; e++) {
+              use(S.a[e]);
+              use(second(d.v, e));
+            }
+          }
+        }
+        const int at = t - plan.ahead;
+        if (at < 0 || (int)plan_of[t].size() > 3 * NT || need.empty()) continue;
+        if (touch[at].empty()) touch[at].resize(NT);
+        std::vector<double>& load = load_of[at];
+        for (size_t i = 0; i < need.size(); i += 12) {
+          const int w = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+          for (size_t q = i; q < std::min(need.size(), i + 12); q++)
+            (need[q] >= ns ? touch[at][w].second : touch[at][w].first).push_back(need[q] >= ns ? need[q] - ns : need[q]);
+          load[w] += 60.0 + 8.0 * 12;
+          P.touched += std::min<size_t>(12, need.size() - i);
+        }
+      }
+    }
+    std::vector<Writer> W(NT);
+    for (int t = 0; t < nticks; t++) {
+      for (const Do& d : plan_of[t]) {
+        if (d.op == DOT_B) row(W[d.w], d.v - ns);
+        else emit_sum(W[d.w], d.op, d.v, d.z, d.t0, d.t1);
+      }
+      if (!touch[t].empty())
+        for (int w = 0; w < NT; w++) {
+          auto& x = touch[t][w];
+          for (size_t i = 0; i < std::max(x.first.size(), x.second.size()); i += 40) {
+            auto cut = [&](const std::vector<int32_t>& l) {
+              return std::vector<int32_t>(l.begin() + std::min(i, l.size()), l.begin() + std::min(i + 40, l.size()));
+            };
+            W[w].touch(cut(x.first), cut(x.second));
+          }
+        }
+      for (auto& w : W) w.bar();
+    }
+    for (auto& w : W) append(P, P.top, w);
+  }
+}
+
+std::string run_dot_host(const Schedule& sc, const DotProgram& P, std::vector<double>& lu,
+                         const std::vector<double>& rhs, std::vector<double>& X, bool& singular) {
+  const int n = sc.n_u, ns = sc.n_slots;
+  const Sums S = make_sums(sc);
+  X.assign(n, 0.0);
+  singular = false;
+  // per value (LU slots, then the solution vector): how many products its sum
+  // has taken, whether it is final, who wrote and read it last and when
+  std::vector<int32_t> taken(ns + n, 0);
+  std::vector<char> fin(ns + n, 0), xdone(n, 0);
+  std::vector<int64_t> wtick(ns + n, -1), rtick(ns + n, -1);
+  std::vector<int32_t> wwarp(ns + n, -1), rwarp(ns + n, -1);
+  for (int k = 0; k < n; k++)
+    for (int v = sc.c_base[k]; v < sc.c_base[k] + sc.c_ulen[k]; v++)
+      if (S.ptr[v + 1] == S.ptr[v]) fin[v] = 1;
+  if (!P.with_subst)
+    for (int k = 0; k < n; k++) fin[ns + k] = 1;
+  std::string err;
+  const size_t nq = P.words.size() / 4;
+  int64_t tick = 0;
+  auto fail = [&](const char* s) {
+    if (err.empty()) err = s;
+    return false;
+  };
+  auto read = [&](int v, int w) {
+    if (wtick[v] == tick && wwarp[v] != w) return fail("a value read in the tick another warp writes it");
+    if (rtick[v] != tick) { rtick[v] = tick; rwarp[v] = w; }
+    else if (rwarp[v] != w) rwarp[v] = -2;  // several warps
+    return true;
+  };
+  auto write = [&](int v, int w) {
+    if (wtick[v] == tick && wwarp[v] != w) return fail("two warps write one value in one tick");
+    if (rtick[v] == tick && rwarp[v] != w) return fail("a value written in the tick another warp reads it");
+    wtick[v] = tick;
+    wwarp[v] = w;
+    return true;
+  };
+  struct Held { uint32_t z, id; };
+  struct Warp {
+    size_t pos;
+    int bars = 0;
+    bool ended = false, waits = false;  // waits: at a mid barrier
+    double inv = 0, car = 0;
+    int pivot = -1, carried = -1;       // slot of the warp's last D, value of the open sum
+  };
+  std::vector<std::pair<uint32_t, double>> mid_inv;  // mid barriers reached by their pivot's warp
+  std::vector<Held> held;
+  // runs a warp up to its next barrier, a mid barrier nobody reached yet, or its end
+  auto step = [&](Warp& A, int w, bool top) -> bool {
+    if (!A.waits && A.bars > 0 && --A.bars > 0) return true;
+    for (;;) {
+      if (A.pos >= nq) return fail("a stream runs past the program");
+      const uint32_t* h = &P.words[A.pos * 4];
+      const uint32_t op = h[0] & 15u;
+      if (op == DOT_END) {
+        A.ended = true;
+        return A.carried < 0 || fail("a sum left open");
+      }
+      if (op == DOT_SKIP) {
+        A.pos = (A.pos / kDotChunk + 1) * kDotChunk;
+        continue;
+      }
+      if (op == DOT_BAR) {
+        A.pos++;
+        A.bars = (int)h[1];
+        return (top && A.bars > 0) || fail("a bin with a barrier");
+      }
+      if (op == DOT_TOUCH) {
+        const size_t nt = (size_t)h[1] + h[2];
+        if (A.pos % kDotChunk + 1 + nt + 1 > (size_t)kDotChunk || A.pos + 1 + nt > nq) return fail("a unit that leaves its chunk");
+        for (size_t i = 0; i < 4 * nt; i++)
+          if (h[4 + i] >= (uint32_t)(i < 4 * (size_t)h[1] ? ns : n)) return fail("a touched value out of range");
+        A.pos += 1 + nt;
+        continue;
+      }
+      const int m = (int)((h[0] >> 12) & 15u);
+      const bool row = op == DOT_Y || op == DOT_B, cin = (h[0] & DOT_CIN) != 0, cout = (h[0] & DOT_COUT) != 0;
+      if (op < DOT_U || op > DOT_B || m > kDotTerms || h[1] >= (uint32_t)(row ? n : ns)) return fail("a unit out of range");
+      if (A.pos % kDotChunk + 1 + (m + 1) / 2 + 1 > kDotChunk) return fail("a unit that leaves its chunk");
+      if (A.pos + 1 + (m + 1) / 2 > nq) return fail("a unit runs past the program");
+      const int v = row ? ns + (int)h[1] : (int)h[1];
+      double mid = 0;
+      if (op == DOT_LH && !cout) {
+        const std::pair<uint32_t, double>* x = nullptr;
+        for (auto& y : mid_inv)
+          if (y.first == ((h[0] >> 8) & 15u)) x = &y;
+        A.waits = x == nullptr;
+        if (A.waits) return true;
+        mid = x->second;
+      }
+      if (cin != (A.carried >= 0) || (cin && A.carried != v)) return fail("a sum carried to another value");
+      A.carried = -1;
+      const bool first = op == DOT_Y && (h[0] & DOT_FIRST);
+      double s = A.car, d = 0;
+      if (!cin) {
+        if (!first && !read(v, w)) return false;
+        s = first ? rhs[h[1]] : row ? X[h[1]] : lu[v];
+      }
+      if (op == DOT_B) {
+        if (!fin[v]) return fail("x before y is final");
+        if (h[2] != (uint32_t)sc.diag_slot[h[1]] || !fin[h[2]]) return fail("a backward row with another pivot");
+        if (!read((int)h[2], w)) return false;
+        d = lu[h[2]];
+        if (!cin) taken[v] = 0;  // counts the backward terms from here on
+      } else {
+        if (fin[v]) return fail("a final value written again");
+        if (op == DOT_Y && !cin && first != (taken[v] == 0)) return fail("a sum that starts twice or not at all");
+      }
+      for (int t = 0; t < m; t++) {
+        const uint32_t* q = h + 4 + 4 * (t / 2) + 2 * (t & 1);
+        if (q[0] >= (uint32_t)ns || q[1] >= (uint32_t)(row ? n : ns)) return fail("a product out of range");
+        const int b = row ? ns + (int)q[1] : (int)q[1];
+        if (!read((int)q[0], w) || !read(b, w)) return false;
+        if (op == DOT_B) {
+          const int e = sc.bw_ptr[h[1]] + taken[v]++;
+          if (e >= sc.bw_ptr[h[1] + 1] || (int)q[0] != sc.bw_slot[e] || (int)q[1] != sc.bw_col[e])
+            return fail("a backward term out of order");
+          if (!fin[q[0]] || !xdone[q[1]]) return fail("a backward term before its x");
+        } else {
+          const int e = S.ptr[v] + taken[v]++;
+          if (e >= S.ptr[v + 1] || S.a[e] != (int)q[0] || S.b[e] != (int)q[1]) return fail("a product out of order");
+          if (!fin[q[0]] || !fin[b]) return fail("a product before its value is final");
+        }
+        s -= lu[q[0]] * (row ? X[q[1]] : lu[b]);
+      }
+      A.pos += 1 + (m + 1) / 2;
+      if (cout) {
+        A.car = s;
+        A.carried = v;
+        if (h[0] & DOT_BARF) return fail("a barrier inside a sum");
+        continue;
+      }
+      if (!write(v, w)) return false;
+      const bool whole = op != DOT_B && taken[v] == S.ptr[v + 1] - S.ptr[v];
+      const int k = row ? 0 : S.col[v];
+      if (op == DOT_U || op == DOT_Y) {
+        (row ? X[h[1]] : lu[v]) = s;
+        // a U unit on the pivot or an L entry is a leading part of its sum
+        if ((row || v < sc.diag_slot[k]) && whole) fin[v] = 1;
+      } else if (op == DOT_D) {
+        if (!whole || v != sc.diag_slot[k]) return fail("an incomplete pivot");
+        lu[v] = s;
+        fin[v] = 1;
+        if (s == 0) singular = true;
+        A.inv = 1.0 / s;
+        A.pivot = v;
+        const uint32_t id = (h[0] >> 8) & 15u;
+        if (id && (!top || id > (uint32_t)kDotMaxMid || (h[2] >> 16) >= (uint32_t)kDotMaxMid))
+          return fail("a mid barrier out of range");
+        if (id) mid_inv.push_back({id, A.inv});
+      } else if (op == DOT_L || op == DOT_LH) {
+        if (!whole || v <= sc.diag_slot[k]) return fail("an incomplete L entry");
+        if (op == DOT_L) {
+          if (A.pivot != sc.diag_slot[k]) return fail("an L entry without its pivot");
+        } else {
+          if (!fin[sc.diag_slot[k]] || wtick[sc.diag_slot[k]] != tick) return fail("an L entry of another column's pivot");
+          held.push_back({h[2], (h[0] >> 8) & 15u});
+          A.pivot = -1;
+        }
+        lu[v] = s * (op == DOT_L ? A.inv : mid);
+        fin[v] = 1;
+      } else {
+        if (taken[v] != sc.bw_ptr[h[1] + 1] - sc.bw_ptr[h[1]]) return fail("an incomplete backward row");
+        const double x = s / d;
+        if (!std::isfinite(x)) singular = true;
+        X[h[1]] = x;
+        xdone[h[1]] = 1;
+      }
+      if (h[0] & DOT_BARF) {
+        if (!top) return fail("a bin with a barrier");
+        A.bars = 1;
+        return true;
+      }
+    }
+  };
+  auto launch = [&](const std::vector<int32_t>& st, auto&& run) {
+    int w = 0;
+    for (int32_t s : st)
+      if (s < 0 || (size_t)s >= nq || !run(s, w++)) return false;
+    tick++;
+    return true;
+  };
+  auto bin = [&](int32_t s, int w) {
+    Warp B{(size_t)s};
+    return step(B, w, false) && (B.ended || fail("a bin that does not end"));
+  };
+  if (!launch(P.bottom, bin) || !launch(P.prep, bin)) return err;
+  const int NT = (int)P.top.size();
+  std::vector<Warp> A;
+  for (int32_t s : P.top) A.push_back({(size_t)s});
+  for (int ended = 0; ended < NT;) {
+    held.clear();
+    mid_inv.clear();
+    ended = 0;
+    // every warp to its barrier; one that waits at a mid barrier goes on when
+    // the pivot's warp has arrived there
+    std::vector<char> run(NT, 1);
+    for (bool moved = true; moved;) {
+      moved = false;
+      for (int w = 0; w < NT; w++) {
+        if (!run[w] || A[w].ended) continue;
+        const size_t at = A[w].pos;
+        const bool waited = A[w].waits;
+        if (!step(A[w], w, true)) return err;
+        run[w] = A[w].waits;
+        moved |= !A[w].waits || A[w].pos != at || !waited;
+      }
+    }
+    for (int w = 0; w < NT; w++) {
+      if (A[w].waits) return "a mid barrier that nobody reaches";
+      ended += A[w].ended;
+    }
+    for (auto& m : mid_inv) {
+      int cnt = 0;
+      for (auto& m2 : mid_inv) cnt += m2.first == m.first;
+      uint32_t same = 1;
+      for (auto& x : held) same += x.id == m.first;
+      if (cnt != 1 || same < 2) return "a mid barrier used twice in one tick, or by nobody";
+    }
+    for (auto& x : held) {
+      uint32_t same = 1;
+      for (auto& y : held) same += y.id == x.id;
+      if ((x.z & 0xffffu) != 32u * same) return "a held L entry without its mid barrier";
+    }
+    if (ended != 0 && ended != NT) return "the warps take different numbers of barriers";
+    tick++;
+  }
+  if (!launch(P.back, bin)) return err;
+  for (int v = 0; v < ns + n; v++)
+    if (!fin[v]) return "a value is left unfinished";
+  if (P.with_subst)
+    for (int k = 0; k < n; k++)
+      if (!xdone[k]) return "a row of the solution is left out";
+  return err;
+}
+
+}  // namespace gox

@@ -1,0 +1,95 @@
+// Dot-product programs for the batched refactor.
+//
+// Every value of the factor and of the two substitutions is one ordered sum
+// of products: an entry (i, k) of L or U is its A value minus the L(i, j)
+// U(j, k) in KLU's update order (an L entry then times the pivot's
+// reciprocal), y_k is b_k minus the L(k, j) y_j, x_k is y_k minus the U(k, j)
+// x_j, divided by the pivot.  A program may run the sums in any order of
+// values, and a sum in pieces, as long as each value's own products stay in
+// order: the result is the stream form's (gox_stream.hpp) bit for bit.
+//
+// Four launches run a refactor with both substitutions:
+//   bottom    columns in independent parts of the elimination forest, whole
+//             parts assigned to bins; one warp runs a bin's columns in order
+//             (no barrier: it wrote every value it reads), a column at a time
+//             in its warp's shared memory
+//   prep      one warp per remaining column: the leading part of each of its
+//             sums that only needs bottom columns
+//   top       the rest of those columns, one CTA per group: the sums as
+//             units of up to 8 products spread over the warps, in ticks that
+//             only read values of earlier ticks, with a CTA barrier after
+//             each; then their backward rows
+//   back      the backward rows of the bottom columns, bin by bin
+#pragma once
+#include <cstdint>
+#include <string>
+#include <vector>
+
+#include "gox_engine.hpp"
+
+namespace gox {
+
+// A stream is a list of 16-byte quads in chunks of 32.  A unit is one header
+// quad, then its products (a, b), two per quad, all in one chunk:
+//   x = op | barrier after << 4 | first << 5 | carry in << 6 | carry out << 7 |
+//       mid << 8 | n << 12
+//   y = the value's slot (U, D, L, LH) or row (Y, B); BAR: how many
+//   z = D, LH: threads of the mid barrier | shared index << 16;  B: pivot slot
+// a and b are LU slots (U, D, L, LH), or an LU slot and a row (Y, B).  A sum of
+// more than 8 products is carried from unit to unit in a register.
+enum : uint32_t {
+  DOT_END = 0,
+  DOT_BAR = 1,   // y CTA barriers
+  DOT_SKIP = 2,  // on to the next chunk
+  DOT_TOUCH = 3, // y quads of LU slots, then z quads of rows: values a later
+                 // unit needs, loaded into the SM's L1 and dropped
+  DOT_U = 4,     // U(j, k), or a leading part of any LU entry's sum
+  DOT_D = 5,     // pivot: also its reciprocal, for the warp's next L units; with
+                 // a mid barrier also to shared memory, for the LH units
+  DOT_L = 6,     // L(i, k): times the reciprocal of the warp's last D
+  DOT_LH = 7,    // L(i, k): its sum first, then the mid barrier, then scaled
+  DOT_Y = 8,     // y_k (first: starts from the right-hand side, else from y)
+  DOT_B = 9      // x_k
+};
+constexpr uint32_t DOT_BARF = 1u << 4, DOT_FIRST = 1u << 5, DOT_CIN = 1u << 6, DOT_COUT = 1u << 7;
+constexpr int kDotTerms = 8;    // products of a unit
+constexpr int kDotChunk = 32;   // quads of a chunk: one 16-byte load per lane
+constexpr int kDotMaxMid = 14;  // mid barriers of one tick (ids 1..14)
+
+struct DotPlan {
+  int bins = 0;        // bins of the bottom (0: every column is in the top)
+  int top_warps = 16;
+  double cap = 1.0;    // largest part, of a bin's even share
+  int ahead = 4;       // ticks by which values are touched before their use (0: not)
+  int keep = 700;      // values touched since, after which one is taken to have left the L1
+};
+
+struct DotProgram {
+  DotPlan plan;
+  std::vector<uint32_t> words;                   // all streams, 4 words per quad
+  std::vector<int32_t> bottom, prep, top, back;  // per bin / warp: first quad of its stream
+  bool with_subst = false;                       // forward and backward substitution included
+  int ticks = 0, back_ticks = 0;
+  int64_t units = 0, parts = 0, bottom_cols = 0, top_terms = 0, prep_terms = 0, touched = 0;
+};
+
+// The plan taken where nothing is timed, for `groups` groups of scenarios, and
+// the plans the autotuner times.
+DotPlan dot_default(const Schedule& sc, int elem, int groups);
+std::vector<DotPlan> dot_candidates(const Schedule& sc, int elem);
+
+// Compiles the refactor of a schedule (with both substitutions when the
+// schedule fuses the forward one).
+void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& out);
+
+// Host interpreter of a program for one scenario in FP64, with the checks
+// that make the device's order of execution irrelevant: every index in
+// range, every value final when it is read and written by the same warp
+// earlier or in an earlier tick or launch (reads checked when the device
+// issues them), no two warps on one value in one tick, equal barrier counts,
+// every sum complete and in order.  Returns an empty string or the first
+// violation.
+std::string run_dot_host(const Schedule& sc, const DotProgram& p, std::vector<double>& lu,
+                         const std::vector<double>& rhs, std::vector<double>& X, bool& singular);
+
+}  // namespace gox

@@ -670,6 +670,14 @@ struct StreamDev {
   int sync;        // levels end in: 0 CTA barriers, 1 per-warp progress flags
 };
 
+// A dot-product program on the device (gox_dot.hpp): its streams, and per
+// launch the first quad of each.
+struct DotDev {
+  const uint4* words;
+  const int32_t *bottom, *prep, *top, *back;
+  int n_bottom, n_prep, n_top, n_back;
+};
+
 // Progress flags (plans with sync = 1).  A warp that has done its work of
 // the first n levels publishes n: every lane fences its shared and global
 // writes (and the copies it waited for) at CTA scope, the warp meets, and
@@ -1291,6 +1299,7 @@ struct __align__(16) MultiJob {
   SchedDev S;
   BatchDev D;
   StreamDev P;
+  DotDev dot;
   int nw;  // warps of the job's refactor plan
 };
 static_assert(sizeof(MultiJob) % 16 == 0, "jobs are copied as int4");
