@@ -320,7 +320,7 @@ struct DevSchedule {
   struct DotPlanDev {
     bool on = false, with_subst = false;
     int top_warps = 0, bins = 0;
-    DevMem words, bottom, prep, top, back;
+    DevMem words, bottom, prep, top, tback, back;
     DotDev d{};
   } dot[2];
   // the plan's substitutions are part of its refactor
@@ -328,7 +328,7 @@ struct DevSchedule {
   // launches of one refactor (with both substitutions when the plan has them)
   int refactor_launches(int i) const {
     if (dot[i].on)
-      return 1 + (dot[i].d.n_bottom > 0) + (dot[i].d.n_prep > 0) + (dot[i].d.n_back > 0);
+      return 1 + (dot[i].d.n_bottom > 0) + (dot[i].d.n_prep > 0) + (dot[i].d.n_tback > 0) + (dot[i].d.n_back > 0);
     return 1 + st_wl[i] + st_wp[i];
   }
 
@@ -344,15 +344,18 @@ struct DevSchedule {
     upload(x.bottom, p->bottom);
     upload(x.prep, p->prep);
     upload(x.top, p->top);
+    upload(x.tback, p->tback);
     upload(x.back, p->back);
     x.d.words = x.words.as<uint4>();
     x.d.bottom = x.bottom.as<int32_t>();
     x.d.prep = x.prep.as<int32_t>();
     x.d.top = x.top.as<int32_t>();
+    x.d.tback = x.tback.as<int32_t>();
     x.d.back = x.back.as<int32_t>();
     x.d.n_bottom = (int)p->bottom.size();
     x.d.n_prep = (int)p->prep.size();
     x.d.n_top = (int)p->top.size();
+    x.d.n_tback = (int)p->tback.size();
     x.d.n_back = (int)p->back.size();
   }
 
@@ -675,25 +678,28 @@ struct Iter {
     GOX_CK(cudaGetDevice(&dev));
     std::call_once(once[dev & 63], [] {
       const cudaFuncAttribute a = cudaFuncAttributePreferredSharedMemoryCarveout;
-      GOX_CK(cudaFuncSetAttribute(k_dot_bins<T>, a, 20));
+      GOX_CK(cudaFuncSetAttribute(k_dot_bins<T, DOT_BOTTOM>, a, 20));
+      GOX_CK(cudaFuncSetAttribute(k_dot_bins<T, DOT_PREP>, a, 20));
+      GOX_CK(cudaFuncSetAttribute(k_dot_bins<T, DOT_BACK>, a, 20));
       GOX_CK(cudaFuncSetAttribute(k_dot_top<T, 16>, a, 20));
       if constexpr (sizeof(T) == 4) GOX_CK(cudaFuncSetAttribute(k_dot_top<T, 32>, a, 20));
+      GOX_CK(cudaFuncSetAttribute(k_dot_topback<T>, a, 20));
     });
   }
-  static void dot_bins(const DotDev& P, const SchedDev& S, const BatchDev& D, int which, int n, int groups,
-                       cudaStream_t st) {
-    if (n == 0) return;
-    k_dot_bins<T><<<dim3((n + kDotBinWarps - 1) / kDotBinWarps, groups), 32 * kDotBinWarps, 0, st>>>(P, S, D, which);
+  template <int WHICH>
+  static void dot_bins(const DotDev& P, const SchedDev& S, const BatchDev& D, int n, int groups, cudaStream_t st) {
+    if (n > 0) k_dot_bins<T, WHICH><<<dim3(dot_blocks(n), groups), 32 * kDotBinWarps, 0, st>>>(P, S, D);
   }
   static void dot(const DotDev& P, const SchedDev& S, const BatchDev& D, int groups, cudaStream_t st) {
     dot_attr();
-    dot_bins(P, S, D, DOT_BOTTOM, P.n_bottom, groups, st);
-    dot_bins(P, S, D, DOT_PREP, P.n_prep, groups, st);
+    dot_bins<DOT_BOTTOM>(P, S, D, P.n_bottom, groups, st);
+    dot_bins<DOT_PREP>(P, S, D, P.n_prep, groups, st);
     if constexpr (sizeof(T) == 4) {
       if (P.n_top == 32) k_dot_top<T, 32><<<groups, 1024, 0, st>>>(P, S, D);
     }
     if (P.n_top == 16) k_dot_top<T, 16><<<groups, 512, 0, st>>>(P, S, D);
-    dot_bins(P, S, D, DOT_BACK, P.n_back, groups, st);
+    if (P.n_tback > 0) k_dot_topback<T><<<groups, 32 * kDotBackWarps, 0, st>>>(P, S, D);
+    dot_bins<DOT_BACK>(P, S, D, P.n_back, groups, st);
   }
   // shared memory of a wide-kernel CTA whose warps stage `rows` rows
   static size_t wide_smem(int rows) { return (size_t)kWideWarps * rows * 32 * sizeof(T); }
@@ -2248,7 +2254,7 @@ struct MultiLists {
   struct L { size_t off = 0, job = 0; int n = 0, ctas = 0; };
   L upd, inj, dec, fill, rf;
   std::vector<L> wide;  // per wide level
-  L dbins[3], dtop[2];  // dot programs: bottom, prep, back; the top with 16 and 32 warps
+  L dbins[3], dtop[2], dtback;  // dot programs: bottom, prep, back; the top with 16 and 32 warps, its rows
   MultiList view(const L& l) const {
     MultiList m;
     m.off = dev.as<int32_t>() + l.off;
@@ -2298,6 +2304,12 @@ static void build_lists(const std::vector<gox_topo*>& ts, const std::vector<Batc
     if (x.on) top[x.top_warps == 32].push_back(j);
   }
   for (int w = 0; w < 2; w++) M.dtop[w] = add(top[w], [&](int j) { return G(j); });
+  {
+    std::vector<int> jl;
+    for (int j : dots)
+      if (ts[j]->dsched.dot[i].d.n_tback > 0) jl.push_back(j);
+    M.dtback = add(jl, [&](int j) { return G(j); });
+  }
   for (int w : {DOT_BOTTOM, DOT_PREP, DOT_BACK}) {
     auto n = [&](int j) {
       const DotDev& d = ts[j]->dsched.dot[i].d;
@@ -2382,7 +2394,10 @@ static void run_multi(const std::vector<gox_topo*>& ts, std::vector<BatchRun>& r
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)Iter<T>::kWideSmem));
       const cudaFuncAttribute a = cudaFuncAttributePreferredSharedMemoryCarveout;  // as the single kernels
-      GOX_CK(cudaFuncSetAttribute(k_dot_bins_multi<T>, a, 20));
+      GOX_CK(cudaFuncSetAttribute(k_dot_bins_multi<T, DOT_BOTTOM>, a, 20));
+      GOX_CK(cudaFuncSetAttribute(k_dot_bins_multi<T, DOT_PREP>, a, 20));
+      GOX_CK(cudaFuncSetAttribute(k_dot_bins_multi<T, DOT_BACK>, a, 20));
+      GOX_CK(cudaFuncSetAttribute(k_dot_topback_multi<T>, a, 20));
       GOX_CK(cudaFuncSetAttribute(k_dot_top_multi<T, 16>, a, 20));
       if constexpr (sizeof(T) == 4) GOX_CK(cudaFuncSetAttribute(k_dot_top_multi<T, 32>, a, 20));
     });
@@ -2459,17 +2474,19 @@ static void run_multi(const std::vector<gox_topo*>& ts, std::vector<BatchRun>& r
     launch(M.rf, [&](unsigned c, MultiList l) {
       k_refactor_multi<T><<<c, 32 * nw_max, smem_max, st>>>(J, l);
     });
-    auto bins = [&](int w) {
-      launch(M.dbins[w], [&](unsigned c, MultiList l) {
-        k_dot_bins_multi<T><<<c, 32 * kDotBinWarps, 0, st>>>(J, l, w);
-      });
-    };
-    bins(DOT_BOTTOM);
-    bins(DOT_PREP);
+    const unsigned bt = 32 * kDotBinWarps;
+    launch(M.dbins[DOT_BOTTOM],
+           [&](unsigned c, MultiList l) { k_dot_bins_multi<T, DOT_BOTTOM><<<c, bt, 0, st>>>(J, l); });
+    launch(M.dbins[DOT_PREP],
+           [&](unsigned c, MultiList l) { k_dot_bins_multi<T, DOT_PREP><<<c, bt, 0, st>>>(J, l); });
     if constexpr (sizeof(T) == 4)
       launch(M.dtop[1], [&](unsigned c, MultiList l) { k_dot_top_multi<T, 32><<<c, 1024, 0, st>>>(J, l); });
     launch(M.dtop[0], [&](unsigned c, MultiList l) { k_dot_top_multi<T, 16><<<c, 512, 0, st>>>(J, l); });
-    bins(DOT_BACK);
+    launch(M.dtback, [&](unsigned c, MultiList l) {
+      k_dot_topback_multi<T><<<c, 32 * kDotBackWarps, 0, st>>>(J, l);
+    });
+    launch(M.dbins[DOT_BACK],
+           [&](unsigned c, MultiList l) { k_dot_bins_multi<T, DOT_BACK><<<c, bt, 0, st>>>(J, l); });
     rec();
     for (size_t L = M.wide.size(); L-- > 0;)
       launch(M.wide[L], [&](unsigned c, MultiList l) {

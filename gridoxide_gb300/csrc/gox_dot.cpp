@@ -97,6 +97,66 @@ struct Writer {
     } while (n > 0);
     return units;
   }
+  // four sums of m products each (the last ones repeated to make four: the
+  // same sum twice stores the same value twice)
+  struct Sum { int32_t v, t0; };
+  void pack(const Sums& S, const Sum* x, int cnt, int m, bool row, bool first, int ns) {
+    flush();
+    room(2 + 2 * m);
+    last = w.size();
+    raw(DOT_PACK | (row ? DOT_ROW : 0u) | (first ? DOT_FIRST : 0u) | ((uint32_t)m << 12), 0u, 0u, 0u);
+    auto at = [&](int i) { return x[std::min(i, cnt - 1)]; };
+    auto val = [&](int i) { return (uint32_t)(row ? at(i).v - ns : at(i).v); };
+    raw(val(0), val(1), val(2), val(3));
+    for (int t = 0; t < m; t++) {
+      auto a = [&](int i) { return (uint32_t)S.a[at(i).t0 + t]; };
+      auto b = [&](int i) { return (uint32_t)S.b[at(i).t0 + t]; };
+      raw(a(0), a(1), a(2), a(3));
+      raw(b(0), b(1), b(2), b(3));
+    }
+  }
+  // backward rows in a row, in one chunk each
+  void chain(const Schedule& sc, const std::vector<int32_t>& rows) {
+    flush();
+    for (size_t i = 0; i < rows.size();) {
+      size_t e = i;
+      int q = 1;
+      auto quads = [&](int k) { return 1 + (sc.bw_ptr[k + 1] - sc.bw_ptr[k] + 1) / 2; };
+      while (e < rows.size() && q + quads(rows[e]) < kDotChunk) q += quads(rows[e++]);
+      // (a chunk has room for 5 rows at least; what is left of one is used when
+      // it holds a row or two more)
+      const int left = kDotChunk - 1 - (int)(w.size() / 4) % kDotChunk;
+      if (q > left) {
+        size_t f = i;
+        int z = 1;
+        while (f < rows.size() && z + quads(rows[f]) <= left) z += quads(rows[f++]);
+        if (f >= i + 2) {
+          e = f;
+          q = z;
+        }
+      }
+      room(q);
+      last = w.size();
+      raw(DOT_CHAIN, (uint32_t)(e - i), 0u, 0u);
+      for (size_t r = i; r < e; r++) {
+        const int k = rows[r], t0 = sc.bw_ptr[k], n = sc.bw_ptr[k + 1] - t0;
+        const bool next = r > i && n > 0 && sc.bw_col[t0] == rows[r - 1];
+        raw((uint32_t)k, (uint32_t)sc.diag_slot[k], (uint32_t)n | (next ? DOT_NEXT : 0u), 0u);
+        for (int t = 0; t < n; t += 2) {
+          const int u = t + 1 < n ? t + 1 : t;
+          raw((uint32_t)sc.bw_slot[t0 + t], (uint32_t)sc.bw_col[t0 + t], (uint32_t)sc.bw_slot[t0 + u],
+              (uint32_t)sc.bw_col[t0 + u]);
+        }
+      }
+      i = e;
+    }
+  }
+  void fin(int diag, int ll) {
+    flush();
+    room(1);
+    last = w.size();
+    raw(DOT_FIN, (uint32_t)diag, (uint32_t)ll, 0u);
+  }
   // LU slots and rows, up to 40 of each
   void touch(const std::vector<int32_t>& lu, const std::vector<int32_t>& x) {
     if (lu.empty() && x.empty()) return;
@@ -147,6 +207,7 @@ static int top_warps(int elem) { return elem == 4 ? 32 : 16; }
 DotPlan dot_default(const Schedule& sc, int elem, int groups) {
   DotPlan p;
   p.top_warps = top_warps(elem);
+  p.chain = dot_chain_terms(elem);
   const int per = groups >= 32 ? 32 : 16;  // unknowns per bin
   while (sc.n_u >= 400 && p.bins < 512 && p.bins * per < sc.n_u) p.bins = p.bins ? 2 * p.bins : 32;
   return p;
@@ -162,6 +223,7 @@ std::vector<DotPlan> dot_candidates(const Schedule& sc, int elem) {
       DotPlan p;
       p.bins = bins;
       p.top_warps = w;
+      p.chain = dot_chain_terms(elem);
       out.push_back(p);
     }
   }
@@ -247,45 +309,114 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
     P.units += W.sum(op | (y && t0 == S.ptr[v] ? DOT_FIRST : 0u), (uint32_t)(y ? v - ns : v), z, S.a.data() + t0,
                      S.b.data() + t0, t1 - t0);
   };
-  for (int b = 0; b < plan.bins; b++) {
-    if (bin[b].empty()) continue;
-    Writer W;
-    for (int k : bin[b]) {
-      const int base = sc.c_base[k], ul = sc.c_ulen[k];
-      for (int d = 0; d < len(k); d++) {
-        const int v = base + d;
-        if (d < ul && nt(v) == 0) continue;
-        emit_sum(W, d < ul ? DOT_U : d == ul ? DOT_D : DOT_L, v, 0, S.ptr[v], S.ptr[v + 1]);
-        taken[v] = nt(v);
-      }
-      if (subst) {
-        emit_sum(W, DOT_Y, ns + k, 0, S.ptr[ns + k], S.ptr[ns + k + 1]);
-        taken[ns + k] = nt(ns + k);
-      }
+  // independent sums of one warp (products [t0, t1) of value v): the short ones
+  // by fours, those of one length together, the long ones one by one
+  struct Part { int32_t v, t0, t1; };
+  auto emit_group = [&](Writer& W, const std::vector<Part>& g) {
+    std::vector<Writer::Sum> by[3][4];  // LU, y, y from its start; by length
+    for (const Part& x : g) {
+      const int m = x.t1 - x.t0, kind = x.v < ns ? 0 : x.t0 == S.ptr[x.v] ? 2 : 1;
+      if (m == 0 && kind < 2) continue;
+      if (m > plan.pack) emit_sum(W, x.v >= ns ? DOT_Y : DOT_U, x.v, 0, x.t0, x.t1);
+      else by[kind][m].push_back({x.v, x.t0});
     }
-    append(P, P.bottom, W);
+    for (int kind = 0; kind < 3; kind++)
+      for (int m = 0; m < 4; m++) {
+        const auto& l = by[kind][m];
+        for (size_t i = 0; i < l.size(); i += 4) {
+          const int cnt = (int)std::min<size_t>(4, l.size() - i);
+          if (cnt == 1) {
+            emit_sum(W, kind ? DOT_Y : DOT_U, l[i].v, 0, l[i].t0, l[i].t0 + m);
+          } else {
+            W.pack(S, &l[i], cnt, m, kind > 0, kind == 2, ns);
+            P.units++;
+          }
+        }
+      }
+  };
+  // a bin's sums by their depth in it (a column's L entries are final one
+  // deeper than its deepest sum): those of one depth are independent
+  {
+    std::vector<int32_t> depth(ns + n, 0);
+    std::vector<std::vector<Part>> at;
+    std::vector<std::vector<int32_t>> fins;
+    for (int b = 0; b < plan.bins; b++) {
+      if (bin[b].empty()) continue;
+      at.clear();
+      fins.clear();
+      auto grow = [&](int d) {
+        if ((int)at.size() <= d) {
+          at.resize(d + 1);
+          fins.resize(d + 1);
+        }
+      };
+      auto sum_depth = [&](int v) {
+        int d = 0;
+        for (int e = S.ptr[v]; e < S.ptr[v + 1]; e++)
+          d = std::max({d, depth[S.a[e]], depth[v >= ns ? ns + S.b[e] : S.b[e]]});
+        grow(d);
+        at[d].push_back({v, S.ptr[v], S.ptr[v + 1]});
+        taken[v] = nt(v);
+        return d + 1;  // what reads it comes after
+      };
+      for (int k : bin[b]) {
+        const int base = sc.c_base[k], ul = sc.c_ulen[k];
+        int f = 0;
+        for (int v = base; v < base + len(k); v++) {
+          depth[v] = nt(v) ? sum_depth(v) : 0;
+          if (v >= base + ul) f = std::max(f, depth[v]);
+        }
+        grow(f);
+        fins[f].push_back(k);
+        for (int v = base + ul; v < base + len(k); v++) depth[v] = f + 1;
+        if (subst) depth[ns + k] = sum_depth(ns + k);
+      }
+      Writer W;
+      for (size_t d = 0; d < at.size(); d++) {
+        emit_group(W, at[d]);
+        for (int k : fins[d]) {
+          W.fin(sc.diag_slot[k], sc.c_llen[k]);
+          P.units++;
+        }
+      }
+      append(P, P.bottom, W);
+    }
   }
   // ---- prep: per top column, the leading products of each sum whose values
   // the bottom (or the prep of this same column) finishes
   if (P.bottom_cols > 0) {
+    std::vector<int32_t> prep_depth(ns + n, 0);
+    std::vector<std::vector<Part>> at;  // the stream's sums, by depth among its columns' U entries
+    int left_cols = n - (int)P.bottom_cols, in_stream = 0;
+    // (two columns fill the packs better; four leave too few warps in flight:
+    // 2,000 buses, 256 bins, 128 groups FP32 0.305 / 0.276 / 0.285 ms for 1 / 2 / 4)
+    const int per_stream = left_cols >= 256 ? 2 : 1;
     for (int k = 0; k < n; k++) {
       if (part[k] >= 0) continue;
-      Writer W;
       const int base = sc.c_base[k];
       auto prefix = [&](int v) {
-        int t = S.ptr[v];
+        int t = S.ptr[v], d = 0;
         for (; t < S.ptr[v + 1]; t++) {
           if (part[S.col[S.a[t]]] < 0) break;  // an L value of a top column
           if (v >= ns ? part[S.b[t]] < 0 : taken[S.b[t]] != nt(S.b[t])) break;
+          if (v < ns) d = std::max(d, prep_depth[S.b[t]]);
         }
         if (t == S.ptr[v]) return;
-        emit_sum(W, v >= ns ? DOT_Y : DOT_U, v, 0, S.ptr[v], t);
+        if ((int)at.size() <= d) at.resize(d + 1);
+        at[d].push_back({v, S.ptr[v], t});
+        prep_depth[v] = d + 1;
         taken[v] = t - S.ptr[v];
         P.prep_terms += taken[v];
       };
       for (int d = 0; d < len(k); d++) prefix(base + d);
       if (subst) prefix(ns + k);
-      if (!W.w.empty()) append(P, P.prep, W);
+      left_cols--;
+      if ((++in_stream < per_stream && left_cols > 0) || at.empty()) continue;
+      Writer W;
+      for (auto& g : at) emit_group(W, g);
+      append(P, P.prep, W);
+      at.clear();
+      in_stream = 0;
     }
   }
 
@@ -331,7 +462,7 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
   };
   // a long sum whose last products come late: its leading ones run as parts in
   // earlier ticks, so the tick that finishes it has few left
-  constexpr int kPartMin = 5, kPartMax = 16;
+  constexpr int kPartMin = 3, kPartMax = 8;
   auto split = [&](int v, int final_tick) {
     int t = S.ptr[v] + taken[v];
     const int t1 = S.ptr[v + 1];
@@ -414,8 +545,8 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
 
   // what each tick's warps do (the backward rows' ticks included)
   struct Do { int32_t w; uint32_t op; int32_t v; uint32_t z; int32_t t0, t1; };
-  std::vector<std::vector<Do>> plan_of;
-  std::vector<std::vector<double>> load_of;
+  std::vector<std::vector<Do>> plan_of, back_of;
+  std::vector<std::vector<double>> load_of, back_load;
   int tick = 0;
   auto emit = [&](int w, uint32_t op, int v, uint32_t z, int t0, int t1) {
     P.top_terms += t1 - t0;
@@ -486,9 +617,10 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
         const int w = least();
         for (int e = 0; e <= ll; e++) {
           const int v = base + ul + e;
-          emit(w, e ? DOT_L : DOT_D, v, 0, from[v], S.ptr[v + 1]);
+          if (left(v)) emit(w, DOT_U, v, 0, from[v], S.ptr[v + 1]);
           load[w] += sum_cost(left(v));
         }
+        plan_of.back().push_back({w, DOT_FIN, k, 0u, 0, 0});
       }
       std::stable_sort(others.begin(), others.end(), [&](int x, int y) { return nodes[x].cost > nodes[y].cost; });
       for (int i : others) {
@@ -526,18 +658,56 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
       if ((int)bylev.size() <= l) bylev.resize(l + 1);
       bylev[l].push_back(k);
     }
-    P.back_ticks = (int)bylev.size();
-    int turn = 0;
+    // levels of a row or two, one after the other, are one warp's chain and one
+    // tick's: what a row reads of the one before is in a register (its first
+    // product), of those before that the warp's own, and no barrier lies
+    // between them
+    constexpr int kChainRows = 16;
+    std::vector<std::vector<int32_t>> ticks_of;
+    std::vector<char> chained;
+    auto fits = [&](int prev, int k) {
+      const int t0 = sc.bw_ptr[k], m = sc.bw_ptr[k + 1] - t0;
+      if (m > plan.chain) return false;
+      for (int t = 1; t < m; t++)
+        if (sc.bw_col[t0 + t] == prev) return false;
+      return true;
+    };
     for (auto& rows : bylev) {
-      std::vector<double> load(NT, 0.0);
-      plan_of.emplace_back();
+      bool ok = rows.size() <= 2;
+      int prev = !chained.empty() && chained.back() ? ticks_of.back().back() : -1;
       for (int k : rows) {
-        const int w = rows.size() <= (size_t)NT ? turn++ % NT
+        ok = ok && fits(prev, k);
+        prev = k;
+      }
+      if (ok && !chained.empty() && chained.back() && ticks_of.back().size() + rows.size() <= (size_t)kChainRows) {
+        ticks_of.back().insert(ticks_of.back().end(), rows.begin(), rows.end());
+      } else {
+        chained.push_back(ok);
+        ticks_of.push_back(rows);
+      }
+    }
+    P.back_ticks = (int)ticks_of.size();
+    int turn = 0;
+    for (size_t t = 0; t < ticks_of.size(); t++) {
+      const std::vector<int32_t>& rows = ticks_of[t];
+      if (chained[t]) {
+        std::vector<double> load(kDotBackWarps, 0.0);
+        back_of.emplace_back();
+        const int w = turn++ % kDotBackWarps;
+        for (int k : rows) back_of.back().push_back({w, DOT_CHAIN, ns + k, 0u, 0, 0});
+        load[w] = 1e6;
+        back_load.push_back(load);
+        continue;
+      }
+      std::vector<double> load(kDotBackWarps, 0.0);
+      back_of.emplace_back();
+      for (int k : rows) {
+        const int w = rows.size() <= (size_t)kDotBackWarps ? turn++ % kDotBackWarps
                                                 : (int)(std::min_element(load.begin(), load.end()) - load.begin());
         load[w] += sum_cost(sc.bw_ptr[k + 1] - sc.bw_ptr[k]);
-        plan_of.back().push_back({w, DOT_B, ns + k, 0u, 0, 0});
+        back_of.back().push_back({w, DOT_B, ns + k, 0u, 0, 0});
       }
-      load_of.push_back(load);
+      back_load.push_back(load);
     }
     for (int b = 0; b < plan.bins; b++) {
       if (bin[b].empty()) continue;
@@ -550,7 +720,8 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
   // the L1 is touched `ahead` ticks before the tick that needs it, by the
   // warps with the least to do there (not for ticks that fill all warps: they
   // hide their loads behind each other)
-  {
+  auto streams = [&](const std::vector<std::vector<Do>>& plan_of, std::vector<std::vector<double>>& load_of, int NT,
+                     std::vector<int32_t>& out) {
     const int nticks = (int)plan_of.size();
     std::vector<std::vector<std::pair<std::vector<int32_t>, std::vector<int32_t>>>> touch(nticks);  // per tick and warp
     if (plan.ahead > 0) {
@@ -564,8 +735,12 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
           last[v] = now++;
         };
         for (const Do& d : plan_of[t]) {
+          if (d.op == DOT_FIN) {
+            for (int v = sc.diag_slot[d.v]; v <= sc.diag_slot[d.v] + sc.c_llen[d.v]; v++) use(v);
+            continue;
+          }
           use(d.v);
-          if (d.op == DOT_B) {
+          if (d.op == DOT_B || d.op == DOT_CHAIN) {
             const int k = d.v - ns;
             use(sc.diag_slot[k]);
             for (int e = sc.bw_ptr[k]; e < sc.bw_ptr[k + 1]; e++) {
@@ -594,10 +769,26 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
     }
     std::vector<Writer> W(NT);
     for (int t = 0; t < nticks; t++) {
+      // per warp: split columns' entries first, then the independent sums, then
+      // the columns they finish
+      std::vector<std::vector<Part>> group(NT);
       for (const Do& d : plan_of[t]) {
         if (d.op == DOT_B) row(W[d.w], d.v - ns);
-        else emit_sum(W[d.w], d.op, d.v, d.z, d.t0, d.t1);
+        else if (d.op == DOT_CHAIN) continue;
+        else if ((d.op & 15u) == DOT_D || (d.op & 15u) == DOT_LH) emit_sum(W[d.w], d.op, d.v, d.z, d.t0, d.t1);
+        else if (d.op != DOT_FIN) group[d.w].push_back({d.v, d.t0, d.t1});
       }
+      if (!plan_of[t].empty() && plan_of[t][0].op == DOT_CHAIN) {
+        std::vector<int32_t> rows;
+        for (const Do& d : plan_of[t]) rows.push_back(d.v - ns);
+        W[plan_of[t][0].w].chain(sc, rows);
+      }
+      for (int w = 0; w < NT; w++) emit_group(W[w], group[w]);
+      for (const Do& d : plan_of[t])
+        if (d.op == DOT_FIN) {
+          W[d.w].fin(sc.diag_slot[d.v], sc.c_llen[d.v]);
+          P.units++;
+        }
       if (!touch[t].empty())
         for (int w = 0; w < NT; w++) {
           auto& x = touch[t][w];
@@ -608,10 +799,13 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
             W[w].touch(cut(x.first), cut(x.second));
           }
         }
-      for (auto& w : W) w.bar();
+      if (t + 1 < nticks)
+        for (auto& w : W) w.bar();
     }
-    for (auto& w : W) append(P, P.top, w);
-  }
+    for (auto& w : W) append(P, out, w);
+  };
+  streams(plan_of, load_of, NT, P.top);
+  if (subst) streams(back_of, back_load, kDotBackWarps, P.tback);
 }
 
 std::string run_dot_host(const Schedule& sc, const DotProgram& P, std::vector<double>& lu,
@@ -634,6 +828,7 @@ std::string run_dot_host(const Schedule& sc, const DotProgram& P, std::vector<do
   std::string err;
   const size_t nq = P.words.size() / 4;
   int64_t tick = 0;
+  uint32_t may = 0;  // the units the running launch has code for
   auto fail = [&](const char* s) {
     if (err.empty()) err = s;
     return false;
@@ -656,8 +851,8 @@ std::string run_dot_host(const Schedule& sc, const DotProgram& P, std::vector<do
     size_t pos;
     int bars = 0;
     bool ended = false, waits = false;  // waits: at a mid barrier
-    double inv = 0, car = 0;
-    int pivot = -1, carried = -1;       // slot of the warp's last D, value of the open sum
+    double car = 0;
+    int carried = -1;                   // value of the open sum
   };
   std::vector<std::pair<uint32_t, double>> mid_inv;  // mid barriers reached by their pivot's warp
   std::vector<Held> held;
@@ -668,6 +863,7 @@ std::string run_dot_host(const Schedule& sc, const DotProgram& P, std::vector<do
       if (A.pos >= nq) return fail("a stream runs past the program");
       const uint32_t* h = &P.words[A.pos * 4];
       const uint32_t op = h[0] & 15u;
+      if (!((may >> op) & 1u)) return fail("a unit in the wrong launch");
       if (op == DOT_END) {
         A.ended = true;
         return A.carried < 0 || fail("a sum left open");
@@ -687,6 +883,111 @@ std::string run_dot_host(const Schedule& sc, const DotProgram& P, std::vector<do
         for (size_t i = 0; i < 4 * nt; i++)
           if (h[4 + i] >= (uint32_t)(i < 4 * (size_t)h[1] ? ns : n)) return fail("a touched value out of range");
         A.pos += 1 + nt;
+        continue;
+      }
+      if (op == DOT_PACK) {
+        const int m = (int)((h[0] >> 12) & 15u);
+        const bool row = (h[0] & DOT_ROW) != 0, first = (h[0] & DOT_FIRST) != 0;
+        if (m > 3 || (first && !row)) return fail("a pack out of range");
+        if (A.pos % kDotChunk + 2 + 2 * m + 1 > (size_t)kDotChunk || A.pos + 2 + 2 * m > nq)
+          return fail("a unit that leaves its chunk");
+        if (A.carried >= 0) return fail("a sum left open");
+        double out[4];
+        for (int i = 0; i < 4; i++) {
+          if (h[4 + i] >= (uint32_t)(row ? n : ns)) return fail("a value out of range");
+          const int v = row ? ns + (int)h[4 + i] : (int)h[4 + i];
+          bool again = false;
+          for (int q = 0; q < i; q++)
+            if (h[4 + q] == h[4 + i]) {
+              again = true;
+              for (int t = 0; t < 2 * m; t++)
+                if (h[8 + 4 * t + q] != h[8 + 4 * t + i]) return fail("a repeated sum with other products");
+            }
+          if (again) continue;
+          if (fin[v]) return fail("a final value written again");
+          if (row && first != (taken[v] == 0)) return fail("a sum that starts twice or not at all");
+          if (!first && !read(v, w)) return false;
+          double s = first ? rhs[h[4 + i]] : row ? X[h[4 + i]] : lu[v];
+          for (int t = 0; t < m; t++) {
+            const uint32_t a = h[8 + 8 * t + i], b = h[12 + 8 * t + i];
+            if (a >= (uint32_t)ns || b >= (uint32_t)(row ? n : ns)) return fail("a product out of range");
+            const int vb = row ? ns + (int)b : (int)b, e = S.ptr[v] + taken[v]++;
+            if (!read((int)a, w) || !read(vb, w)) return false;
+            if (e >= S.ptr[v + 1] || S.a[e] != (int)a || S.b[e] != (int)b) return fail("a product out of order");
+            if (!fin[a] || !fin[vb]) return fail("a product before its value is final");
+            s -= lu[a] * (row ? X[b] : lu[b]);
+          }
+          out[i] = s;
+        }
+        for (int i = 0; i < 4; i++) {
+          const int v = row ? ns + (int)h[4 + i] : (int)h[4 + i];
+          bool again = false;
+          for (int q = 0; q < i; q++) again |= h[4 + q] == h[4 + i];
+          if (again) continue;
+          if (!write(v, w)) return false;
+          (row ? X[h[4 + i]] : lu[v]) = out[i];
+          if ((row || v < sc.diag_slot[S.col[v]]) && taken[v] == S.ptr[v + 1] - S.ptr[v]) fin[v] = 1;
+        }
+        A.pos += 2 + 2 * m;
+      } else if (op == DOT_FIN) {
+        const int d = (int)h[1];
+        if (h[1] >= (uint32_t)ns || d != sc.diag_slot[S.col[d]] || (int)h[2] != sc.c_llen[S.col[d]])
+          return fail("a column out of range");
+        for (int v = d; v <= d + (int)h[2]; v++) {
+          if (fin[v] || taken[v] != S.ptr[v + 1] - S.ptr[v]) return fail("a column finished before its sums");
+          if (!read(v, w) || !write(v, w)) return false;
+          fin[v] = 1;
+        }
+        if (lu[d] == 0) singular = true;
+        const double inv = 1.0 / lu[d];
+        for (int v = d + 1; v <= d + (int)h[2]; v++) lu[v] = lu[v] * inv;
+        A.pos++;
+      }
+      if (op == DOT_CHAIN) {
+        if (A.carried >= 0) return fail("a sum left open");
+        size_t q = A.pos + 1;
+        int prev = -1;
+        for (uint32_t r = 0; r < h[1]; r++) {
+          if (q >= nq || q / kDotChunk != A.pos / kDotChunk) return fail("a unit that leaves its chunk");
+          const uint32_t* x = &P.words[q * 4];
+          const int m = (int)(x[2] & 0xffffu);
+          if (x[0] >= (uint32_t)n || m > P.plan.chain) return fail("a chain's row out of range");
+          const int k = (int)x[0], v = ns + k;
+          if (!fin[v] || !read(v, w)) return fail("x before y is final");
+          if (x[1] != (uint32_t)sc.diag_slot[k] || !fin[x[1]] || !read((int)x[1], w))
+            return fail("a backward row with another pivot");
+          if (m != sc.bw_ptr[k + 1] - sc.bw_ptr[k]) return fail("an incomplete backward row");
+          if (q + 1 + (m + 1) / 2 > nq || (q + (m + 1) / 2) / kDotChunk != A.pos / kDotChunk)
+            return fail("a unit that leaves its chunk");
+          double s = X[k];
+          for (int t = 0; t < m; t++) {
+            const uint32_t* y = x + 4 + 4 * (t / 2) + 2 * (t & 1);
+            const int e = sc.bw_ptr[k] + t;
+            if ((uint32_t)sc.bw_slot[e] != y[0] || (uint32_t)sc.bw_col[e] != y[1]) return fail("a backward term out of order");
+            if (!fin[y[0]] || !xdone[y[1]]) return fail("a backward term before its x");
+            if (!read((int)y[0], w) || !read(ns + (int)y[1], w)) return false;
+            // the loads of a row are issued before the row before it is stored
+            const bool next = t == 0 && (x[2] & DOT_NEXT);
+            if (next != ((int)y[1] == prev)) return fail("a chain's row that misses the one before it");
+            s -= lu[y[0]] * X[y[1]];
+          }
+          const double xx = s / lu[x[1]];
+          if (!std::isfinite(xx)) singular = true;
+          if (!write(v, w)) return false;
+          X[k] = xx;
+          xdone[k] = 1;
+          prev = k;
+          q += 1 + (m + 1) / 2;
+        }
+        if (q % kDotChunk == 0) return fail("a unit that leaves its chunk");
+        A.pos = q;
+      }
+      if (op == DOT_PACK || op == DOT_FIN || op == DOT_CHAIN) {
+        if (h[0] & DOT_BARF) {
+          if (!top) return fail("a bin with a barrier");
+          A.bars = 1;
+          return true;
+        }
         continue;
       }
       const int m = (int)((h[0] >> 12) & 15u);
@@ -758,22 +1059,15 @@ std::string run_dot_host(const Schedule& sc, const DotProgram& P, std::vector<do
         lu[v] = s;
         fin[v] = 1;
         if (s == 0) singular = true;
-        A.inv = 1.0 / s;
-        A.pivot = v;
         const uint32_t id = (h[0] >> 8) & 15u;
-        if (id && (!top || id > (uint32_t)kDotMaxMid || (h[2] >> 16) >= (uint32_t)kDotMaxMid))
+        if (id == 0 || !top || id > (uint32_t)kDotMaxMid || (h[2] >> 16) >= (uint32_t)kDotMaxMid)
           return fail("a mid barrier out of range");
-        if (id) mid_inv.push_back({id, A.inv});
-      } else if (op == DOT_L || op == DOT_LH) {
+        mid_inv.push_back({id, 1.0 / s});
+      } else if (op == DOT_LH) {
         if (!whole || v <= sc.diag_slot[k]) return fail("an incomplete L entry");
-        if (op == DOT_L) {
-          if (A.pivot != sc.diag_slot[k]) return fail("an L entry without its pivot");
-        } else {
-          if (!fin[sc.diag_slot[k]] || wtick[sc.diag_slot[k]] != tick) return fail("an L entry of another column's pivot");
-          held.push_back({h[2], (h[0] >> 8) & 15u});
-          A.pivot = -1;
-        }
-        lu[v] = s * (op == DOT_L ? A.inv : mid);
+        if (!fin[sc.diag_slot[k]] || wtick[sc.diag_slot[k]] != tick) return fail("an L entry of another column's pivot");
+        held.push_back({h[2], (h[0] >> 8) & 15u});
+        lu[v] = s * mid;
         fin[v] = 1;
       } else {
         if (taken[v] != sc.bw_ptr[h[1] + 1] - sc.bw_ptr[h[1]]) return fail("an incomplete backward row");
@@ -789,8 +1083,11 @@ std::string run_dot_host(const Schedule& sc, const DotProgram& P, std::vector<do
       }
     }
   };
-  auto launch = [&](const std::vector<int32_t>& st, auto&& run) {
+  constexpr uint32_t kAny = 1u << DOT_END | 1u << DOT_SKIP, kTick = kAny | 1u << DOT_BAR | 1u << DOT_TOUCH,
+                     kSums = 1u << DOT_PACK | 1u << DOT_FIN | 1u << DOT_U | 1u << DOT_Y;
+  auto launch = [&](const std::vector<int32_t>& st, uint32_t units, auto&& run) {
     int w = 0;
+    may = units;
     for (int32_t s : st)
       if (s < 0 || (size_t)s >= nq || !run(s, w++)) return false;
     tick++;
@@ -800,48 +1097,59 @@ std::string run_dot_host(const Schedule& sc, const DotProgram& P, std::vector<do
     Warp B{(size_t)s};
     return step(B, w, false) && (B.ended || fail("a bin that does not end"));
   };
-  if (!launch(P.bottom, bin) || !launch(P.prep, bin)) return err;
-  const int NT = (int)P.top.size();
-  std::vector<Warp> A;
-  for (int32_t s : P.top) A.push_back({(size_t)s});
-  for (int ended = 0; ended < NT;) {
-    held.clear();
-    mid_inv.clear();
-    ended = 0;
-    // every warp to its barrier; one that waits at a mid barrier goes on when
-    // the pivot's warp has arrived there
-    std::vector<char> run(NT, 1);
-    for (bool moved = true; moved;) {
-      moved = false;
-      for (int w = 0; w < NT; w++) {
-        if (!run[w] || A[w].ended) continue;
-        const size_t at = A[w].pos;
-        const bool waited = A[w].waits;
-        if (!step(A[w], w, true)) return err;
-        run[w] = A[w].waits;
-        moved |= !A[w].waits || A[w].pos != at || !waited;
+  if (!launch(P.bottom, kAny | kSums, bin) || !launch(P.prep, kAny | kSums, bin)) return err;
+  // the top's warps, tick by tick
+  auto ticks = [&](const std::vector<int32_t>& st, uint32_t units) -> bool {
+    may = units;
+    const int NT = (int)st.size();
+    std::vector<Warp> A;
+    for (int32_t s : st) {
+      if (s < 0 || (size_t)s >= nq) return fail("a stream out of range");
+      A.push_back({(size_t)s});
+    }
+    for (int ended = 0; ended < NT;) {
+      held.clear();
+      mid_inv.clear();
+      ended = 0;
+      // every warp to its barrier; one that waits at a mid barrier goes on when
+      // the pivot's warp has arrived there
+      std::vector<char> run(NT, 1);
+      for (bool moved = true; moved;) {
+        moved = false;
+        for (int w = 0; w < NT; w++) {
+          if (!run[w] || A[w].ended) continue;
+          const size_t at = A[w].pos;
+          const bool waited = A[w].waits;
+          if (!step(A[w], w, true)) return false;
+          run[w] = A[w].waits;
+          moved |= !A[w].waits || A[w].pos != at || !waited;
+        }
       }
+      for (int w = 0; w < NT; w++) {
+        if (A[w].waits) return fail("a mid barrier that nobody reaches");
+        ended += A[w].ended;
+      }
+      for (auto& m : mid_inv) {
+        int cnt = 0;
+        for (auto& m2 : mid_inv) cnt += m2.first == m.first;
+        uint32_t same = 1;
+        for (auto& x : held) same += x.id == m.first;
+        if (cnt != 1 || same < 2) return fail("a mid barrier used twice in one tick, or by nobody");
+      }
+      for (auto& x : held) {
+        uint32_t same = 1;
+        for (auto& y : held) same += y.id == x.id;
+        if ((x.z & 0xffffu) != 32u * same) return fail("a held L entry without its mid barrier");
+      }
+      if (ended != 0 && ended != NT) return fail("the warps take different numbers of barriers");
+      tick++;
     }
-    for (int w = 0; w < NT; w++) {
-      if (A[w].waits) return "a mid barrier that nobody reaches";
-      ended += A[w].ended;
-    }
-    for (auto& m : mid_inv) {
-      int cnt = 0;
-      for (auto& m2 : mid_inv) cnt += m2.first == m.first;
-      uint32_t same = 1;
-      for (auto& x : held) same += x.id == m.first;
-      if (cnt != 1 || same < 2) return "a mid barrier used twice in one tick, or by nobody";
-    }
-    for (auto& x : held) {
-      uint32_t same = 1;
-      for (auto& y : held) same += y.id == x.id;
-      if ((x.z & 0xffffu) != 32u * same) return "a held L entry without its mid barrier";
-    }
-    if (ended != 0 && ended != NT) return "the warps take different numbers of barriers";
-    tick++;
-  }
-  if (!launch(P.back, bin)) return err;
+    return true;
+  };
+  if (!ticks(P.top, kTick | kSums | 1u << DOT_D | 1u << DOT_LH) ||
+      !ticks(P.tback, kTick | 1u << DOT_B | 1u << DOT_CHAIN))
+    return err;
+  if (!launch(P.back, kAny | 1u << DOT_B, bin)) return err;
   for (int v = 0; v < ns + n; v++)
     if (!fin[v]) return "a value is left unfinished";
   if (P.with_subst)

@@ -8,17 +8,16 @@
 // values, and a sum in pieces, as long as each value's own products stay in
 // order: the result is the stream form's (gox_stream.hpp) bit for bit.
 //
-// Four launches run a refactor with both substitutions:
+// Five launches run a refactor with both substitutions:
 //   bottom    columns in independent parts of the elimination forest, whole
-//             parts assigned to bins; one warp runs a bin's columns in order
-//             (no barrier: it wrote every value it reads), a column at a time
-//             in its warp's shared memory
-//   prep      one warp per remaining column: the leading part of each of its
-//             sums that only needs bottom columns
+//             parts assigned to bins; one warp runs a bin's sums in order and
+//             needs no barrier, since it wrote every value it reads
+//   prep      one warp per remaining column or two: the leading part of each
+//             of its sums that only needs bottom columns
 //   top       the rest of those columns, one CTA per group: the sums as
 //             units of up to 8 products spread over the warps, in ticks that
-//             only read values of earlier ticks, with a CTA barrier after
-//             each; then their backward rows
+//             only read values of earlier ticks, with a CTA barrier after each
+//   top back  their backward rows, one CTA per group, in ticks too
 //   back      the backward rows of the bottom columns, bin by bin
 #pragma once
 #include <cstdint>
@@ -33,9 +32,9 @@ namespace gox {
 // quad, then its products (a, b), two per quad, all in one chunk:
 //   x = op | barrier after << 4 | first << 5 | carry in << 6 | carry out << 7 |
 //       mid << 8 | n << 12
-//   y = the value's slot (U, D, L, LH) or row (Y, B); BAR: how many
+//   y = the value's slot (U, D, LH) or row (Y, B); BAR: how many
 //   z = D, LH: threads of the mid barrier | shared index << 16;  B: pivot slot
-// a and b are LU slots (U, D, L, LH), or an LU slot and a row (Y, B).  A sum of
+// a and b are LU slots (U, D, LH), or an LU slot and a row (Y, B).  A sum of
 // more than 8 products is carried from unit to unit in a register.
 enum : uint32_t {
   DOT_END = 0,
@@ -43,16 +42,25 @@ enum : uint32_t {
   DOT_SKIP = 2,  // on to the next chunk
   DOT_TOUCH = 3, // y quads of LU slots, then z quads of rows: values a later
                  // unit needs, loaded into the SM's L1 and dropped
-  DOT_U = 4,     // U(j, k), or a leading part of any LU entry's sum
-  DOT_D = 5,     // pivot: also its reciprocal, for the warp's next L units; with
-                 // a mid barrier also to shared memory, for the LH units
-  DOT_L = 6,     // L(i, k): times the reciprocal of the warp's last D
-  DOT_LH = 7,    // L(i, k): its sum first, then the mid barrier, then scaled
-  DOT_Y = 8,     // y_k (first: starts from the right-hand side, else from y)
-  DOT_B = 9      // x_k
+  DOT_PACK = 4,  // four U or (DOT_ROW) Y sums of n <= 3 products each: one quad of
+                 // values, then per product a quad of a's and one of b's
+  DOT_FIN = 5,   // a column's pivot in slot y and the z L entries after it, all
+                 // sums done: reciprocal, L entries scaled
+  DOT_CHAIN = 6, // y backward rows, one after the other: per row a quad k, pivot
+                 // slot, n | DOT_NEXT, 0, then its products; DOT_NEXT: the first
+                 // one's x is the row before's
+  DOT_U = 7,     // U(j, k), or a leading part of any LU entry's sum
+  DOT_D = 8,     // pivot: its reciprocal to shared memory, for the LH units
+  DOT_LH = 9,    // L(i, k): its sum first, then the mid barrier, then scaled
+  DOT_Y = 10,    // y_k (first: starts from the right-hand side, else from y)
+  DOT_B = 11     // x_k
 };
-constexpr uint32_t DOT_BARF = 1u << 4, DOT_FIRST = 1u << 5, DOT_CIN = 1u << 6, DOT_COUT = 1u << 7;
+constexpr uint32_t DOT_BARF = 1u << 4, DOT_FIRST = 1u << 5, DOT_CIN = 1u << 6, DOT_COUT = 1u << 7,
+                   DOT_ROW = 1u << 16, DOT_NEXT = 1u << 16;
 constexpr int kDotTerms = 8;    // products of a unit
+constexpr int kDotBackWarps = 16;  // warps of the top's backward CTA
+// products of a chain's row (two rows in registers)
+constexpr int dot_chain_terms(int elem) { return elem == 4 ? 10 : 8; }
 constexpr int kDotChunk = 32;   // quads of a chunk: one 16-byte load per lane
 constexpr int kDotMaxMid = 14;  // mid barriers of one tick (ids 1..14)
 
@@ -60,14 +68,16 @@ struct DotPlan {
   int bins = 0;        // bins of the bottom (0: every column is in the top)
   int top_warps = 16;
   double cap = 1.0;    // largest part, of a bin's even share
-  int ahead = 4;       // ticks by which values are touched before their use (0: not)
+  int chain = 8;       // longest rows of a chain
+  int pack = 3;        // longest sums that are packed by fours (0: none)
+  int ahead = 2;       // ticks by which values are touched before their use (0: not)
   int keep = 700;      // values touched since, after which one is taken to have left the L1
 };
 
 struct DotProgram {
   DotPlan plan;
   std::vector<uint32_t> words;                   // all streams, 4 words per quad
-  std::vector<int32_t> bottom, prep, top, back;  // per bin / warp: first quad of its stream
+  std::vector<int32_t> bottom, prep, top, tback, back;  // per bin / warp: first quad of its stream
   bool with_subst = false;                       // forward and backward substitution included
   int ticks = 0, back_ticks = 0;
   int64_t units = 0, parts = 0, bottom_cols = 0, top_terms = 0, prep_terms = 0, touched = 0;

@@ -674,8 +674,8 @@ struct StreamDev {
 // launch the first quad of each.
 struct DotDev {
   const uint4* words;
-  const int32_t *bottom, *prep, *top, *back;
-  int n_bottom, n_prep, n_top, n_back;
+  const int32_t *bottom, *prep, *top, *tback, *back;
+  int n_bottom, n_prep, n_top, n_tback, n_back;
 };
 
 // Progress flags (plans with sync = 1).  A warp that has done its work of
