@@ -89,6 +89,9 @@ struct BatchDev {
   const double *o_dre, *o_dim;
   float piv_tol;                   // pivot-ratio threshold (mixed path)
   int32_t* err;                    // [0] set when a bounded device wait gave up
+  // a start point that all scenarios share, per bus: cos, sin of its angle, e, f
+  // and the current sum_k Y_ik V_k (k_shared_start); null: each has its own
+  const double* st0;               // [6][n_bus]
   int32_t* itp;                    // [1] iteration of the graph-captured loop (kernels given it < 0)
 };
 
@@ -153,6 +156,18 @@ __device__ __forceinline__ void update_body(const SchedDev& S, const BatchDev& D
   const int s = g * 32 + lane;
   const bool upd = D.status[s] == ST_RUNNING && (it > 0 || mode == 1) && D.sing[s] == 0;
   const size_t x = gidx(g, N, i, lane);
+  if (it == 0 && mode == 0 && D.st0 != nullptr) {
+    // the shared start: its trigonometry once per bus instead of per scenario
+    const double e = D.st0[2 * (size_t)N + i], f = D.st0[3 * (size_t)N + i];
+    D.cth[x] = D.st0[i];
+    D.sth[x] = D.st0[(size_t)N + i];
+    D.e[x] = e;
+    D.f[x] = f;
+    ((T*)D.eT)[x] = to_T<T>(e);
+    ((T*)D.fT)[x] = to_T<T>(f);
+    ((T*)D.ivT)[x] = (T)1 / to_T<T>(D.vm[x]);
+    return;
+  }
   double vm = D.vm[x], va = D.va[x];
   double dth = 0.0;
   float step = 0.0f;  // the angle step as solved (FP32 path): picks the formula below
@@ -251,6 +266,36 @@ __device__ __forceinline__ void y_row(const SchedDev& S, const double* __restric
   }
 }
 
+// A start point that every scenario has: cos, sin, e, f and the injected
+// current of each bus, once (the mismatch kernels of iteration 0 would compute
+// them for every scenario: a sincos and 4 FMAs per Y entry).  The same
+// operations in the same order as k_update and k_inject.  Those are bound by
+// FP64 operations.  Measured, all mismatch kernels of a solve: 2,000 buses x
+// 4096 scenarios, six of them, mixed 4.16 -> 3.63 ms; 10,000 x 4096, five,
+// 14.6 -> 12.0 ms.
+__global__ void k_shared_start(SchedDev S, const double* __restrict__ vm, const double* __restrict__ va,
+                               double* __restrict__ st0) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, N = S.n_bus;
+  if (i >= N) return;
+  double ir = 0.0, ii = 0.0, sn, cs;
+  for (int p = S.yp[i]; p < S.yp[i + 1]; p++) {
+    const int k = S.yi[p];
+    sincos(va[k], &sn, &cs);
+    const double e = vm[k] * cs, f = vm[k] * sn, gr = S.yre[p], gi = S.yim[p];
+    ir = fma(gr, e, ir);
+    ir = fma(-gi, f, ir);
+    ii = fma(gr, f, ii);
+    ii = fma(gi, e, ii);
+  }
+  sincos(va[i], &sn, &cs);
+  st0[i] = cs;
+  st0[(size_t)N + i] = sn;
+  st0[2 * (size_t)N + i] = vm[i] * cs;
+  st0[3 * (size_t)N + i] = vm[i] * sn;
+  st0[4 * (size_t)N + i] = ir;
+  st0[5 * (size_t)N + i] = ii;
+}
+
 __device__ __forceinline__ unsigned long long abs_bits(double v) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
   return b > 0x7ff0000000000000ull ? 0ull : b;  // NaN: skipped
@@ -275,24 +320,30 @@ __device__ __forceinline__ void inject_body(const SchedDev& S, const BatchDev& D
   // a block is 8 warps; a wider CTA's other warps only take its barrier
   const bool in_block = warp < 8;
   const int i0 = in_block ? (BX * 8 + warp) * BPW : N;
+  const double* st0 = it == 0 ? D.st0 : nullptr;  // the shared start's currents
   for (int i = i0; i < min(N, i0 + BPW); i++) {
     double ir = 0.0, ii = 0.0;
-    int p = __ldg(S.yp + i);
-    const int pe = __ldg(S.yp + i + 1);
-    while (pe - p > 8) {
-      y_row<8>(S, e, f, g, N, lane, p, ir, ii);
-      p += 8;
-    }
-    switch (pe - p) {
-      case 1: y_row<1>(S, e, f, g, N, lane, p, ir, ii); break;
-      case 2: y_row<2>(S, e, f, g, N, lane, p, ir, ii); break;
-      case 3: y_row<3>(S, e, f, g, N, lane, p, ir, ii); break;
-      case 4: y_row<4>(S, e, f, g, N, lane, p, ir, ii); break;
-      case 5: y_row<5>(S, e, f, g, N, lane, p, ir, ii); break;
-      case 6: y_row<6>(S, e, f, g, N, lane, p, ir, ii); break;
-      case 7: y_row<7>(S, e, f, g, N, lane, p, ir, ii); break;
-      case 8: y_row<8>(S, e, f, g, N, lane, p, ir, ii); break;
-      default: break;
+    if (st0 != nullptr) {
+      ir = st0[4 * (size_t)N + i];
+      ii = st0[5 * (size_t)N + i];
+    } else {
+      int p = __ldg(S.yp + i);
+      const int pe = __ldg(S.yp + i + 1);
+      while (pe - p > 8) {
+        y_row<8>(S, e, f, g, N, lane, p, ir, ii);
+        p += 8;
+      }
+      switch (pe - p) {
+        case 1: y_row<1>(S, e, f, g, N, lane, p, ir, ii); break;
+        case 2: y_row<2>(S, e, f, g, N, lane, p, ir, ii); break;
+        case 3: y_row<3>(S, e, f, g, N, lane, p, ir, ii); break;
+        case 4: y_row<4>(S, e, f, g, N, lane, p, ir, ii); break;
+        case 5: y_row<5>(S, e, f, g, N, lane, p, ir, ii); break;
+        case 6: y_row<6>(S, e, f, g, N, lane, p, ir, ii); break;
+        case 7: y_row<7>(S, e, f, g, N, lane, p, ir, ii); break;
+        case 8: y_row<8>(S, e, f, g, N, lane, p, ir, ii); break;
+        default: break;
+      }
     }
     const size_t x = gidx(g, N, i, lane);
     const double ei = e[x], fi = f[x];
