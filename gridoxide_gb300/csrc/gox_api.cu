@@ -12,6 +12,7 @@
 #include <map>
 #include <cstdio>
 #include <cstdlib>
+#include <climits>
 #include <cstring>
 #include <memory>
 #include <mutex>
@@ -300,6 +301,19 @@ __global__ void k_unpack_scen(int B, const int32_t* st_in, const int32_t* it_in,
 
 // ---------------------------------------------------------------------------
 
+// A topology's dot programs: for batches of few groups (with a mid stage, where
+// one pays) and for larger ones; one of them alone serves both.
+struct DotPair {
+  std::shared_ptr<const DotProgram> few, many;
+  int few_groups() const {
+    if (!few) return 0;
+    if (!many) return INT_MAX;
+    int g = 1;
+    while (dot_few(few->plan, g + 1)) g++;
+    return g;
+  }
+};
+
 struct DevSchedule {
   DevMem yp, yi, yre, yim, bus_rowP, bus_rowQ, bus_colA, bus_colV, a_kind, a_bi, a_bk, a_yslot,
       a_dst, lev_ptr, lev_cols, c_base, c_ulen, c_llen, c_abeg, c_aend, op_ptr, op_slot, op_pos, ph_ptr,
@@ -317,46 +331,69 @@ struct DevSchedule {
   int st_wr[2] = {0, 0};                      // their stage rows per warp
   std::vector<int32_t> lev_ptr_h;  // host copy: columns per refactor level
   // a dot-product program in place of the streams, per precision (on: used)
+  struct DotOne {
+    DevMem words, starts;
+    DotDev d{};
+  };
   struct DotPlanDev {
     bool on = false, with_subst = false;
-    int top_warps = 0, bins = 0;
-    DevMem words, bottom, prep, top, tback, back;
-    DotDev d{};
+    int few_groups = 0;  // batches of up to that many groups run few, larger ones many
+    DotOne few, many;
+    const DotDev& pick(int groups) const { return groups <= few_groups ? few.d : many.d; }
   } dot[2];
   // the plan's substitutions are part of its refactor
   bool has_bwd(int i) const { return dot[i].on ? dot[i].with_subst : st_bwd[i]; }
   // launches of one refactor (with both substitutions when the plan has them)
-  int refactor_launches(int i) const {
-    if (dot[i].on)
-      return 1 + (dot[i].d.n_bottom > 0) + (dot[i].d.n_prep > 0) + (dot[i].d.n_tback > 0) + (dot[i].d.n_back > 0);
+  int refactor_launches(int i, int groups) const {
+    if (dot[i].on) {
+      const DotDev& d = dot[i].pick(groups);
+      return 1 + (d.n_bottom > 0) + (d.n_prep > 0) + (d.n_mid > 0) + (d.n_prep2 > 0) + (d.n_tback > 0) +
+             (d.n_midback > 0) + (d.n_back > 0);
+    }
     return 1 + st_wl[i] + st_wp[i];
   }
 
-  // (null: the streams)
-  void load_dot(int i, const DotProgram* p) {
+  static void load_one(DotOne& x, const DotProgram& p) {
+    upload(x.words, p.words);
+    std::vector<int32_t> all;  // the launches' streams, one after the other
+    for (const auto* l : {&p.bottom, &p.prep, &p.mid, &p.prep2, &p.top, &p.tback, &p.midback, &p.back})
+      all.insert(all.end(), l->begin(), l->end());
+    upload(x.starts, all);
+    const int32_t* at = x.starts.as<int32_t>();
+    auto next = [&](const std::vector<int32_t>& l) {
+      const int32_t* r = at;
+      at += l.size();
+      return r;
+    };
+    DotDev& d = x.d;
+    const int nt = (int)p.top.size();
+    d.words = x.words.as<uint4>();
+    d.bottom = next(p.bottom);
+    d.prep = next(p.prep);
+    d.mid = next(p.mid);
+    d.prep2 = next(p.prep2);
+    d.top = next(p.top);
+    d.tback = next(p.tback);
+    d.midback = next(p.midback);
+    d.back = next(p.back);
+    d.n_bottom = (int)p.bottom.size();
+    d.n_prep = (int)p.prep.size();
+    d.n_top = nt;
+    d.n_tback = (int)p.tback.size();
+    d.n_back = (int)p.back.size();
+    d.n_mid = (int)p.mid.size() / nt;
+    d.n_prep2 = (int)p.prep2.size() / nt;
+    d.n_midback = (int)p.midback.size() / kDotBackWarps;
+  }
+  // (none: the streams)
+  void load_dot(int i, const DotPair& p) {
     DotPlanDev& x = dot[i];
-    x.on = p != nullptr;
-    if (!p) return;
-    x.with_subst = p->with_subst;
-    x.top_warps = (int)p->top.size();
-    x.bins = p->plan.bins;
-    upload(x.words, p->words);
-    upload(x.bottom, p->bottom);
-    upload(x.prep, p->prep);
-    upload(x.top, p->top);
-    upload(x.tback, p->tback);
-    upload(x.back, p->back);
-    x.d.words = x.words.as<uint4>();
-    x.d.bottom = x.bottom.as<int32_t>();
-    x.d.prep = x.prep.as<int32_t>();
-    x.d.top = x.top.as<int32_t>();
-    x.d.tback = x.tback.as<int32_t>();
-    x.d.back = x.back.as<int32_t>();
-    x.d.n_bottom = (int)p->bottom.size();
-    x.d.n_prep = (int)p->prep.size();
-    x.d.n_top = (int)p->top.size();
-    x.d.n_tback = (int)p->tback.size();
-    x.d.n_back = (int)p->back.size();
+    x.on = p.few || p.many;
+    if (!x.on) return;
+    x.with_subst = (p.few ? p.few : p.many)->with_subst;
+    x.few_groups = p.few_groups();
+    if (p.few) load_one(x.few, *p.few);
+    if (p.many) load_one(x.many, *p.many);
   }
 
   void load_streams(const Stream& s32, const Stream& s64) {
@@ -642,7 +679,7 @@ struct Iter {
   static void refactor(const DevSchedule& ds, const BatchDev& D, cudaStream_t st) {
     const int i = sizeof(T) == 4 ? 0 : 1;
     if (ds.dot[i].on) {
-      dot(ds.dot[i].d, ds.d, D, D.G, st);
+      dot(ds.dot[i].pick(D.G), ds.d, D, D.G, st);
       return;
     }
     refactor_with(ds, ds.st[i], ds.st_nw[i], ds.st_smem[i], ds.st_wl[i], ds.st_wp[i], ds.st_wr[i], D,
@@ -691,15 +728,24 @@ struct Iter {
   static void dot_bins(const DotDev& P, const SchedDev& S, const BatchDev& D, int n, int groups, cudaStream_t st) {
     if (n > 0) k_dot_bins<T, WHICH><<<dim3(dot_blocks(n), groups), 32 * kDotBinWarps, 0, st>>>(P, S, D);
   }
+  static void dot_top(const DotDev& P, const SchedDev& S, const BatchDev& D, int stage, int groups, cudaStream_t st) {
+    const dim3 grid(dot_ctas(P, stage), groups);
+    if (grid.x == 0) return;
+    if constexpr (sizeof(T) == 4) {
+      if (P.n_top == 32) k_dot_top<T, 32><<<grid, 1024, 0, st>>>(P, S, D, stage);
+    }
+    if (P.n_top == 16) k_dot_top<T, 16><<<grid, 512, 0, st>>>(P, S, D, stage);
+  }
   static void dot(const DotDev& P, const SchedDev& S, const BatchDev& D, int groups, cudaStream_t st) {
     dot_attr();
     dot_bins<DOT_BOTTOM>(P, S, D, P.n_bottom, groups, st);
     dot_bins<DOT_PREP>(P, S, D, P.n_prep, groups, st);
-    if constexpr (sizeof(T) == 4) {
-      if (P.n_top == 32) k_dot_top<T, 32><<<groups, 1024, 0, st>>>(P, S, D);
-    }
-    if (P.n_top == 16) k_dot_top<T, 16><<<groups, 512, 0, st>>>(P, S, D);
-    if (P.n_tback > 0) k_dot_topback<T><<<groups, 32 * kDotBackWarps, 0, st>>>(P, S, D);
+    dot_top(P, S, D, DOT_IN_MID, groups, st);
+    dot_top(P, S, D, DOT_IN_PREP2, groups, st);
+    dot_top(P, S, D, DOT_IN_TOP, groups, st);
+    const unsigned bt = 32 * kDotBackWarps;
+    if (P.n_tback > 0) k_dot_topback<T><<<dim3(1, groups), bt, 0, st>>>(P, S, D, DOT_IN_TOP);
+    if (P.n_midback > 0) k_dot_topback<T><<<dim3(P.n_midback, groups), bt, 0, st>>>(P, S, D, DOT_IN_MID);
     dot_bins<DOT_BACK>(P, S, D, P.n_back, groups, st);
   }
   // shared memory of a wide-kernel CTA whose warps stage `rows` rows
@@ -825,8 +871,10 @@ struct gox_topo {
   Numeric num;
   Schedule sc;
   Stream s32, s64;
-  // the dot program used in place of the streams, per precision (null: the streams)
-  std::shared_ptr<const DotProgram> dot[2];
+  // the dot programs used in place of the streams, per precision (none: the
+  // streams), and the one the tuner chose or found
+  DotPair dot[2];
+  std::shared_ptr<const DotProgram> dot_main[2];
   DevSchedule dsched;
   DevBatch batch;
   // re-packing: the smaller batch the running scenarios move to, and their
@@ -1022,8 +1070,10 @@ static int fix_pivots(gox_topo* t, int B, const double* p_spec, const double* q_
       t->num = std::move(N);
       build_schedule(&t->jac, t->csc, t->sym, t->num, t->sc);
       make_streams(t->sc, t->s32, t->s64);
-      t->dot[0].reset();
-      t->dot[1].reset();
+      for (int i = 0; i < 2; i++) {
+        t->dot[i] = DotPair();
+        t->dot_main[i].reset();
+      }
       t->factored = true;
       t->uploaded = false;
       (void)nu;
@@ -1038,7 +1088,7 @@ static int fix_pivots(gox_topo* t, int B, const double* p_spec, const double* q_
 static void upload_plans(gox_topo* t) {
   t->dsched.load(t->sc, t->yp, t->yi, t->yre, t->yim);
   t->dsched.load_streams(t->s32, t->s64);
-  for (int i = 0; i < 2; i++) t->dsched.load_dot(i, t->dot[i].get());
+  for (int i = 0; i < 2; i++) t->dsched.load_dot(i, t->dot[i]);
   t->uploaded = true;
 }
 
@@ -1136,7 +1186,7 @@ static std::vector<unsigned char> loop_key(const gox_topo* t, const BatchDev& D,
   put(&t->dsched.st_smem[i], sizeof(size_t)); put(&t->dsched.st_bwd[i], sizeof(bool));
   put(&t->dsched.st_wl[i], sizeof(int)); put(&t->dsched.st_wp[i], sizeof(int));
   put(&t->dsched.st_wr[i], sizeof(int));
-  put(&t->dsched.dot[i].on, sizeof(bool)); put(&t->dsched.dot[i].d, sizeof(DotDev));
+  put(&t->dsched.dot[i].on, sizeof(bool)); put(&t->dsched.dot[i].pick(D.G), sizeof(DotDev));
   return key;
 }
 
@@ -1290,7 +1340,7 @@ static void tune_cache_load() {
 }
 
 // A dot program's entry: its top's warps, the words of its streams' chunks
-// (no stream plan has chunks that short), 0, its bins.
+// (no stream plan has chunks that short), its mid stage's CTAs, its bins.
 static constexpr int kDotChunkWords = 4 * kDotChunk;
 
 static void tune_cache_store(const std::array<int, 4>& k, const std::array<int, 4>& v) {
@@ -1330,16 +1380,36 @@ static void drop_loops(gox_topo* t, int i) {
   t->loop_graphs = std::move(keep);
 }
 
-static void install_dot(gox_topo* t, int i, std::shared_ptr<const DotProgram> p) {
+// p: chosen for batches of `groups` groups; other: for those of the other
+// kind (few or many), null: p for those too.  Both null: the streams.
+static void install_dot(gox_topo* t, int i, std::shared_ptr<const DotProgram> p, int groups,
+                        std::shared_ptr<const DotProgram> other) {
+  const bool few = p && dot_few(p->plan, groups);
   for (gox_topo* x = t; x; x = x->twin.get()) {  // and the split solves' twins
-    x->dot[i] = p;
-    if (x->uploaded) x->dsched.load_dot(i, p.get());
+    x->dot[i] = few ? DotPair{p, other} : DotPair{other, p};
+    x->dot_main[i] = p;
+    if (x->uploaded) x->dsched.load_dot(i, x->dot[i]);
     drop_loops(x, i);
   }
 }
+// the plan for batches of the other kind than one of `groups` groups
+static DotPlan dot_other(const Schedule& sc, int elem, int groups) {
+  return dot_default(sc, elem, groups * 3 <= 152 ? 152 : 1);
+}
+// Before a solve of `groups` groups: the program of that kind, where the
+// topology's plan was found in the cache and only its own kind is built.
+static void ensure_dot_kind(gox_topo* t, int i, int groups) {
+  const std::shared_ptr<const DotProgram> p = t->dot_main[i];
+  if (!p || t->tune_cache_only || (t->dot[i].few && t->dot[i].many)) return;
+  const int elem = i == 0 ? 4 : 8;
+  const bool few = p == t->dot[i].few;
+  if (few ? dot_few(p->plan, groups) : !dot_few(dot_default(t->sc, elem, 1), groups)) return;
+  const int own = few ? 1 : 152;
+  install_dot(t, i, p, own, make_dot(t->sc, dot_other(t->sc, elem, own)));
+}
 
 static void install_stream(gox_topo* t, int i, Stream&& s) {
-  install_dot(t, i, nullptr);
+  install_dot(t, i, nullptr, 1, nullptr);
   (i == 0 ? t->s32 : t->s64) = std::move(s);
   t->dsched.load_streams(t->s32, t->s64);
   drop_loops(t, i);
@@ -1367,16 +1437,23 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st) {
     auto it = g_tune.find(key);
     if (it == g_tune.end() && t->tune_cache_only) {
       // not timed: the program the measured rule gives
-      install_dot(t, i, make_dot(sc, dot_default(sc, elem, D.G)));
+      install_dot(t, i, make_dot(sc, dot_default(sc, elem, D.G)), D.G, nullptr);
       return;
     }
     if (it != g_tune.end() && it->second[1] == kDotChunkWords) {
-      for (const DotPlan& p : dot_candidates(sc, elem))
-        if (p.top_warps == it->second[0] && p.bins == it->second[3]) {
-          install_dot(t, i, make_dot(sc, p));
-          TU.source = 2;
-          return;
-        }
+      // (timed on a batch of the key's smallest size, its mid stage can have more
+      // CTAs than this batch allows: the most that it does)
+      const DotPlan* found = nullptr;
+      const std::vector<DotPlan> plans = dot_candidates(sc, elem, D.G);
+      for (const DotPlan& p : plans)
+        if (p.top_warps == it->second[0] && p.bins == it->second[3] && p.mid <= it->second[2] &&
+            (!found || p.mid > found->mid))
+          found = &p;
+      if (found) {
+        install_dot(t, i, make_dot(sc, *found), D.G, nullptr);
+        TU.source = 2;
+        return;
+      }
       if (t->tune_cache_only) return;
     } else if (it != g_tune.end()) {
       const Stream& cur = i == 0 ? t->s32 : t->s64;
@@ -1408,7 +1485,8 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st) {
   std::vector<StreamPlan> cand = candidate_plans(sc, elem, kRefactorSmem);
   std::vector<Stream> built(cand.size());
   std::vector<char> ok(cand.size(), 0);
-  const std::vector<DotPlan> dcand = dot_candidates(sc, elem);
+  std::vector<DotPlan> dcand = dot_candidates(sc, elem, D.G);
+  dcand.push_back(dot_other(sc, elem, D.G));  // (not timed)
   std::vector<std::shared_ptr<const DotProgram>> dbuilt(dcand.size());
   {
     std::vector<std::thread> th;
@@ -1432,6 +1510,7 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st) {
   const int Gt = std::min(D.G, 152);
   const size_t img_bytes = (size_t)Gt * sc.n_slots * 32 * sizeof(T);
   DevMem bak, words, c0, nc;
+  DevSchedule::DotOne dev;
   bak.ensure(img_bytes);
   GOX_CK(cudaMemcpyAsync(bak.p, D.lu, img_bytes, cudaMemcpyDeviceToDevice, st));
   cudaEvent_t e0, e1;
@@ -1461,17 +1540,15 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st) {
     GOX_CK(cudaMemcpyAsync(D.err - 1, z, 8, cudaMemcpyHostToDevice, st));
     return -1.0f;
   };
-  for (size_t c = 0; c < cand.size() + dcand.size(); c++) {
+  for (size_t c = 0; c + 1 < cand.size() + dcand.size(); c++) {
     if (c >= cand.size()) {
       const DotProgram* p = dbuilt[c - cand.size()].get();
       if (!p) continue;
-      DevSchedule::DotPlanDev& x = t->dsched.dot[i];
-      t->dsched.load_dot(i, p);
-      x.on = false;  // until one is installed
-      const float ms = time_plan([&] { Iter<T>::dot(x.d, t->dsched.d, D, Gt, st); });
+      DevSchedule::load_one(dev, *p);
+      const float ms = time_plan([&] { Iter<T>::dot(dev.d, t->dsched.d, D, Gt, st); });
       if (ms < 0.0f) continue;
       TU.table.push_back({(double)p->plan.top_warps, (double)kDotChunkWords, 0.0, (double)ms, 0.0,
-                          (double)p->plan.bins, (double)p->plan.bins});
+                          (double)p->plan.bins, (double)p->plan.mid});
       if (ms < best_ms) {
         best_ms = ms;
         best = (int)c;
@@ -1510,12 +1587,13 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st) {
   GOX_CK(cudaStreamSynchronize(st));
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
+  std::stable_sort(TU.table.begin(), TU.table.end(), [](const auto& x, const auto& y) { return x[3] < y[3]; });
   if (best < 0) return;
   std::array<int, 4> entry;
   if (best >= (int)cand.size()) {
     const std::shared_ptr<const DotProgram> p = dbuilt[best - (int)cand.size()];
-    entry = {p->plan.top_warps, kDotChunkWords, 0, p->plan.bins};
-    install_dot(t, i, p);
+    entry = {p->plan.top_warps, kDotChunkWords, p->plan.mid, p->plan.bins};
+    install_dot(t, i, p, D.G, dbuilt.back());
   } else {
     const StreamPlan& p = cand[best];
     entry = {p.nw, p.chunk_words, p.sync, p.wide_levels > 0 ? p.wide_min : 0};
@@ -1643,7 +1721,7 @@ static void run_iterations(gox_topo* t, BatchDev D, int max_iter, bool outage, c
     const int its = h[1], ran_out = (h[0] > 0 && its >= max_iter) ? 1 : 0;
     const int fills = h[0] > 0 ? its : its - 1;
     const int ns = t->dsched.has_bwd(sizeof(T) == 4 ? 0 : 1) ? 0 : 1;
-    const int nr = t->dsched.refactor_launches(sizeof(T) == 4 ? 0 : 1);
+    const int nr = t->dsched.refactor_launches(sizeof(T) == 4 ? 0 : 1, D.G);
     t->launches += (int64_t)its * 4 + (int64_t)fills * (1 + nr + ns) + ran_out * 2;
     return;
   }
@@ -1694,7 +1772,7 @@ static void run_iterations(gox_topo* t, BatchDev D, int max_iter, bool outage, c
       ns = Iter<T>::solve_rest(t->dsched, D, st);
     }
     rec();
-    t->launches += 1 + t->dsched.refactor_launches(sizeof(T) == 4 ? 0 : 1) + ns;
+    t->launches += 1 + t->dsched.refactor_launches(sizeof(T) == 4 ? 0 : 1, D.G) + ns;
     GOX_CK(cudaGetLastError());
   }
   if (it == max_iter) t->launches += Iter<T>::mismatch(S, D, max_iter, 1, outage, st);
@@ -1810,7 +1888,7 @@ static void guess_build(gox_topo* t, const double* p0, const double* q0) {
   std::vector<double> dummy_x;
   G.dsched.load(G.sc, dummy_p, dummy_i, dummy_x, dummy_x);
   G.dsched.load_streams(G.s32, G.s64);
-  G.dsched.load_dot(1, make_dot(G.sc, dot_default(G.sc, 8, 128)).get());
+  G.dsched.load_dot(1, DotPair{make_dot(G.sc, dot_default(G.sc, 8, 1)), make_dot(G.sc, dot_default(G.sc, 8, 152))});
   // value recipe per LU slot, then per off-diagonal entry
   const int ns = G.sc.n_slots, no = G.sc.n_off;
   std::vector<int32_t> rec((size_t)(ns + no) * 4);
@@ -2265,7 +2343,9 @@ struct MultiLists {
   struct L { size_t off = 0, job = 0; int n = 0, ctas = 0; };
   L upd, inj, dec, fill, rf;
   std::vector<L> wide;  // per wide level
-  L dbins[3], dtop[2], dtback;  // dot programs: bottom, prep, back; the top with 16 and 32 warps, its rows
+  // dot programs: bottom, prep, back; the tick launches (top, mid, prep 2) with
+  // 16 and 32 warps; the top's rows, the mid stage's
+  L dbins[3], dtop[3][2], dtback[2];
   MultiList view(const L& l) const {
     MultiList m;
     m.off = dev.as<int32_t>() + l.off;
@@ -2309,21 +2389,29 @@ static void build_lists(const std::vector<gox_topo*>& ts, const std::vector<Batc
   // jobs whose plan is a dot program: a list per launch, the top's by its warps
   // (longest first too); the others run their streams
   std::vector<int> dots, streams, top[2];
+  auto dd = [&](int j) -> const DotDev& { return ts[j]->dsched.dot[i].pick(G(j)); };
   for (int j : order) {
-    const auto& x = ts[j]->dsched.dot[i];
-    (x.on ? dots : streams).push_back(j);
-    if (x.on) top[x.top_warps == 32].push_back(j);
+    const bool on = ts[j]->dsched.dot[i].on;
+    (on ? dots : streams).push_back(j);
+    if (on) top[dd(j).n_top == 32].push_back(j);
   }
-  for (int w = 0; w < 2; w++) M.dtop[w] = add(top[w], [&](int j) { return G(j); });
-  {
+  for (int w = 0; w < 2; w++)
+    for (int s : {DOT_IN_TOP, DOT_IN_MID, DOT_IN_PREP2}) {
+      std::vector<int> jl;
+      for (int j : top[w])
+        if (dot_ctas(dd(j), s) > 0) jl.push_back(j);
+      M.dtop[s][w] = add(jl, [&](int j) { return dot_ctas(dd(j), s) * G(j); });
+    }
+  for (int s : {DOT_IN_TOP, DOT_IN_MID}) {
+    auto n = [&](int j) { return s == DOT_IN_MID ? dd(j).n_midback : dd(j).n_tback > 0 ? 1 : 0; };
     std::vector<int> jl;
     for (int j : dots)
-      if (ts[j]->dsched.dot[i].d.n_tback > 0) jl.push_back(j);
-    M.dtback = add(jl, [&](int j) { return G(j); });
+      if (n(j) > 0) jl.push_back(j);
+    M.dtback[s] = add(jl, [&](int j) { return n(j) * G(j); });
   }
   for (int w : {DOT_BOTTOM, DOT_PREP, DOT_BACK}) {
     auto n = [&](int j) {
-      const DotDev& d = ts[j]->dsched.dot[i].d;
+      const DotDev& d = dd(j);
       return w == DOT_BOTTOM ? d.n_bottom : w == DOT_PREP ? d.n_prep : d.n_back;
     };
     std::vector<int> jl;
@@ -2360,7 +2448,7 @@ static void upload_jobs(const std::vector<gox_topo*>& ts, const std::vector<Batc
     jobs[j].S = ts[j]->dsched.d;
     jobs[j].D = runs[j].D;
     jobs[j].P = ts[j]->dsched.st[i];
-    jobs[j].dot = ts[j]->dsched.dot[i].d;
+    jobs[j].dot = ts[j]->dsched.dot[i].pick(runs[j].D.G);
     jobs[j].nw = ts[j]->dsched.st_nw[i];
   }
   dev.ensure(jobs.size() * sizeof(MultiJob));
@@ -2490,12 +2578,15 @@ static void run_multi(const std::vector<gox_topo*>& ts, std::vector<BatchRun>& r
            [&](unsigned c, MultiList l) { k_dot_bins_multi<T, DOT_BOTTOM><<<c, bt, 0, st>>>(J, l); });
     launch(M.dbins[DOT_PREP],
            [&](unsigned c, MultiList l) { k_dot_bins_multi<T, DOT_PREP><<<c, bt, 0, st>>>(J, l); });
-    if constexpr (sizeof(T) == 4)
-      launch(M.dtop[1], [&](unsigned c, MultiList l) { k_dot_top_multi<T, 32><<<c, 1024, 0, st>>>(J, l); });
-    launch(M.dtop[0], [&](unsigned c, MultiList l) { k_dot_top_multi<T, 16><<<c, 512, 0, st>>>(J, l); });
-    launch(M.dtback, [&](unsigned c, MultiList l) {
-      k_dot_topback_multi<T><<<c, 32 * kDotBackWarps, 0, st>>>(J, l);
-    });
+    for (int s : {DOT_IN_MID, DOT_IN_PREP2, DOT_IN_TOP}) {
+      if constexpr (sizeof(T) == 4)
+        launch(M.dtop[s][1], [&](unsigned c, MultiList l) { k_dot_top_multi<T, 32><<<c, 1024, 0, st>>>(J, l, s); });
+      launch(M.dtop[s][0], [&](unsigned c, MultiList l) { k_dot_top_multi<T, 16><<<c, 512, 0, st>>>(J, l, s); });
+    }
+    for (int s : {DOT_IN_TOP, DOT_IN_MID})
+      launch(M.dtback[s], [&](unsigned c, MultiList l) {
+        k_dot_topback_multi<T><<<c, 32 * kDotBackWarps, 0, st>>>(J, l, s);
+      });
     launch(M.dbins[DOT_BACK],
            [&](unsigned c, MultiList l) { k_dot_bins_multi<T, DOT_BACK><<<c, bt, 0, st>>>(J, l); });
     rec();
@@ -2956,7 +3047,10 @@ static std::unique_ptr<gox_topo> clone_factored(const gox_topo* t) {
   v->yp = t->yp; v->yi = t->yi; v->yre = t->yre; v->yim = t->yim; v->bus_type = t->bus_type;
   v->jac = t->jac; v->csc = t->csc; v->sym = t->sym; v->num = t->num; v->sc = t->sc;
   v->s32 = t->s32; v->s64 = t->s64;
-  v->dot[0] = t->dot[0]; v->dot[1] = t->dot[1];
+  for (int i = 0; i < 2; i++) {
+    v->dot[i] = t->dot[i];
+    v->dot_main[i] = t->dot_main[i];
+  }
   v->factored = true;
   v->uploaded = false;
   v->device = t->device;
@@ -3017,6 +3111,7 @@ static int batch_split(gox_topo* t, int B, const double* p_spec, const double* q
   // 10,000-bus N-1 batch of 8,192: 4 parts 117-121 ms, 2 parts 122-124 ms
   // with host buffers; the 2,000-bus batch of 4,096 alike for 2, 4 and 8)
   const int want = t->split_parts > 0 ? t->split_parts : (B >= 8192 ? 4 : 2);
+  if (t->factored) ensure_dot_kind(t, precision == GOX_PRECISION_MIXED ? 0 : 1, (B + 31) / 32);
   if (want < 2 || !t->factored || t->guess_mode != 0 || t->timing.on ||
       B < kSplitMinScenarios || precision != GOX_PRECISION_MIXED || !t->tune[0].done)
     return batch_any(t, B, p_spec, q_spec, vm0, va0, v_stride, o_slot, o_dre, o_dim, tol, max_iter,
@@ -3186,8 +3281,10 @@ int gox_topo_reset(gox_topo* t) {
   t->uploaded = false;
   t->num = Numeric();
   t->sc = Schedule();
-  t->dot[0].reset();
-  t->dot[1].reset();
+  for (int i = 0; i < 2; i++) {
+    t->dot[i] = DotPair();
+    t->dot_main[i].reset();
+  }
   t->tune[0] = gox_topo::Tuning();
   t->tune[1] = gox_topo::Tuning();
   return GOX_OK;
@@ -3746,9 +3843,10 @@ int gox_topo_emulate_step(const gox_topo* t, const double* jac_vals, const doubl
       if (!(lu[x] == lu64[x]) && !(std::isnan(lu[x]) && std::isnan(lu64[x])))
         throw std::runtime_error("the two refactor streams disagree");
     // ... and the dot programs of both precisions, the same factor again
-    for (int elem : {4, 8}) {
+    for (int c = 0; c < 4; c++) {  // for few groups, for many
+      const int elem = c & 1 ? 8 : 4;
       DotProgram p;
-      build_dot(sc, dot_default(sc, elem, 1), p);
+      build_dot(sc, dot_default(sc, elem, c & 2 ? 152 : 1), p);
       std::vector<double> lud(sc.n_slots, 0.0), Xd;
       for (int x = 0; x < sc.n_slots; x++)
         lud[x] = sc.slot_a[x] >= 0 ? packed[sc.a_csc[sc.slot_a[x]]] : 0.0;
@@ -3990,12 +4088,13 @@ int gox_topo_tuning(const gox_topo* t, int32_t precision, int64_t* plan, double*
   plan[6] = s.plan.sync;
   plan[7] = s.plan.wide_levels;
   plan[8] = s.plan.wide_phases;
-  if (const DotProgram* p = t->dot[i].get()) {
+  if (const DotProgram* p = t->dot_main[i].get()) {
     plan[0] = p->plan.top_warps;
     plan[1] = plan[2] = 0;
     plan[3] = kDotChunkWords;
     plan[6] = 0;
-    plan[7] = plan[8] = p->plan.bins;
+    plan[7] = p->plan.bins;
+    plan[8] = p->plan.mid;
   }
   int rows = 0;
   for (const auto& r : TU.table) {
@@ -4201,7 +4300,7 @@ int gox_ls_create(int32_t n, int32_t nnz, const int32_t* rows, const int32_t* co
     std::vector<double> dummy_x;
     h->dsched.load(h->sc, dummy_p, dummy_i, dummy_x, dummy_x);
     h->dsched.load_streams(h->s32, h->s64);
-    h->dsched.load_dot(1, make_dot(h->sc, dot_default(h->sc, 8, 1)).get());
+    h->dsched.load_dot(1, DotPair{make_dot(h->sc, dot_default(h->sc, 8, 1)), nullptr});
     const SchedDev& S = h->dsched.d;
     h->jbuf.ensure((size_t)S.n_a * 32 * 8 + 8);
     h->lu.ensure((size_t)S.n_slots * 32 * 8 + 8);

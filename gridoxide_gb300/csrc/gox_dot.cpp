@@ -198,33 +198,50 @@ void append(DotProgram& P, std::vector<int32_t>& starts, Writer& W) {
 static int top_warps(int elem) { return elem == 4 ? 32 : 16; }
 
 // Bins: the more there are, the more of the chip the bottom fills but the more
-// columns are left to the top's ticks (measured, ms per refactor with 32 / 64 /
-// 128 / 256 / 512 / 1024 bins: 2,000 buses, 128 groups FP32 - / 1.93 / 1.79 /
-// 1.77 / 1.78 / -; one group - / - / 1.13 / 1.07 / 1.12 / -; 10,000 buses, 128
-// groups - / 7.4 / 6.4 / 6.1 / 6.0 / -; 20,000 buses, one group - / - / 5.1 /
-// 4.4 / 4.3 / 4.7).  Below 400 unknowns the launches around the top cost what
-// the bottom saves (118 buses FP64, one group: no bins 0.221, 32 bins 0.219).
+// columns are left to the ticks (measured, ms per refactor with 32 / 64 / 128 /
+// 256 / 512 / 1024 / 2048 bins and no mid stage: 2,000 buses, 128 groups FP32 - / 1.93
+// / 1.79 / 1.77 / 1.78 / - / -; 10,000 buses, 128 groups - / 7.4 / 6.4 / 6.1 / 6.0 /
+// - / -; with a mid stage: 2,000 buses, one group - / - / .84 / .78 / .73 / - / -;
+// 20,000 buses, one group - / - / - / 2.63 / 1.96 / 1.75 / 1.67).  Below 400 unknowns
+// the launches around the top cost what the bottom saves (118 buses FP64, one
+// group: no bins 0.221, 32 bins 0.219).
+// Mid stage: while its CTAs of all groups find an SM each, it takes the early,
+// wide ticks off the one SM of a group (ms per refactor without and with 4 / 8 /
+// 16 / 32 CTAs: 2,000 buses, one group FP32, 256 bins .99, .79 / .78 / .81 / .83;
+// 32 groups 1.03, .84 / .86 / - / -; 128 groups 1.46, - / 1.59; 47 groups FP64
+// 2.07, 1.74 with 3 and 1.95 with 8; 20,000 buses, one group 3.86, 2.32 / 2.00 /
+// 1.96 / -; 118 buses, one group FP64 .196, .156 with 8).
+constexpr int kSMs = 152;
+
+bool dot_few(const DotPlan& p, int groups) { return groups * std::max(p.mid, 3) <= kSMs; }
+
 DotPlan dot_default(const Schedule& sc, int elem, int groups) {
   DotPlan p;
   p.top_warps = top_warps(elem);
   p.chain = dot_chain_terms(elem);
-  const int per = groups >= 32 ? 32 : 16;  // unknowns per bin
-  while (sc.n_u >= 400 && p.bins < 512 && p.bins * per < sc.n_u) p.bins = p.bins ? 2 * p.bins : 32;
+  const bool few = groups * 3 <= kSMs;
+  const int per = few ? 8 : 32;  // unknowns per bin
+  while (sc.n_u >= 400 && p.bins < (few ? 2048 : 512) && p.bins * per < sc.n_u) p.bins = p.bins ? 2 * p.bins : 32;
+  if (few && sc.n_u >= 100) p.mid = std::min(kSMs / groups, sc.n_u >= 20000 ? 16 : 8);
   return p;
 }
 
-std::vector<DotPlan> dot_candidates(const Schedule& sc, int elem) {
+std::vector<DotPlan> dot_candidates(const Schedule& sc, int elem, int groups) {
   std::vector<DotPlan> out;
-  for (int bins : {0, 32, 64, 128, 256, 512, 1024}) {
+  for (int bins : {0, 32, 64, 128, 256, 512, 1024, 2048}) {
     if (bins > 0 && (bins * 4 > sc.n_u || bins * 400 < sc.n_u)) continue;
     if (bins == 0 && sc.n_u > 1500) continue;
-    for (int w : {32, 16}) {
-      if (w > top_warps(elem)) continue;
-      DotPlan p;
-      p.bins = bins;
-      p.top_warps = w;
-      p.chain = dot_chain_terms(elem);
-      out.push_back(p);
+    for (int mid : {0, 3, 4, 8, 16, 32}) {
+      if (mid > 0 && (mid * groups > kSMs || mid * 20 > sc.n_u || (bins > 0 && bins * 64 < sc.n_u))) continue;
+      for (int w : {32, 16}) {
+        if (w > top_warps(elem) || (mid > 0 && w < top_warps(elem))) continue;
+        DotPlan p;
+        p.bins = bins;
+        p.mid = mid;
+        p.top_warps = w;
+        p.chain = dot_chain_terms(elem);
+        out.push_back(p);
+      }
     }
   }
   return out;
@@ -252,21 +269,25 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
     if (subst) ccost[k] += 8.0 * nt(ns + k);
     total += ccost[k];
   }
-  std::vector<int32_t> part(n, -1);  // union-find parent of bottom columns, -1: top
+  std::vector<char> stage(n, 2);  // 0 bottom, 1 mid, 2 top
+  std::vector<int32_t> part(n), cta(n, -1);  // union-find parent; the mid column's CTA
   std::vector<double> pcost(n, 0.0);
   auto find = [&](int k) {
     while (part[k] != k) k = part[k] = part[part[k]];
     return k;
   };
-  if (plan.bins > 0) {
-    const double cap = plan.cap * total / plan.bins;
+  // columns into stage st: those whose dependences are in earlier stages or in a
+  // part of theirs, as long as their part is small enough
+  auto grow_parts = [&](char st, double cap) {
     std::vector<int32_t> roots;
     for (int k = 0; k < n; k++) {
+      if (stage[k] < st) continue;
       bool ok = true;
       roots.clear();
       double c = ccost[k];
       auto dep = [&](int j) {
-        if (part[j] < 0) { ok = false; return; }
+        if (stage[j] < st) return;
+        if (stage[j] > st) { ok = false; return; }
         const int r = find(j);
         if (std::find(roots.begin(), roots.end(), r) == roots.end()) {
           roots.push_back(r);
@@ -277,32 +298,53 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
       if (subst)
         for (int t = sc.fw_ptr[k]; ok && t < sc.fw_ptr[k + 1]; t++) dep(sc.fw_col[t]);
       if (!ok || c > cap) continue;
+      stage[k] = st;
       part[k] = k;
       for (int r : roots) part[r] = k;
       pcost[k] = c;
     }
-  }
-  // parts to bins, largest first onto the least loaded bin
-  std::vector<std::vector<int32_t>> members(n);
-  std::vector<int32_t> parts;
-  for (int k = 0; k < n; k++)
-    if (part[k] >= 0) {
-      const int r = find(k);
-      members[r].push_back(k);
-      if (r == k) parts.push_back(k);
-      P.bottom_cols++;
-    }
-  std::stable_sort(parts.begin(), parts.end(), [&](int x, int y) { return pcost[x] > pcost[y]; });
-  std::vector<std::vector<int32_t>> bin(plan.bins);
-  {
+  };
+  // a stage's parts to its workers, largest first onto the least loaded one
+  auto deal_parts = [&](char st, int workers) {
+    std::vector<std::vector<int32_t>> members(n), out(workers);
+    std::vector<int32_t> parts;
+    for (int k = 0; k < n; k++)
+      if (stage[k] == st) {
+        const int r = find(k);
+        members[r].push_back(k);
+        if (r == k) parts.push_back(k);
+      }
+    std::stable_sort(parts.begin(), parts.end(), [&](int x, int y) { return pcost[x] > pcost[y]; });
     std::priority_queue<std::pair<double, int>, std::vector<std::pair<double, int>>, std::greater<>> q;
-    for (int b = 0; b < plan.bins; b++) q.push({0.0, b});
+    for (int b = 0; b < workers; b++) q.push({0.0, b});
     for (int r : parts) {
       auto [c, b] = q.top();
       q.pop();
-      bin[b].insert(bin[b].end(), members[r].begin(), members[r].end());
+      out[b].insert(out[b].end(), members[r].begin(), members[r].end());
       q.push({c + pcost[r], b});
     }
+    return out;
+  };
+  std::vector<std::vector<int32_t>> bin, mid;
+  if (plan.bins > 0) {
+    grow_parts(0, plan.cap * total / plan.bins);
+    bin = deal_parts(0, plan.bins);
+  }
+  if (plan.mid > 0) {
+    double rest = 0;
+    for (int k = 0; k < n; k++)
+      if (stage[k] > 0) rest += ccost[k];
+    grow_parts(1, plan.mid_cap * rest / plan.mid);
+    for (auto& m : deal_parts(1, plan.mid)) {
+      if (m.empty()) continue;
+      std::sort(m.begin(), m.end());
+      for (int k : m) cta[k] = (int)mid.size();
+      mid.push_back(std::move(m));
+    }
+  }
+  for (int k = 0; k < n; k++) {
+    P.bottom_cols += stage[k] == 0;
+    P.mid_cols += stage[k] == 1;
   }
   auto emit_sum = [&](Writer& W, uint32_t op, int v, uint32_t z, int t0, int t1) {
     const bool y = v >= ns;
@@ -382,7 +424,7 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
       append(P, P.bottom, W);
     }
   }
-  // ---- prep: per top column, the leading products of each sum whose values
+  // ---- prep: per later column, the leading products of each sum whose values
   // the bottom (or the prep of this same column) finishes
   if (P.bottom_cols > 0) {
     std::vector<int32_t> prep_depth(ns + n, 0);
@@ -392,13 +434,13 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
     // 2,000 buses, 256 bins, 128 groups FP32 0.305 / 0.276 / 0.285 ms for 1 / 2 / 4)
     const int per_stream = left_cols >= 256 ? 2 : 1;
     for (int k = 0; k < n; k++) {
-      if (part[k] >= 0) continue;
+      if (stage[k] == 0) continue;
       const int base = sc.c_base[k];
       auto prefix = [&](int v) {
         int t = S.ptr[v], d = 0;
         for (; t < S.ptr[v + 1]; t++) {
-          if (part[S.col[S.a[t]]] < 0) break;  // an L value of a top column
-          if (v >= ns ? part[S.b[t]] < 0 : taken[S.b[t]] != nt(S.b[t])) break;
+          if (stage[S.col[S.a[t]]] > 0) break;  // an L value of a later column
+          if (v >= ns ? stage[S.b[t]] > 0 : taken[S.b[t]] != nt(S.b[t])) break;
           if (v < ns) d = std::max(d, prep_depth[S.b[t]]);
         }
         if (t == S.ptr[v]) return;
@@ -420,8 +462,8 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
     }
   }
 
-  // ---- top: nodes (a leading part of a sum, a U entry, a column's pivot and
-  // L entries, a y), each in a tick after the ticks of what it reads
+  // ---- top and mid: nodes (a leading part of a sum, a U entry, a column's pivot
+  // and L entries, a y), each in a tick after the ticks of what it reads
   struct Node {
     int32_t kind;    // 0 part, 1 U, 2 column, 3 y
     int32_t v;       // value, or the column
@@ -435,9 +477,16 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
   std::vector<int32_t> node_of(ns + n, -1);  // value -> the node that finishes it (-1: before the top)
   std::vector<int32_t> done(ns + n, -1);     // value -> tick it is final after
   std::vector<int32_t> from(ns + n, 0);      // first product left for the node that finishes it
+  std::vector<int32_t> stop(S.ptr.begin() + 1, S.ptr.end());  // and the end of the products run here
   const int NT = plan.top_warps;
   int makespan = 0;
   std::vector<int32_t> preds;
+  // what each tick's warps do
+  struct Do { int32_t w; uint32_t op; int32_t v; uint32_t z; int32_t t0, t1; };
+  struct Ticks {
+    std::vector<std::vector<Do>> plan;
+    std::vector<std::vector<double>> load;
+  };
   auto add_node = [&](Node nd) {
     std::sort(preds.begin(), preds.end());
     preds.erase(std::unique(preds.begin(), preds.end()), preds.end());
@@ -465,7 +514,7 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
   constexpr int kPartMin = 3, kPartMax = 8;
   auto split = [&](int v, int final_tick) {
     int t = S.ptr[v] + taken[v];
-    const int t1 = S.ptr[v + 1];
+    const int t1 = stop[v];
     int prev = -1, prev_tick = -1;
     while (t1 - t >= kPartMin) {
       int q = t, r = std::max(0, prev_tick + 1);
@@ -487,172 +536,186 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
     from[v] = t;
     return prev;
   };
-  auto left = [&](int v) { return S.ptr[v + 1] - from[v]; };
-  for (int k = 0; k < n; k++) {
-    if (part[k] >= 0) continue;
-    const int base = sc.c_base[k], ul = sc.c_ulen[k];
-    for (int v = base; v < base + ul; v++) {
-      if (nt(v) == taken[v]) continue;
-      const int r = ready(v, S.ptr[v] + taken[v], S.ptr[v + 1]);
-      const int p = split(v, r);
-      preds.clear();
-      take_preds(v, from[v], S.ptr[v + 1]);
-      preds.push_back(p);
-      node_of[v] = add_node({1, v, from[v], S.ptr[v + 1], r, 0, sum_cost(left(v))});
-      done[v] = r;
-    }
-    int r = 0;
-    for (int v = base + ul; v < base + len(k); v++) r = std::max(r, ready(v, S.ptr[v] + taken[v], S.ptr[v + 1]));
-    std::vector<int32_t> cp;
-    double cost = 0;
-    for (int v = base + ul; v < base + len(k); v++) {
-      cp.push_back(split(v, r));
-      cost += sum_cost(left(v));
-    }
-    preds = cp;
-    for (int v = base + ul; v < base + len(k); v++) take_preds(v, from[v], S.ptr[v + 1]);
-    const int id = add_node({2, k, 0, 0, r, 0, cost});
-    for (int v = base + ul; v < base + len(k); v++) {
-      node_of[v] = id;
-      done[v] = r;
-    }
-    if (subst && (taken[ns + k] < nt(ns + k) || taken[ns + k] == 0)) {
-      const int v = ns + k;
-      const int ry = ready(v, S.ptr[v] + taken[v], S.ptr[v + 1]);
-      const int p = split(v, ry);
-      preds.clear();
-      take_preds(v, from[v], S.ptr[v + 1]);
-      preds.push_back(p);
-      node_of[v] = add_node({3, v, from[v], S.ptr[v + 1], ry, 0, sum_cost(left(v))});
-      done[v] = ry;
-    }
-  }
-  // as late as possible
-  const int nn = (int)nodes.size();
-  for (auto& x : nodes) x.late = makespan - 1;
-  std::vector<int32_t> sptr(nn + 1, 0), succ(edges.size()), npred(nn, 0);
-  for (auto& e : edges) {
-    sptr[e.first + 1]++;
-    npred[e.second]++;
-  }
-  for (int i = 0; i < nn; i++) sptr[i + 1] += sptr[i];
-  {
-    std::vector<int32_t> at(sptr.begin(), sptr.end() - 1);
-    for (auto& e : edges) succ[at[e.first]++] = e.second;
-  }
-  for (int i = nn - 1; i >= 0; i--)
-    for (int q = sptr[i]; q < sptr[i + 1]; q++) nodes[i].late = std::min(nodes[i].late, nodes[succ[q]].late - 1);
-
-  // what each tick's warps do (the backward rows' ticks included)
-  struct Do { int32_t w; uint32_t op; int32_t v; uint32_t z; int32_t t0, t1; };
-  std::vector<std::vector<Do>> plan_of, back_of;
-  std::vector<std::vector<double>> load_of, back_load;
-  int tick = 0;
-  auto emit = [&](int w, uint32_t op, int v, uint32_t z, int t0, int t1) {
-    P.top_terms += t1 - t0;
-    plan_of.back().push_back({w, op, v, z, t0, t1});
-  };
-
-  // ticks: what cannot wait, then ready nodes (the most urgent first) while
-  // the warps have room beside it
-  {
-    using Item = std::pair<int32_t, int32_t>;  // late, node
-    std::priority_queue<Item, std::vector<Item>, std::greater<>> q;
-    for (int i = 0; i < nn; i++)
-      if (npred[i] == 0) q.push({nodes[i].late, i});
-    int todo = nn;
-    std::vector<int32_t> now;
-    std::vector<double> load(NT);
-    while (todo > 0) {
-      now.clear();
-      double room = 0, sum = 0, ready_cost = 0;
-      std::vector<Item> rest;
-      while (!q.empty()) {
-        Item it = q.top();
-        q.pop();
-        ready_cost += nodes[it.second].cost;
-        if (it.first <= tick) {
-          now.push_back(it.second);
-          sum += nodes[it.second].cost;
-          room = std::max(room, nodes[it.second].kind == 2 ? 250.0 : nodes[it.second].cost);
-        } else {
-          rest.push_back(it);
-        }
+  auto left = [&](int v) { return stop[v] - from[v]; };
+  // the ticks of a CTA's columns (part: of their sums' products up to `stop`)
+  auto schedule = [&](const std::vector<int32_t>& columns, bool part) {
+    nodes.clear();
+    edges.clear();
+    makespan = 0;
+    for (int k : columns) {
+      const int base = sc.c_base[k], ul = sc.c_ulen[k];
+      auto sum = [&](int kind, int v) {
+        const int r = ready(v, S.ptr[v] + taken[v], stop[v]);
+        const int p = split(v, r);
+        preds.clear();
+        take_preds(v, from[v], stop[v]);
+        preds.push_back(p);
+        node_of[v] = add_node({kind, v, from[v], stop[v], r, 0, sum_cost(left(v))});
+        done[v] = r;
+      };
+      for (int v = base; v < base + (part ? len(k) : ul); v++)
+        if (stop[v] > S.ptr[v] + taken[v]) sum(1, v);
+      if (part) {
+        if (subst && stop[ns + k] > S.ptr[ns + k] + taken[ns + k]) sum(3, ns + k);
+        continue;
       }
-      room = std::max({room, 250.0, std::min(ready_cost / NT, 6000.0)});
-      for (Item& it : rest) {
-        if (sum + nodes[it.second].cost <= 0.8 * room * NT) {
-          now.push_back(it.second);
-          sum += nodes[it.second].cost;
-        } else {
-          q.push(it);
-        }
+      int r = 0;
+      for (int v = base + ul; v < base + len(k); v++) r = std::max(r, ready(v, S.ptr[v] + taken[v], S.ptr[v + 1]));
+      std::vector<int32_t> cp;
+      double cost = 0;
+      for (int v = base + ul; v < base + len(k); v++) {
+        cp.push_back(split(v, r));
+        cost += sum_cost(left(v));
       }
-      // warps: columns first (split over warps while there are warps for all
-      // their entries), then the other sums onto the least loaded warp
-      std::fill(load.begin(), load.end(), 0.0);
-      plan_of.emplace_back();
-      std::vector<int32_t> cols, others, whole;
-      for (int i : now) (nodes[i].kind == 2 ? cols : others).push_back(i);
-      std::stable_sort(cols.begin(), cols.end(), [&](int x, int y) { return nodes[x].late < nodes[y].late; });
-      int used = 0, mids = 0;
-      const int shift = (tick * 7) % NT;
-      auto least = [&]() { return (int)(std::min_element(load.begin(), load.end()) - load.begin()); };
-      for (int i : cols) {
-        const int k = nodes[i].v, ul = sc.c_ulen[k], ll = sc.c_llen[k], base = sc.c_base[k];
-        if (ll > 0 && used + 1 + ll <= NT && mids < kDotMaxMid) {
-          const uint32_t z = (uint32_t)(32 * (1 + ll)) | ((uint32_t)mids << 16), id = (uint32_t)(mids + 1) << 8;
-          mids++;
-          for (int e = 0; e <= ll; e++) {
-            const int v = base + ul + e, w = (used++ + shift) % NT;
-            emit(w, (e ? DOT_LH : DOT_D) | id, v, z, from[v], S.ptr[v + 1]);
-            load[w] += sum_cost(left(v)) + (e ? 60 : 0);
+      preds = cp;
+      for (int v = base + ul; v < base + len(k); v++) take_preds(v, from[v], S.ptr[v + 1]);
+      const int id = add_node({2, k, 0, 0, r, 0, cost});
+      for (int v = base + ul; v < base + len(k); v++) {
+        node_of[v] = id;
+        done[v] = r;
+      }
+      if (subst && (taken[ns + k] < nt(ns + k) || taken[ns + k] == 0)) sum(3, ns + k);
+    }
+    // as late as possible
+    const int nn = (int)nodes.size();
+    for (auto& x : nodes) x.late = makespan - 1;
+    std::vector<int32_t> sptr(nn + 1, 0), succ(edges.size()), npred(nn, 0);
+    for (auto& e : edges) {
+      sptr[e.first + 1]++;
+      npred[e.second]++;
+    }
+    for (int i = 0; i < nn; i++) sptr[i + 1] += sptr[i];
+    {
+      std::vector<int32_t> at(sptr.begin(), sptr.end() - 1);
+      for (auto& e : edges) succ[at[e.first]++] = e.second;
+    }
+    for (int i = nn - 1; i >= 0; i--)
+      for (int q = sptr[i]; q < sptr[i + 1]; q++) nodes[i].late = std::min(nodes[i].late, nodes[succ[q]].late - 1);
+
+    Ticks out;
+    std::vector<std::vector<Do>>& plan_of = out.plan;
+    std::vector<std::vector<double>>& load_of = out.load;
+    int tick = 0;
+    auto emit = [&](int w, uint32_t op, int v, uint32_t z, int t0, int t1) {
+      P.top_terms += t1 - t0;
+      plan_of.back().push_back({w, op, v, z, t0, t1});
+    };
+
+    // ticks: what cannot wait, then ready nodes (the most urgent first) while
+    // the warps have room beside it
+    {
+      using Item = std::pair<int32_t, int32_t>;  // late, node
+      std::priority_queue<Item, std::vector<Item>, std::greater<>> q;
+      for (int i = 0; i < nn; i++)
+        if (npred[i] == 0) q.push({nodes[i].late, i});
+      int todo = nn;
+      std::vector<int32_t> now;
+      std::vector<double> load(NT);
+      while (todo > 0) {
+        now.clear();
+        double room = 0, sum = 0, ready_cost = 0;
+        std::vector<Item> rest;
+        while (!q.empty()) {
+          Item it = q.top();
+          q.pop();
+          ready_cost += nodes[it.second].cost;
+          if (it.first <= tick) {
+            now.push_back(it.second);
+            sum += nodes[it.second].cost;
+            room = std::max(room, nodes[it.second].kind == 2 ? 250.0 : nodes[it.second].cost);
+          } else {
+            rest.push_back(it);
           }
-        } else {
-          whole.push_back(i);
         }
-      }
-      for (int i : whole) {
-        const int k = nodes[i].v, ul = sc.c_ulen[k], ll = sc.c_llen[k], base = sc.c_base[k];
-        const int w = least();
-        for (int e = 0; e <= ll; e++) {
-          const int v = base + ul + e;
-          if (left(v)) emit(w, DOT_U, v, 0, from[v], S.ptr[v + 1]);
-          load[w] += sum_cost(left(v));
+        room = std::max({room, 250.0, std::min(ready_cost / NT, 6000.0)});
+        for (Item& it : rest) {
+          if (sum + nodes[it.second].cost <= 0.8 * room * NT) {
+            now.push_back(it.second);
+            sum += nodes[it.second].cost;
+          } else {
+            q.push(it);
+          }
         }
-        plan_of.back().push_back({w, DOT_FIN, k, 0u, 0, 0});
+        // warps: columns first (split over warps while there are warps for all
+        // their entries), then the other sums onto the least loaded warp
+        std::fill(load.begin(), load.end(), 0.0);
+        plan_of.emplace_back();
+        std::vector<int32_t> cols, others, whole;
+        for (int i : now) (nodes[i].kind == 2 ? cols : others).push_back(i);
+        std::stable_sort(cols.begin(), cols.end(), [&](int x, int y) { return nodes[x].late < nodes[y].late; });
+        int used = 0, mids = 0;
+        const int shift = (tick * 7) % NT;
+        auto least = [&]() { return (int)(std::min_element(load.begin(), load.end()) - load.begin()); };
+        for (int i : cols) {
+          const int k = nodes[i].v, ul = sc.c_ulen[k], ll = sc.c_llen[k], base = sc.c_base[k];
+          if (ll > 0 && used + 1 + ll <= NT && mids < kDotMaxMid) {
+            const uint32_t z = (uint32_t)(32 * (1 + ll)) | ((uint32_t)mids << 16), id = (uint32_t)(mids + 1) << 8;
+            mids++;
+            for (int e = 0; e <= ll; e++) {
+              const int v = base + ul + e, w = (used++ + shift) % NT;
+              emit(w, (e ? DOT_LH : DOT_D) | id, v, z, from[v], S.ptr[v + 1]);
+              load[w] += sum_cost(left(v)) + (e ? 60 : 0);
+            }
+          } else {
+            whole.push_back(i);
+          }
+        }
+        for (int i : whole) {
+          const int k = nodes[i].v, ul = sc.c_ulen[k], ll = sc.c_llen[k], base = sc.c_base[k];
+          const int w = least();
+          for (int e = 0; e <= ll; e++) {
+            const int v = base + ul + e;
+            if (left(v)) emit(w, DOT_U, v, 0, from[v], S.ptr[v + 1]);
+            load[w] += sum_cost(left(v));
+          }
+          plan_of.back().push_back({w, DOT_FIN, k, 0u, 0, 0});
+        }
+        std::stable_sort(others.begin(), others.end(), [&](int x, int y) { return nodes[x].cost > nodes[y].cost; });
+        for (int i : others) {
+          const Node& nd = nodes[i];
+          const int w = least();
+          const bool y = nd.v >= ns;
+          emit(w, y ? DOT_Y : DOT_U, nd.v, 0, nd.t0, nd.t1);
+          load[w] += nd.cost;
+        }
+        load_of.push_back(load);
+        todo -= (int)now.size();
+        tick++;
+        for (int i : now)
+          for (int s = sptr[i]; s < sptr[i + 1]; s++)
+            if (--npred[succ[s]] == 0) q.push({nodes[succ[s]].late, succ[s]});
       }
-      std::stable_sort(others.begin(), others.end(), [&](int x, int y) { return nodes[x].cost > nodes[y].cost; });
-      for (int i : others) {
-        const Node& nd = nodes[i];
-        const int w = least();
-        const bool y = nd.v >= ns;
-        emit(w, y ? DOT_Y : DOT_U, nd.v, 0, nd.t0, nd.t1);
-        load[w] += nd.cost;
-      }
-      load_of.push_back(load);
-      todo -= (int)now.size();
-      tick++;
-      for (int i : now)
-        for (int s = sptr[i]; s < sptr[i + 1]; s++)
-          if (--npred[succ[s]] == 0) q.push({nodes[succ[s]].late, succ[s]});
     }
-  }
-  P.ticks = tick;
+    for (int k : columns) {  // (for a later launch all of this is done before)
+      auto ran = [&](int v) {
+        node_of[v] = done[v] = -1;
+        taken[v] = stop[v] - S.ptr[v];
+        stop[v] = S.ptr[v + 1];
+      };
+      for (int v = sc.c_base[k]; v < sc.c_base[k] + len(k); v++) ran(v);
+      if (subst) ran(ns + k);
+    }
+    return out;
+  };
   auto row = [&](Writer& w, int k) {
     P.units += w.sum(DOT_B, (uint32_t)k, (uint32_t)sc.diag_slot[k], sc.bw_slot.data() + sc.bw_ptr[k],
                      sc.bw_col.data() + sc.bw_ptr[k], sc.bw_ptr[k + 1] - sc.bw_ptr[k]);
   };
-  // ---- backward rows of the top columns, level by level, then the bottom's
-  if (subst) {
-    std::vector<int32_t> lev(n, 0);
+  // ---- a CTA's backward rows, level by level
+  std::vector<int32_t> lev(n, 0);
+  auto backward = [&](const std::vector<int32_t>& columns) {
+    Ticks out;
+    std::vector<std::vector<Do>>& back_of = out.plan;
+    std::vector<std::vector<double>>& back_load = out.load;
     std::vector<std::vector<int32_t>> bylev;
-    for (int k = n - 1; k >= 0; k--) {
-      if (part[k] >= 0) continue;
+    for (size_t i = columns.size(); i-- > 0;) {
+      const int k = columns[i];
       int l = 0;
       for (int t = sc.bw_ptr[k]; t < sc.bw_ptr[k + 1]; t++) {
-        if (part[sc.bw_col[t]] >= 0) throw std::runtime_error("a top row reads a bottom row");
-        l = std::max(l, lev[sc.bw_col[t]] + 1);
+        const int j = sc.bw_col[t];
+        if (stage[j] > stage[k]) continue;  // an earlier launch's
+        if (stage[j] < stage[k] || cta[j] != cta[k]) throw std::runtime_error("a row reads a later launch's");
+        l = std::max(l, lev[j] + 1);
       }
       lev[k] = l;
       if ((int)bylev.size() <= l) bylev.resize(l + 1);
@@ -686,7 +749,6 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
         ticks_of.push_back(rows);
       }
     }
-    P.back_ticks = (int)ticks_of.size();
     int turn = 0;
     for (size_t t = 0; t < ticks_of.size(); t++) {
       const std::vector<int32_t>& rows = ticks_of[t];
@@ -709,19 +771,15 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
       }
       back_load.push_back(load);
     }
-    for (int b = 0; b < plan.bins; b++) {
-      if (bin[b].empty()) continue;
-      Writer w;
-      for (size_t i = bin[b].size(); i-- > 0;) row(w, bin[b][i]);
-      append(P, P.back, w);
-    }
-  }
-  // the top's streams; a value whose last use lies too far back to be still in
+    return out;
+  };
+  // a CTA's streams; a value whose last use lies too far back to be still in
   // the L1 is touched `ahead` ticks before the tick that needs it, by the
   // warps with the least to do there (not for ticks that fill all warps: they
   // hide their loads behind each other)
-  auto streams = [&](const std::vector<std::vector<Do>>& plan_of, std::vector<std::vector<double>>& load_of, int NT,
-                     std::vector<int32_t>& out) {
+  auto streams = [&](Ticks&& ticks, int NT, std::vector<int32_t>& out) {
+    const std::vector<std::vector<Do>>& plan_of = ticks.plan;
+    std::vector<std::vector<double>>& load_of = ticks.load;
     const int nticks = (int)plan_of.size();
     std::vector<std::vector<std::pair<std::vector<int32_t>, std::vector<int32_t>>>> touch(nticks);  // per tick and warp
     if (plan.ahead > 0) {
@@ -804,8 +862,55 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
     }
     for (auto& w : W) append(P, out, w);
   };
-  streams(plan_of, load_of, NT, P.top);
-  if (subst) streams(back_of, back_load, kDotBackWarps, P.tback);
+  for (auto& m : mid) streams(schedule(m, false), NT, P.mid);
+  std::vector<int32_t> top;
+  for (int k = 0; k < n; k++)
+    if (stage[k] == 2) top.push_back(k);
+  // ---- the top columns' products that the mid stage's values (and the same
+  // column's, then final) allow, in ticks too: a column's U entries along a
+  // path of the mid stage's columns depend on each other
+  if (!mid.empty())
+    for (size_t i = 0; i < top.size();) {
+      std::vector<int32_t> cols;
+      for (; i < top.size() && (int)cols.size() < plan.prep_cols; i++) {
+        const int k = top[i], base = sc.c_base[k];
+        bool any = false;
+        auto prefix = [&](int v) {
+          const int t0 = S.ptr[v] + taken[v];
+          for (stop[v] = t0; stop[v] < S.ptr[v + 1]; stop[v]++) {
+            const int a = S.a[stop[v]], b = S.b[stop[v]];
+            if (stage[S.col[a]] > 1 || (v >= ns ? stage[b] > 1 : stop[b] < S.ptr[b + 1])) break;
+          }
+          any |= stop[v] > t0;
+          P.prep_terms += stop[v] - t0;
+        };
+        for (int d = 0; d < len(k); d++) prefix(base + d);
+        if (subst) prefix(ns + k);
+        if (any) cols.push_back(k);
+        else
+          for (int d = 0; d < len(k); d++) stop[base + d] = S.ptr[base + d + 1];
+        if (!any && subst) stop[ns + k] = S.ptr[ns + k + 1];
+      }
+      if (!cols.empty()) streams(schedule(cols, true), NT, P.prep2);
+    }
+  {
+    Ticks t = schedule(top, false);
+    P.ticks = (int)t.plan.size();
+    streams(std::move(t), NT, P.top);
+  }
+  if (!subst) return;
+  {
+    Ticks t = backward(top);
+    P.back_ticks = (int)t.plan.size();
+    streams(std::move(t), kDotBackWarps, P.tback);
+  }
+  for (auto& m : mid) streams(backward(m), kDotBackWarps, P.midback);
+  for (int b = 0; b < plan.bins; b++) {
+    if (bin[b].empty()) continue;
+    Writer w;
+    for (size_t i = bin[b].size(); i-- > 0;) row(w, bin[b][i]);
+    append(P, P.back, w);
+  }
 }
 
 std::string run_dot_host(const Schedule& sc, const DotProgram& P, std::vector<double>& lu,
@@ -820,6 +925,10 @@ std::string run_dot_host(const Schedule& sc, const DotProgram& P, std::vector<do
   std::vector<char> fin(ns + n, 0), xdone(n, 0);
   std::vector<int64_t> wtick(ns + n, -1), rtick(ns + n, -1);
   std::vector<int32_t> wwarp(ns + n, -1), rwarp(ns + n, -1);
+  // ... and the CTA, of a launch of several CTAs with ticks (numbered through all
+  // launches; 0: the launch has none): launch and CTA of the last write and read
+  std::vector<int32_t> wlaunch(ns + n, -1), rlaunch(ns + n, -1), wcta(ns + n, -1), rcta(ns + n, -1);
+  int32_t launch_no = 0, cta = 0;
   for (int k = 0; k < n; k++)
     for (int v = sc.c_base[k]; v < sc.c_base[k] + sc.c_ulen[k]; v++)
       if (S.ptr[v + 1] == S.ptr[v]) fin[v] = 1;
@@ -835,6 +944,9 @@ std::string run_dot_host(const Schedule& sc, const DotProgram& P, std::vector<do
   };
   auto read = [&](int v, int w) {
     if (wtick[v] == tick && wwarp[v] != w) return fail("a value read in the tick another warp writes it");
+    if (wlaunch[v] == launch_no && wcta[v] != cta) return fail("a value read in the launch another CTA writes it");
+    if (rlaunch[v] != launch_no) { rlaunch[v] = launch_no; rcta[v] = cta; }
+    else if (rcta[v] != cta) rcta[v] = -2;
     if (rtick[v] != tick) { rtick[v] = tick; rwarp[v] = w; }
     else if (rwarp[v] != w) rwarp[v] = -2;  // several warps
     return true;
@@ -842,8 +954,12 @@ std::string run_dot_host(const Schedule& sc, const DotProgram& P, std::vector<do
   auto write = [&](int v, int w) {
     if (wtick[v] == tick && wwarp[v] != w) return fail("two warps write one value in one tick");
     if (rtick[v] == tick && rwarp[v] != w) return fail("a value written in the tick another warp reads it");
+    if ((wlaunch[v] == launch_no && wcta[v] != cta) || (rlaunch[v] == launch_no && rcta[v] != cta))
+      return fail("a value written in the launch another CTA uses it");
     wtick[v] = tick;
     wwarp[v] = w;
+    wlaunch[v] = launch_no;
+    wcta[v] = cta;
     return true;
   };
   struct Held { uint32_t z, id; };
@@ -1088,6 +1204,8 @@ std::string run_dot_host(const Schedule& sc, const DotProgram& P, std::vector<do
   auto launch = [&](const std::vector<int32_t>& st, uint32_t units, auto&& run) {
     int w = 0;
     may = units;
+    launch_no++;
+    cta = 0;
     for (int32_t s : st)
       if (s < 0 || (size_t)s >= nq || !run(s, w++)) return false;
     tick++;
@@ -1098,7 +1216,7 @@ std::string run_dot_host(const Schedule& sc, const DotProgram& P, std::vector<do
     return step(B, w, false) && (B.ended || fail("a bin that does not end"));
   };
   if (!launch(P.bottom, kAny | kSums, bin) || !launch(P.prep, kAny | kSums, bin)) return err;
-  // the top's warps, tick by tick
+  // a CTA's warps, tick by tick
   auto ticks = [&](const std::vector<int32_t>& st, uint32_t units) -> bool {
     may = units;
     const int NT = (int)st.size();
@@ -1146,8 +1264,21 @@ std::string run_dot_host(const Schedule& sc, const DotProgram& P, std::vector<do
     }
     return true;
   };
-  if (!ticks(P.top, kTick | kSums | 1u << DOT_D | 1u << DOT_LH) ||
-      !ticks(P.tback, kTick | 1u << DOT_B | 1u << DOT_CHAIN))
+  // a launch of CTAs of NT warps each
+  auto ctas = [&](const std::vector<int32_t>& st, size_t NT, uint32_t units) {
+    launch_no++;
+    if (st.size() % NT) return fail("a CTA with missing warps");
+    for (size_t c = 0; c * NT < st.size(); c++) {
+      cta = (int32_t)c;
+      if (!ticks(std::vector<int32_t>(st.begin() + c * NT, st.begin() + (c + 1) * NT), units)) return false;
+    }
+    return true;
+  };
+  const uint32_t fwd = kTick | kSums | 1u << DOT_D | 1u << DOT_LH, bwd = kTick | 1u << DOT_B | 1u << DOT_CHAIN;
+  const size_t NT = (size_t)P.plan.top_warps;
+  if (P.top.size() != NT || P.tback.size() > (size_t)kDotBackWarps) return "a top of other than one CTA";
+  if (!ctas(P.mid, NT, fwd) || !ctas(P.prep2, NT, fwd) || !ctas(P.top, NT, fwd) ||
+      !ctas(P.tback, kDotBackWarps, bwd) || !ctas(P.midback, kDotBackWarps, bwd))
     return err;
   if (!launch(P.back, kAny | 1u << DOT_B, bin)) return err;
   for (int v = 0; v < ns + n; v++)

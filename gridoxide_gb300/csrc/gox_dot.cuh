@@ -19,10 +19,16 @@
 // Why chains: a backward row of the tail took about 950 cycles, the loads of
 // the next row now run under it (2,000 buses, 128 groups FP32: 1.62 -> 1.45 ms
 // with the kernels split by launch).
-// Refactor with both substitutions, streams -> programs, ms: 2,000 buses, 128
-// groups FP32 2.15 -> 1.43, 47 groups FP64 5.94 -> 2.0, one group FP32 2.07 ->
-// 0.95; 10,000 buses, 128 groups FP32 9.4 -> 4.9; 20,000 buses, one group FP32
-// 9.5 -> 3.8; 118 buses, one group FP64 0.41 -> 0.19.
+// Why the mid stage: a group's top ran on one SM, its early ticks 10 to 20k
+// cycles wide, while with few groups the other SMs were idle.  Its second prep
+// runs in ticks because a top column's U entries along a path of mid columns
+// depend on each other (20,000 buses, one warp per column 0.35 ms, depth by
+// depth over a CTA 0.35, with the sums' leading parts in earlier ticks 0.17).
+// Refactor with both substitutions, streams -> programs without -> with the mid
+// stage, ms: 2,000 buses, 128 groups FP32 2.15 -> 1.43 (none), 47 groups FP64
+// 5.94 -> 2.07 -> 1.74, one group FP32 2.07 -> 0.95 -> 0.73; 10,000 buses, 128
+// groups FP32 9.4 -> 4.9 (none); 20,000 buses, one group FP32 9.5 -> 3.8 -> 1.67;
+// 118 buses, one group FP64 0.41 -> 0.19 -> 0.156.
 #pragma once
 #include "gox_dot.hpp"
 #include "gox_kernels.cuh"
@@ -317,34 +323,44 @@ __global__ void __launch_bounds__(32 * kDotBinWarps) k_dot_bins(DotDev P, SchedD
   dot_bins_body<T, WHICH>(P, S, D, blockIdx.x, blockIdx.y);
 }
 
+// The launches of the tick kernels, and a group's CTAs in each.
+enum : int { DOT_IN_TOP = 0, DOT_IN_MID = 1, DOT_IN_PREP2 = 2 };
+__device__ __host__ __forceinline__ int dot_ctas(const DotDev& P, int stage) {
+  return stage == DOT_IN_MID ? P.n_mid : stage == DOT_IN_PREP2 ? P.n_prep2 : 1;
+}
+
 template <typename T, int NT>
-__device__ __forceinline__ void dot_top_body(const DotDev& P, const SchedDev& S, const BatchDev& D, int g) {
+__device__ __forceinline__ void dot_top_body(const DotDev& P, const SchedDev& S, const BatchDev& D, int stage,
+                                             int BX, int g) {
   __shared__ uint4 win[NT][64];
   __shared__ T sinv[kDotMaxMid * 2 * 32];
   __shared__ T sink[32];
   if (!D.gact[g]) return;
   const int warp = threadIdx.x >> 5;
-  dot_run<T, DOT_TOP>(P.words + P.top[warp], win[warp], S, D, g, sinv, sink);
+  const int32_t* start = stage == DOT_IN_MID ? P.mid : stage == DOT_IN_PREP2 ? P.prep2 : P.top;
+  dot_run<T, DOT_TOP>(P.words + start[BX * NT + warp], win[warp], S, D, g, sinv, sink);
 }
 template <typename T, int NT>
-__global__ void __launch_bounds__(32 * NT, 1) k_dot_top(DotDev P, SchedDev S, BatchDev D) {
-  dot_top_body<T, NT>(P, S, D, blockIdx.x);
+__global__ void __launch_bounds__(32 * NT, 1) k_dot_top(DotDev P, SchedDev S, BatchDev D, int stage) {
+  dot_top_body<T, NT>(P, S, D, stage, blockIdx.x, blockIdx.y);
 }
 template <typename T>
-__device__ __forceinline__ void dot_topback_body(const DotDev& P, const SchedDev& S, const BatchDev& D, int g) {
+__device__ __forceinline__ void dot_topback_body(const DotDev& P, const SchedDev& S, const BatchDev& D, int stage,
+                                                 int BX, int g) {
   __shared__ uint4 win[kDotBackWarps][64];
   __shared__ T sink[32];
   if (!D.gact[g]) return;
   const int warp = threadIdx.x >> 5;
-  dot_run<T, DOT_TOPBACK>(P.words + P.tback[warp], win[warp], S, D, g, (T*)nullptr, sink);
+  dot_run<T, DOT_TOPBACK>(P.words + (stage == DOT_IN_MID ? P.midback : P.tback)[BX * kDotBackWarps + warp], win[warp], S, D, g,
+                          (T*)nullptr, sink);
 }
 template <typename T>
-__global__ void __launch_bounds__(32 * kDotBackWarps, 1) k_dot_topback(DotDev P, SchedDev S, BatchDev D) {
-  dot_topback_body<T>(P, S, D, blockIdx.x);
+__global__ void __launch_bounds__(32 * kDotBackWarps, 1) k_dot_topback(DotDev P, SchedDev S, BatchDev D, int stage) {
+  dot_topback_body<T>(P, S, D, stage, blockIdx.x, blockIdx.y);
 }
 
 // The same over a list of jobs (their CTAs: kDotBinWarps streams each, group by
-// group; the top's: one per group).
+// group; the top's: one per group, the mid stage's: n_mid per group).
 __device__ __host__ __forceinline__ int dot_blocks(int streams) {
   return (streams + kDotBinWarps - 1) / kDotBinWarps;
 }
@@ -358,17 +374,18 @@ __global__ void __launch_bounds__(32 * kDotBinWarps) k_dot_bins_multi(const Mult
   dot_bins_body<T, WHICH>(J.dot, J.S, J.D, b % nb, b / nb);
 }
 template <typename T, int NT>
-__global__ void __launch_bounds__(32 * NT, 1) k_dot_top_multi(const MultiJob* __restrict__ jobs, MultiList L) {
+__global__ void __launch_bounds__(32 * NT, 1) k_dot_top_multi(const MultiJob* __restrict__ jobs, MultiList L,
+                                                                   int stage) {
   __shared__ __align__(16) MultiJob J;
-  const int b = enter_job(J, jobs, L);
-  dot_top_body<T, NT>(J.dot, J.S, J.D, b);
+  const int b = enter_job(J, jobs, L), nb = dot_ctas(J.dot, stage);
+  dot_top_body<T, NT>(J.dot, J.S, J.D, stage, b % nb, b / nb);
 }
 template <typename T>
 __global__ void __launch_bounds__(32 * kDotBackWarps, 1) k_dot_topback_multi(const MultiJob* __restrict__ jobs,
-                                                                              MultiList L) {
+                                                                              MultiList L, int stage) {
   __shared__ __align__(16) MultiJob J;
-  const int b = enter_job(J, jobs, L);
-  dot_topback_body<T>(J.dot, J.S, J.D, b);
+  const int b = enter_job(J, jobs, L), nb = stage == DOT_IN_MID ? J.dot.n_midback : 1;
+  dot_topback_body<T>(J.dot, J.S, J.D, stage, b % nb, b / nb);
 }
 
 }  // namespace gox

@@ -8,16 +8,21 @@
 // values, and a sum in pieces, as long as each value's own products stay in
 // order: the result is the stream form's (gox_stream.hpp) bit for bit.
 //
-// Five launches run a refactor with both substitutions:
+// Five to eight launches run a refactor with both substitutions:
 //   bottom    columns in independent parts of the elimination forest, whole
 //             parts assigned to bins; one warp runs a bin's sums in order and
 //             needs no barrier, since it wrote every value it reads
 //   prep      one warp per remaining column or two: the leading part of each
 //             of its sums that only needs bottom columns
-//   top       the rest of those columns, one CTA per group: the sums as
-//             units of up to 8 products spread over the warps, in ticks that
-//             only read values of earlier ticks, with a CTA barrier after each
+//   mid       (few groups) columns in independent parts of what is left, dealt
+//             out to a few CTAs per group: the sums as units of up to 8 products
+//             spread over the warps, in ticks that only read values of earlier
+//             ticks, with a CTA barrier after each
+//   prep 2    the leading parts of the remaining sums that the mid columns
+//             allow, a few columns per CTA, in ticks
+//   top       the rest of the columns, one CTA per group, in ticks
 //   top back  their backward rows, one CTA per group, in ticks too
+//   mid back  the mid columns' backward rows, CTA by CTA, in ticks
 //   back      the backward rows of the bottom columns, bin by bin
 #pragma once
 #include <cstdint>
@@ -68,6 +73,9 @@ struct DotPlan {
   int bins = 0;        // bins of the bottom (0: every column is in the top)
   int top_warps = 16;
   double cap = 1.0;    // largest part, of a bin's even share
+  int mid = 0;         // CTAs of the mid stage (0: none)
+  double mid_cap = 1.0;  // largest part, of such a CTA's even share
+  int prep_cols = 4;   // columns of a CTA of the prep after it
   int chain = 8;       // longest rows of a chain
   int pack = 3;        // longest sums that are packed by fours (0: none)
   int ahead = 2;       // ticks by which values are touched before their use (0: not)
@@ -77,16 +85,19 @@ struct DotPlan {
 struct DotProgram {
   DotPlan plan;
   std::vector<uint32_t> words;                   // all streams, 4 words per quad
-  std::vector<int32_t> bottom, prep, top, tback, back;  // per bin / warp: first quad of its stream
+  std::vector<int32_t> bottom, prep, mid, prep2, top, tback, midback, back;  // per bin / warp: first quad of its stream
   bool with_subst = false;                       // forward and backward substitution included
   int ticks = 0, back_ticks = 0;
-  int64_t units = 0, parts = 0, bottom_cols = 0, top_terms = 0, prep_terms = 0, touched = 0;
+  int64_t units = 0, parts = 0, bottom_cols = 0, mid_cols = 0, top_terms = 0, prep_terms = 0, touched = 0;
 };
 
 // The plan taken where nothing is timed, for `groups` groups of scenarios, and
 // the plans the autotuner times.
 DotPlan dot_default(const Schedule& sc, int elem, int groups);
-std::vector<DotPlan> dot_candidates(const Schedule& sc, int elem);
+std::vector<DotPlan> dot_candidates(const Schedule& sc, int elem, int groups);
+// Whether a plan made for few groups is the one to run `groups` groups with: an
+// SM for each CTA of the mid stage (three of them at least, the fewest that pay).
+bool dot_few(const DotPlan& p, int groups);
 
 // Compiles the refactor of a schedule (with both substitutions when the
 // schedule fuses the forward one).

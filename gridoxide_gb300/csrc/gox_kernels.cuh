@@ -725,8 +725,9 @@ struct StreamDev {
 // launch the first quad of each.
 struct DotDev {
   const uint4* words;
-  const int32_t *bottom, *prep, *top, *tback, *back;
-  int n_bottom, n_prep, n_top, n_tback, n_back;
+  const int32_t *bottom, *prep, *mid, *prep2, *top, *tback, *midback, *back;
+  int n_bottom, n_prep, n_top, n_tback, n_back;  // streams
+  int n_mid, n_prep2, n_midback;                 // CTAs
 };
 
 // Progress flags (plans with sync = 1).  A warp that has done its work of

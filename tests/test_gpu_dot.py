@@ -22,13 +22,13 @@ pytestmark = pytest.mark.gpu
 
 _CHILD = r"""
 import sys
-root, prec, warps, bins = sys.argv[1], int(sys.argv[2]), int(sys.argv[3]), int(sys.argv[4])
+root, prec, warps, bins, mid = sys.argv[1], *[int(x) for x in sys.argv[2:6]]
 sys.path.insert(0, root)
 import numpy as np
 import gridoxide_gb300 as gox
 from gridoxide_gb300 import grids as G
 from gridoxide_gb300 import solver as S
-for n in [int(x) for x in sys.argv[5:]]:
+for n in [int(x) for x in sys.argv[6:]]:
     g = G.family_grid(n, 3)
     yb = G.build_ybus(g)
     topo = {}
@@ -36,7 +36,7 @@ for n in [int(x) for x in sys.argv[5:]]:
         S.set_autotune(plan == "dot")
         topo[plan] = gox.Topology(yb, g.bus_type)
         assert topo[plan].prepare(g.p_spec, g.q_spec, g.vm, g.va)
-        for b in (1, 33, 70):
+        for b in (1, 33, 70) + ((1700,) if n <= 131 else ()):
             p, q = G.load_scenarios(g, b, 0.15, b)
             r = topo[plan].solve(p, q, g.vm, g.va, precision=prec)
             if plan == "streams":
@@ -45,16 +45,20 @@ for n in [int(x) for x in sys.argv[5:]]:
             for k in ("voltage_mag", "voltage_ang", "iterations", "status", "max_mismatch"):
                 np.testing.assert_array_equal(getattr(topo[b], k), getattr(r, k), err_msg=f"{n} {b} {k}")
     tu = topo["dot"].tuning(prec)
-    assert (tu["source"], tu["warps"], tu["chunk_words"], tu["wide_levels"]) == ("cached", warps, 128, bins), (n, tu)
+    assert (tu["source"], tu["warps"], tu["chunk_words"], tu["wide_levels"], tu["wide_phases"]) == (
+        "cached", warps, 128, bins, mid), (n, tu)
 print("same")
 """
 
 
-@pytest.mark.parametrize("precision,warps,bins,sizes", [
-    (0, 32, 0, (3, 5, 9, 30, 119)), (0, 16, 32, (131, 300)), (0, 32, 64, (700,)),
-    (1, 16, 0, (3, 5, 9, 30, 119)), (1, 16, 32, (131, 300)), (1, 16, 64, (700,))])
-def test_dot_plan_equals_streams(tmp_path, precision, warps, bins, sizes):
-    """precision: 0 mixed, 1 FP64 (the cache file's numbering)."""
+@pytest.mark.parametrize("precision,warps,bins,mid,sizes", [
+    (0, 32, 0, 0, (3, 5, 9, 30, 119)), (0, 16, 32, 0, (131, 300)), (0, 32, 64, 0, (700,)),
+    (1, 16, 0, 0, (3, 5, 9, 30, 119)), (1, 16, 32, 0, (131, 300)), (1, 16, 64, 0, (700,)),
+    (0, 32, 0, 3, (119, 131)), (0, 32, 64, 8, (700,)), (0, 32, 32, 16, (300,)),
+    (1, 16, 0, 3, (119, 131)), (1, 16, 64, 8, (700,)), (1, 16, 32, 4, (300,))])
+def test_dot_plan_equals_streams(tmp_path, precision, warps, bins, mid, sizes):
+    """precision: 0 mixed, 1 FP64 (the cache file's numbering); mid: CTAs of the
+    mid stage.  54 groups run the program for many groups."""
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     sys.path.insert(0, root)
     import gridoxide_gb300 as gox
@@ -63,9 +67,9 @@ def test_dot_plan_equals_streams(tmp_path, precision, warps, bins, sizes):
         for bb in range(0, 25):
             for fill in range(0, 60):
                 for gb in range(5):
-                    f.write(f"gox-tune-3 {precision} {bb} {fill} {gb} {warps} 128 0 {bins}\n")
+                    f.write(f"gox-tune-3 {precision} {bb} {fill} {gb} {warps} 128 {mid} {bins}\n")
     prec = (gox.GOX_PRECISION_MIXED, gox.GOX_PRECISION_FP64)[precision]
-    out = subprocess.run([sys.executable, "-c", _CHILD, root, str(int(prec)), str(warps), str(bins)] +
+    out = subprocess.run([sys.executable, "-c", _CHILD, root, str(int(prec)), str(warps), str(bins), str(mid)] +
                          [str(n) for n in sizes], env=dict(os.environ, GOX_TUNE_CACHE=str(cache)),
                          capture_output=True, text=True, timeout=600)
     assert out.returncode == 0, out.stderr[-3000:]
