@@ -1429,6 +1429,7 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st) {
   TU.done = true;
   if (!g_autotune.load()) return;
   const Schedule& sc = t->sc;
+  const bool fits = dot_fits(sc);
   const int elem = (int)sizeof(T);
   const std::array<int, 4> key = tune_key(t, i, D.G);
   {
@@ -1437,7 +1438,7 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st) {
     auto it = g_tune.find(key);
     if (it == g_tune.end() && t->tune_cache_only) {
       // not timed: the program the measured rule gives
-      install_dot(t, i, make_dot(sc, dot_default(sc, elem, D.G)), D.G, nullptr);
+      if (fits) install_dot(t, i, make_dot(sc, dot_default(sc, elem, D.G)), D.G, nullptr);
       return;
     }
     if (it != g_tune.end() && it->second[1] == kDotChunkWords) {
@@ -1449,7 +1450,7 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st) {
         if (p.top_warps == it->second[0] && p.bins == it->second[3] && p.mid <= it->second[2] &&
             (!found || p.mid > found->mid))
           found = &p;
-      if (found) {
+      if (found && fits) {
         install_dot(t, i, make_dot(sc, *found), D.G, nullptr);
         TU.source = 2;
         return;
@@ -1485,7 +1486,8 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st) {
   std::vector<StreamPlan> cand = candidate_plans(sc, elem, kRefactorSmem);
   std::vector<Stream> built(cand.size());
   std::vector<char> ok(cand.size(), 0);
-  std::vector<DotPlan> dcand = dot_candidates(sc, elem, D.G);
+  std::vector<DotPlan> dcand;
+  if (fits) dcand = dot_candidates(sc, elem, D.G);
   dcand.push_back(dot_other(sc, elem, D.G));  // (not timed)
   std::vector<std::shared_ptr<const DotProgram>> dbuilt(dcand.size());
   {
@@ -1888,7 +1890,7 @@ static void guess_build(gox_topo* t, const double* p0, const double* q0) {
   std::vector<double> dummy_x;
   G.dsched.load(G.sc, dummy_p, dummy_i, dummy_x, dummy_x);
   G.dsched.load_streams(G.s32, G.s64);
-  G.dsched.load_dot(1, DotPair{make_dot(G.sc, dot_default(G.sc, 8, 1)), make_dot(G.sc, dot_default(G.sc, 8, 152))});
+  if (dot_fits(G.sc)) G.dsched.load_dot(1, DotPair{make_dot(G.sc, dot_default(G.sc, 8, 1)), make_dot(G.sc, dot_default(G.sc, 8, 152))});
   // value recipe per LU slot, then per off-diagonal entry
   const int ns = G.sc.n_slots, no = G.sc.n_off;
   std::vector<int32_t> rec((size_t)(ns + no) * 4);
@@ -3843,7 +3845,7 @@ int gox_topo_emulate_step(const gox_topo* t, const double* jac_vals, const doubl
       if (!(lu[x] == lu64[x]) && !(std::isnan(lu[x]) && std::isnan(lu64[x])))
         throw std::runtime_error("the two refactor streams disagree");
     // ... and the dot programs of both precisions, the same factor again
-    for (int c = 0; c < 4; c++) {  // for few groups, for many
+    for (int c = 0; c < 4 && dot_fits(sc); c++) {  // for few groups, for many
       const int elem = c & 1 ? 8 : 4;
       DotProgram p;
       build_dot(sc, dot_default(sc, elem, c & 2 ? 152 : 1), p);
@@ -4300,7 +4302,7 @@ int gox_ls_create(int32_t n, int32_t nnz, const int32_t* rows, const int32_t* co
     std::vector<double> dummy_x;
     h->dsched.load(h->sc, dummy_p, dummy_i, dummy_x, dummy_x);
     h->dsched.load_streams(h->s32, h->s64);
-    h->dsched.load_dot(1, DotPair{make_dot(h->sc, dot_default(h->sc, 8, 1)), nullptr});
+    if (dot_fits(h->sc)) h->dsched.load_dot(1, DotPair{make_dot(h->sc, dot_default(h->sc, 8, 1)), nullptr});
     const SchedDev& S = h->dsched.d;
     h->jbuf.ensure((size_t)S.n_a * 32 * 8 + 8);
     h->lu.ensure((size_t)S.n_slots * 32 * 8 + 8);

@@ -84,7 +84,8 @@ struct Writer {
       const int m = std::min(n, kDotTerms);
       room(1 + (m + 1) / 2);
       last = w.size();
-      raw(op | (cin ? DOT_CIN : 0u) | (m < n ? DOT_COUT : 0u) | ((uint32_t)m << 12), y, z, 0u);
+      raw(op | (op == DOT_U && !cin && m == n ? DOT_PLAIN : 0u) | (cin ? DOT_CIN : 0u) | (m < n ? DOT_COUT : 0u) |
+              ((uint32_t)m << 12), y, z, 0u);
       for (int t = 0; t < m; t += 2) {
         const int u = t + 1 < m ? t + 1 : t;
         raw((uint32_t)a[t], (uint32_t)b[t], (uint32_t)a[u], (uint32_t)b[u]);
@@ -248,6 +249,7 @@ std::vector<DotPlan> dot_candidates(const Schedule& sc, int elem, int groups) {
 }
 
 void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
+  if (!dot_fits(sc)) throw std::runtime_error("too many slots for a dot program");
   P = DotProgram();
   P.plan = plan;
   const int n = sc.n_u, ns = sc.n_slots;
@@ -1106,6 +1108,7 @@ std::string run_dot_host(const Schedule& sc, const DotProgram& P, std::vector<do
         }
         continue;
       }
+      if ((h[0] & DOT_PLAIN) && (op != DOT_U || (h[0] & (DOT_CIN | DOT_COUT | DOT_FIRST)))) return fail("a plain unit with flags");
       const int m = (int)((h[0] >> 12) & 15u);
       const bool row = op == DOT_Y || op == DOT_B, cin = (h[0] & DOT_CIN) != 0, cout = (h[0] & DOT_COUT) != 0;
       if (op < DOT_U || op > DOT_B || m > kDotTerms || h[1] >= (uint32_t)(row ? n : ns)) return fail("a unit out of range");

@@ -25,9 +25,9 @@
 // depend on each other (20,000 buses, one warp per column 0.35 ms, depth by
 // depth over a CTA 0.35, with the sums' leading parts in earlier ticks 0.17).
 // Refactor with both substitutions, streams -> programs without -> with the mid
-// stage, ms: 2,000 buses, 128 groups FP32 2.15 -> 1.43 (none), 47 groups FP64
-// 5.94 -> 2.07 -> 1.74, one group FP32 2.07 -> 0.95 -> 0.73; 10,000 buses, 128
-// groups FP32 9.4 -> 4.9 (none); 20,000 buses, one group FP32 9.5 -> 3.8 -> 1.67;
+// stage, ms: 2,000 buses, 128 groups FP32 2.15 -> 1.32 (none), 47 groups FP64
+// 5.94 -> 2.07 -> 1.74, one group FP32 2.07 -> 0.95 -> 0.67; 10,000 buses, 128
+// groups FP32 9.4 -> 4.9 (none); 20,000 buses, one group FP32 9.5 -> 3.8 -> 1.52;
 // 118 buses, one group FP64 0.41 -> 0.19 -> 0.156.
 #pragma once
 #include "gox_dot.hpp"
@@ -35,49 +35,83 @@
 
 namespace gox {
 
-template <typename T>
+// A value's address.  O32: base is the group's and the lane's value lies at a
+// 32-bit offset from it (the base is the same for the whole grid row, so an
+// address is one 32-bit multiply-add and no 64-bit one); else base is the
+// lane's.  Measured (2,000 buses, 128 groups FP32, ms, 64-bit -> O32): top .604
+// -> .561, back .125 -> .100; the bottom and prep get slower (.256 -> .283, .217
+// -> .233: 48 registers, or 40 with fewer loads in flight), the top's backward
+// rows too (.236 -> .254).
+template <typename T, bool O32>
+__device__ __forceinline__ size_t dot_at(uint32_t row) {
+  if constexpr (O32) return (size_t)(row * (uint32_t)(32u * sizeof(T)) + (threadIdx.x & 31u) * (uint32_t)sizeof(T));
+  return (size_t)row * (32u * sizeof(T));
+}
+template <typename T, bool O32 = false>
 __device__ __forceinline__ T dot_ld(const char* base, uint32_t row) {
-  return *reinterpret_cast<const T*>(base + (size_t)row * (32u * sizeof(T)));
+  return *reinterpret_cast<const T*>(base + dot_at<T, O32>(row));
 }
 
-template <typename T>
+template <typename T, bool O32 = false>
 __device__ __forceinline__ void dot_st(char* base, uint32_t row, T v) {
-  *reinterpret_cast<T*>(base + (size_t)row * (32u * sizeof(T))) = v;
+  *reinterpret_cast<T*>(base + dot_at<T, O32>(row)) = v;
 }
 
 // M products at q: every load before the first multiply
-template <typename T, int M>
+template <typename T, int M, bool O32 = false>
 __device__ __forceinline__ void dot_terms(const uint4* q, const char* A, const char* B, T& v) {
   T a[M], b[M];
 #pragma unroll
   for (int t = 0; t < M; t += 2) {
     const uint4 e = q[t / 2];
-    a[t] = dot_ld<T>(A, e.x);
-    b[t] = dot_ld<T>(B, e.y);
+    a[t] = dot_ld<T, O32>(A, e.x);
+    b[t] = dot_ld<T, O32>(B, e.y);
     if (t + 1 < M) {
-      a[t + 1] = dot_ld<T>(A, e.z);
-      b[t + 1] = dot_ld<T>(B, e.w);
+      a[t + 1] = dot_ld<T, O32>(A, e.z);
+      b[t + 1] = dot_ld<T, O32>(B, e.w);
     }
   }
 #pragma unroll
   for (int t = 0; t < M; t++) v -= a[t] * b[t];
 }
 
+// n products (0 to 8) at p.  Comparisons, not a jump table: an indirect branch
+// costs more (one per unit over all units: the 2,000-bus top of one group FP32
+// .346 -> .385 ms; a switch over n as a table against this tree .346 / .330).
+template <typename T, bool O32 = false>
+__device__ __forceinline__ void dot_sum(int n, const uint4* p, const char* A, const char* B, T& v) {
+  if (n <= 4) {
+    if (n <= 2) {
+      if (n == 2) dot_terms<T, 2, O32>(p, A, B, v);
+      else if (n == 1) dot_terms<T, 1, O32>(p, A, B, v);
+    } else {
+      if (n == 3) dot_terms<T, 3, O32>(p, A, B, v);
+      else dot_terms<T, 4, O32>(p, A, B, v);
+    }
+  } else if (n <= 6) {
+    if (n == 5) dot_terms<T, 5, O32>(p, A, B, v);
+    else dot_terms<T, 6, O32>(p, A, B, v);
+  } else {
+    if (n == 7) dot_terms<T, 7, O32>(p, A, B, v);
+    else dot_terms<T, 8, O32>(p, A, B, v);
+  }
+}
+
 // Four sums of M products each at q (a quad of a's, then one of b's per product)
-template <typename T, int M>
+template <typename T, int M, bool O32 = false>
 __device__ __forceinline__ void dot_pack(const uint4* q, const char* A, const char* B, T* v) {
   T a[M][4], b[M][4];
 #pragma unroll
   for (int t = 0; t < M; t++) {
     const uint4 x = q[2 * t], y = q[2 * t + 1];
-    a[t][0] = dot_ld<T>(A, x.x);
-    a[t][1] = dot_ld<T>(A, x.y);
-    a[t][2] = dot_ld<T>(A, x.z);
-    a[t][3] = dot_ld<T>(A, x.w);
-    b[t][0] = dot_ld<T>(B, y.x);
-    b[t][1] = dot_ld<T>(B, y.y);
-    b[t][2] = dot_ld<T>(B, y.z);
-    b[t][3] = dot_ld<T>(B, y.w);
+    a[t][0] = dot_ld<T, O32>(A, x.x);
+    a[t][1] = dot_ld<T, O32>(A, x.y);
+    a[t][2] = dot_ld<T, O32>(A, x.z);
+    a[t][3] = dot_ld<T, O32>(A, x.w);
+    b[t][0] = dot_ld<T, O32>(B, y.x);
+    b[t][1] = dot_ld<T, O32>(B, y.y);
+    b[t][2] = dot_ld<T, O32>(B, y.z);
+    b[t][3] = dot_ld<T, O32>(B, y.w);
   }
 #pragma unroll
   for (int t = 0; t < M; t++)
@@ -161,12 +195,12 @@ __device__ __forceinline__ const uint4* dot_chain(const uint4* p, int rows, cons
 
 // four values into the L1: asynchronous copies (cached at every level) into a
 // row of shared memory that nobody reads
-template <typename T>
+template <typename T, bool O32 = false>
 __device__ __forceinline__ void dot_touch(const char* base, const uint4& q, uint32_t sink) {
   const uint32_t r[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
   for (int t = 0; t < 4; t++)
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(sink), "l"(base + (size_t)r[t] * (32u * sizeof(T))),
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(sink), "l"(base + dot_at<T, O32>(r[t])),
                  "n"((int)sizeof(T)) : "memory");
 }
 
@@ -183,7 +217,8 @@ __device__ __forceinline__ void dot_run(const uint4* __restrict__ gs, uint4* win
   constexpr bool BAR = WHICH == DOT_TOP || WHICH == DOT_TOPBACK;  // ticks
   constexpr bool FWD = WHICH != DOT_BACK && WHICH != DOT_TOPBACK;
   const int lane = threadIdx.x & 31;
-  const size_t lb = (size_t)lane * sizeof(T);
+  constexpr bool O32 = WHICH == DOT_TOP || WHICH == DOT_BACK;
+  const size_t lb = O32 ? 0 : (size_t)lane * sizeof(T);
   char* LU = (char*)D.lu + (size_t)g * S.n_slots * 32u * sizeof(T) + lb;
   char* X = (char*)D.sol + (size_t)g * S.n_u * 32u * sizeof(T) + lb;
   const char* R = (const char*)D.rhs + (size_t)g * S.n_u * 32u * sizeof(T) + lb;
@@ -207,32 +242,32 @@ __device__ __forceinline__ void dot_run(const uint4* __restrict__ gs, uint4* win
         const uint4 e = *p++;
         char* B = (h.x & DOT_ROW) ? X : LU;
         const char* F = (h.x & DOT_FIRST) ? R : B;
-        T x[4] = {dot_ld<T>(F, e.x), dot_ld<T>(F, e.y), dot_ld<T>(F, e.z), dot_ld<T>(F, e.w)};
+        T x[4] = {dot_ld<T, O32>(F, e.x), dot_ld<T, O32>(F, e.y), dot_ld<T, O32>(F, e.z), dot_ld<T, O32>(F, e.w)};
         switch ((h.x >> 12) & 15u) {
-          case 1: dot_pack<T, 1>(p, LU, B, x); p += 2; break;
-          case 2: dot_pack<T, 2>(p, LU, B, x); p += 4; break;
-          case 3: dot_pack<T, 3>(p, LU, B, x); p += 6; break;
+          case 1: dot_pack<T, 1, O32>(p, LU, B, x); p += 2; break;
+          case 2: dot_pack<T, 2, O32>(p, LU, B, x); p += 4; break;
+          case 3: dot_pack<T, 3, O32>(p, LU, B, x); p += 6; break;
           default: break;
         }
-        dot_st<T>(B, e.x, x[0]);
-        dot_st<T>(B, e.y, x[1]);
-        dot_st<T>(B, e.z, x[2]);
-        dot_st<T>(B, e.w, x[3]);
+        dot_st<T, O32>(B, e.x, x[0]);
+        dot_st<T, O32>(B, e.y, x[1]);
+        dot_st<T, O32>(B, e.z, x[2]);
+        dot_st<T, O32>(B, e.w, x[3]);
       } else if (FWD && op == DOT_FIN) {
         char* C = LU + (size_t)h.y * (32u * sizeof(T));
-        const T d = dot_ld<T>(C, 0);
+        const T d = dot_ld<T, O32>(C, 0);
         const T r = rcp_rn(d), pa = fabs(d);
         T m = pa;
         const int z = (int)h.z;
         for (int i = 1; i <= z; i += 4) {  // (the last entry again where fewer than four are left)
           const int i1 = min(i + 1, z), i2 = min(i + 2, z), i3 = min(i + 3, z);
-          const T x0 = dot_ld<T>(C, i), x1 = dot_ld<T>(C, i1), x2 = dot_ld<T>(C, i2), x3 = dot_ld<T>(C, i3);
+          const T x0 = dot_ld<T, O32>(C, i), x1 = dot_ld<T, O32>(C, i1), x2 = dot_ld<T, O32>(C, i2), x3 = dot_ld<T, O32>(C, i3);
           if (sizeof(T) == 4) m = fmax(fmax(m, fmax(fabs(x0), fabs(x1))), fmax(fabs(x2), fabs(x3)));
-          dot_st<T>(C, i, x0 * r);
+          dot_st<T, O32>(C, i, x0 * r);
           // (in FP64 a multiply costs more than a branch)
-          if (sizeof(T) == 4 || i1 != i) dot_st<T>(C, i1, x1 * r);
-          if (sizeof(T) == 4 || i2 != i1) dot_st<T>(C, i2, x2 * r);
-          if (sizeof(T) == 4 || i3 != i2) dot_st<T>(C, i3, x3 * r);
+          if (sizeof(T) == 4 || i1 != i) dot_st<T, O32>(C, i1, x1 * r);
+          if (sizeof(T) == 4 || i2 != i1) dot_st<T, O32>(C, i2, x2 * r);
+          if (sizeof(T) == 4 || i3 != i2) dot_st<T, O32>(C, i3, x3 * r);
         }
         bad |= d == (T)0;
         tiny |= ptol > 0.0f && (float)pa < ptol * (float)m;
@@ -248,8 +283,8 @@ __device__ __forceinline__ void dot_run(const uint4* __restrict__ gs, uint4* win
         __syncwarp();
         continue;
       } else if (BAR && op == DOT_TOUCH) {
-        for (uint32_t i = 0; i < h.y; i++) dot_touch<T>(LU, *p++, sink);
-        for (uint32_t i = 0; i < h.z; i++) dot_touch<T>(X, *p++, sink);
+        for (uint32_t i = 0; i < h.y; i++) dot_touch<T, O32>(LU, *p++, sink);
+        for (uint32_t i = 0; i < h.z; i++) dot_touch<T, O32>(X, *p++, sink);
         continue;
       } else if (BAR && op == DOT_BAR) {
         for (uint32_t i = 0; i < h.y; i++) __syncthreads();
@@ -258,23 +293,22 @@ __device__ __forceinline__ void dot_run(const uint4* __restrict__ gs, uint4* win
         break;  // DOT_END
       }
     } else {
+      if (FWD && (h.x & DOT_PLAIN)) {  // the most frequent unit: no other flag to look at
+        const int n = (int)((h.x >> 12) & 15u);
+        T s = dot_ld<T, O32>(LU, h.y);
+        dot_sum<T, O32>(n, p, LU, LU, s);
+        dot_st<T, O32>(LU, h.y, s);
+        p += (n + 1) >> 1;
+        if (BAR && (h.x & DOT_BARF)) __syncthreads();
+        continue;
+      }
       const bool row = !FWD || op >= DOT_Y;
       char* B = row ? X : LU;
-      if (!(h.x & DOT_CIN)) v = dot_ld<T>(FWD && (h.x & DOT_FIRST) ? R : B, h.y);
+      if (!(h.x & DOT_CIN)) v = dot_ld<T, O32>(FWD && (h.x & DOT_FIRST) ? R : B, h.y);
       T d = (T)1;
-      if (!FWD) d = dot_ld<T>(LU, h.z);
+      if (!FWD) d = dot_ld<T, O32>(LU, h.z);
       const int n = (int)((h.x >> 12) & 15u);
-      switch (n) {
-        case 1: dot_terms<T, 1>(p, LU, B, v); break;
-        case 2: dot_terms<T, 2>(p, LU, B, v); break;
-        case 3: dot_terms<T, 3>(p, LU, B, v); break;
-        case 4: dot_terms<T, 4>(p, LU, B, v); break;
-        case 5: dot_terms<T, 5>(p, LU, B, v); break;
-        case 6: dot_terms<T, 6>(p, LU, B, v); break;
-        case 7: dot_terms<T, 7>(p, LU, B, v); break;
-        case 8: dot_terms<T, 8>(p, LU, B, v); break;
-        default: break;
-      }
+      dot_sum<T, O32>(n, p, LU, B, v);
       p += (n + 1) >> 1;
       if (h.x & DOT_COUT) continue;
       T out = v;
@@ -296,7 +330,7 @@ __device__ __forceinline__ void dot_run(const uint4* __restrict__ gs, uint4* win
         tiny |= ptol > 0.0f && (float)fabs(piv) < ptol * (float)fabs(v);
         out = v * inv;
       }
-      dot_st<T>(B, h.y, out);
+      dot_st<T, O32>(B, h.y, out);
     }
     if (BAR && (h.x & DOT_BARF)) __syncthreads();
   }
@@ -306,6 +340,10 @@ __device__ __forceinline__ void dot_run(const uint4* __restrict__ gs, uint4* win
 }
 
 constexpr int kDotBinWarps = 8;  // streams per CTA of the bin launches
+// CTAs of an SM: 40 registers in FP32 and for the backward rows, 64 in FP64 (72
+// and 88 where the compiler may: 2,000 buses, 128 groups FP32, the whole
+// refactor 1.47 ms against 1.33)
+constexpr int dot_bin_ctas(size_t elem, int which) { return elem == 4 || which == DOT_BACK ? 6 : 4; }
 
 template <typename T, int WHICH>
 __device__ __forceinline__ void dot_bins_body(const DotDev& P, const SchedDev& S, const BatchDev& D, int BX,
@@ -319,7 +357,8 @@ __device__ __forceinline__ void dot_bins_body(const DotDev& P, const SchedDev& S
   dot_run<T, WHICH>(P.words + start[b], win[warp], S, D, g, (T*)nullptr, (T*)nullptr);
 }
 template <typename T, int WHICH>
-__global__ void __launch_bounds__(32 * kDotBinWarps) k_dot_bins(DotDev P, SchedDev S, BatchDev D) {
+__global__ void __launch_bounds__(32 * kDotBinWarps, dot_bin_ctas(sizeof(T), WHICH))
+    k_dot_bins(DotDev P, SchedDev S, BatchDev D) {
   dot_bins_body<T, WHICH>(P, S, D, blockIdx.x, blockIdx.y);
 }
 
@@ -365,8 +404,8 @@ __device__ __host__ __forceinline__ int dot_blocks(int streams) {
   return (streams + kDotBinWarps - 1) / kDotBinWarps;
 }
 template <typename T, int WHICH>
-__global__ void __launch_bounds__(32 * kDotBinWarps) k_dot_bins_multi(const MultiJob* __restrict__ jobs,
-                                                                       MultiList L) {
+__global__ void __launch_bounds__(32 * kDotBinWarps, dot_bin_ctas(sizeof(T), WHICH))
+    k_dot_bins_multi(const MultiJob* __restrict__ jobs, MultiList L) {
   __shared__ __align__(16) MultiJob J;
   const int b = enter_job(J, jobs, L);
   const int n = WHICH == DOT_BOTTOM ? J.dot.n_bottom : WHICH == DOT_PREP ? J.dot.n_prep : J.dot.n_back;

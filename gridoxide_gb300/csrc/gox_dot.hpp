@@ -25,6 +25,7 @@
 //   mid back  the mid columns' backward rows, CTA by CTA, in ticks
 //   back      the backward rows of the bottom columns, bin by bin
 #pragma once
+#include <algorithm>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -36,7 +37,7 @@ namespace gox {
 // A stream is a list of 16-byte quads in chunks of 32.  A unit is one header
 // quad, then its products (a, b), two per quad, all in one chunk:
 //   x = op | barrier after << 4 | first << 5 | carry in << 6 | carry out << 7 |
-//       mid << 8 | n << 12
+//       mid << 8 | n << 12 | row << 16 | plain << 17 (U without a carry)
 //   y = the value's slot (U, D, LH) or row (Y, B); BAR: how many
 //   z = D, LH: threads of the mid barrier | shared index << 16;  B: pivot slot
 // a and b are LU slots (U, D, LH), or an LU slot and a row (Y, B).  A sum of
@@ -61,7 +62,7 @@ enum : uint32_t {
   DOT_B = 11     // x_k
 };
 constexpr uint32_t DOT_BARF = 1u << 4, DOT_FIRST = 1u << 5, DOT_CIN = 1u << 6, DOT_COUT = 1u << 7,
-                   DOT_ROW = 1u << 16, DOT_NEXT = 1u << 16;
+                   DOT_ROW = 1u << 16, DOT_NEXT = 1u << 16, DOT_PLAIN = 1u << 17;
 constexpr int kDotTerms = 8;    // products of a unit
 constexpr int kDotBackWarps = 16;  // warps of the top's backward CTA
 // products of a chain's row (two rows in registers)
@@ -90,6 +91,10 @@ struct DotProgram {
   int ticks = 0, back_ticks = 0;
   int64_t units = 0, parts = 0, bottom_cols = 0, mid_cols = 0, top_terms = 0, prep_terms = 0, touched = 0;
 };
+
+// Programs address a group's values by 32-bit byte offsets: a matrix with more
+// slots (some 16 million, an 800,000-bus grid) keeps the streams.
+inline bool dot_fits(const Schedule& sc) { return (int64_t)std::max(sc.n_slots, sc.n_u) * 256 < ((int64_t)1 << 32); }
 
 // The plan taken where nothing is timed, for `groups` groups of scenarios, and
 // the plans the autotuner times.
