@@ -15,7 +15,8 @@ CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libgridoxide_gb300.so")
 OBJ = os.path.join(HERE, "_build")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-SOURCES = ["gox_symbolic.cpp", "gox_engine.cpp", "gox_stream.cpp", "gox_dot.cpp", "gox_api.cu"]
+SOURCES = ["gox_symbolic.cpp", "gox_engine.cpp", "gox_stream.cpp", "gox_dot.cpp", "gox_solo.cpp",
+           "gox_api.cu"]
 
 
 def _nvcc() -> str:

@@ -25,9 +25,11 @@
 #include "../../include/gridoxide_gb300.h"
 #include "gox_engine.hpp"
 #include "gox_dot.hpp"
+#include "gox_solo.hpp"
 #include "gox_stream.hpp"
 #include "gox_kernels.cuh"
 #include "gox_dot.cuh"
+#include "gox_solo.cuh"
 #include "gox_pivot.cuh"
 
 namespace gox {
@@ -341,10 +343,49 @@ struct DevSchedule {
     DotOne few, many;
     const DotDev& pick(int groups) const { return groups <= few_groups ? few.d : many.d; }
   } dot[2];
+  // solo programs beside the dot programs: the one for the fewest scenarios
+  // first; max: the most scenarios it runs
+  struct SoloOne {
+    int max = 0;
+    DevMem words, lists, ctas;
+    SoloDev d{};
+  } solo[2][2];
+  const SoloOne* pick_solo(int i, int nb) const {
+    if (dot[i].on && nb > 0)
+      for (const SoloOne& x : solo[i])
+        if (nb <= x.max) return &x;
+    return nullptr;
+  }
+  // (null: none)
+  static void load_solo(SoloOne& x, const SoloProgram* p, int stride) {
+    x.max = 0;
+    if (!p) return;
+    upload(x.words, p->words);
+    upload(x.lists, p->lists);
+    std::vector<SoloCta> all;
+    for (const auto& l : p->launch) all.insert(all.end(), l.begin(), l.end());
+    upload(x.ctas, all);
+    x.d.words = x.words.as<uint4>();
+    x.d.lists = x.lists.as<uint32_t>();
+    const SoloCta* at = x.ctas.as<SoloCta>();
+    for (int i = 0; i < 4; i++) {
+      x.d.cta[i] = at;
+      x.d.ctas[i] = (int)p->launch[i].size();
+      x.d.bytes[i] = kSoloRingBytes + p->max_values[i] * p->plan.elem;
+      at += p->launch[i].size();
+    }
+    x.d.stride = stride;
+    x.max = solo_scenarios(*p);
+  }
   // the plan's substitutions are part of its refactor
   bool has_bwd(int i) const { return dot[i].on ? dot[i].with_subst : st_bwd[i]; }
   // launches of one refactor (with both substitutions when the plan has them)
-  int refactor_launches(int i, int groups) const {
+  int refactor_launches(int i, int groups, int nb) const {
+    if (const SoloOne* x = pick_solo(i, nb)) {
+      int n = 0;
+      for (int c : x->d.ctas) n += c > 0;
+      return n;
+    }
     if (dot[i].on) {
       const DotDev& d = dot[i].pick(groups);
       return 1 + (d.n_bottom > 0) + (d.n_prep > 0) + (d.n_mid > 0) + (d.n_prep2 > 0) + (d.n_tback > 0) +
@@ -640,6 +681,29 @@ static std::shared_ptr<const DotProgram> make_dot(const Schedule& sc, const DotP
   return p;
 }
 
+// A solo program, checked likewise (null: there is none).
+static std::shared_ptr<const SoloProgram> make_solo(const Schedule& sc, int elem, bool wide) {
+  auto p = std::make_shared<SoloProgram>();
+  if (!build_solo_default(sc, elem, wide, *p)) return nullptr;
+  std::vector<double> lu(sc.n_slots, 1.0), rhs(sc.n_u, 0.0), X;
+  bool sing = false;
+  const std::string e = run_solo_host(sc, *p, lu, rhs, X, sing);
+  if (!e.empty()) throw std::runtime_error("solo program check: " + e);
+  return p;
+}
+// The solo programs of a schedule: one for the fewest scenarios and, where that
+// one has several CTAs, one for more.
+struct SoloPair {
+  bool tried = false;
+  std::shared_ptr<const SoloProgram> p[2];
+};
+static void make_solos(const Schedule& sc, int elem, SoloPair& x) {
+  x.tried = true;
+  x.p[0] = make_solo(sc, elem, true);
+  if (x.p[0] && x.p[0]->ctas() > 1) x.p[1] = make_solo(sc, elem, false);
+  if (x.p[1] && x.p[1]->ctas() == x.p[0]->ctas()) x.p[1].reset();
+}
+
 struct Timing {
   bool on = false;
   double iters = 0, total = 0, k1 = 0, k2 = 0, k3 = 0, k4 = 0;
@@ -678,6 +742,10 @@ struct Iter {
   }
   static void refactor(const DevSchedule& ds, const BatchDev& D, cudaStream_t st) {
     const int i = sizeof(T) == 4 ? 0 : 1;
+    if (const auto* x = ds.pick_solo(i, D.nb)) {
+      solo(x->d, ds.d, D, st);
+      return;
+    }
     if (ds.dot[i].on) {
       dot(ds.dot[i].pick(D.G), ds.d, D, D.G, st);
       return;
@@ -723,6 +791,16 @@ struct Iter {
       if constexpr (sizeof(T) == 4) GOX_CK(cudaFuncSetAttribute(k_dot_top<T, 32>, a, 20));
       GOX_CK(cudaFuncSetAttribute(k_dot_topback<T>, a, 20));
     });
+  }
+  static void solo(const SoloDev& P, const SchedDev& S, const BatchDev& D, cudaStream_t st) {
+    static std::once_flag once[64];
+    int dev = 0;
+    GOX_CK(cudaGetDevice(&dev));
+    std::call_once(once[dev & 63], [] {
+      GOX_CK(cudaFuncSetAttribute(k_solo<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSoloRingBytes + kSoloMaxBytes));
+    });
+    for (int i = 0; i < 4; i++)
+      if (P.ctas[i] > 0) k_solo<T><<<dim3(P.ctas[i], D.nb), 32 * kSoloWarps, P.bytes[i], st>>>(P, S, D, i);
   }
   template <int WHICH>
   static void dot_bins(const DotDev& P, const SchedDev& S, const BatchDev& D, int n, int groups, cudaStream_t st) {
@@ -875,6 +953,8 @@ struct gox_topo {
   // streams), and the one the tuner chose or found
   DotPair dot[2];
   std::shared_ptr<const DotProgram> dot_main[2];
+  SoloPair solo[2];            // beside them, from the topology's second solve of few scenarios on
+  int small_solves[2] = {0, 0};
   DevSchedule dsched;
   DevBatch batch;
   // re-packing: the smaller batch the running scenarios move to, and their
@@ -1073,6 +1153,7 @@ static int fix_pivots(gox_topo* t, int B, const double* p_spec, const double* q_
       for (int i = 0; i < 2; i++) {
         t->dot[i] = DotPair();
         t->dot_main[i].reset();
+        t->solo[i] = SoloPair();
       }
       t->factored = true;
       t->uploaded = false;
@@ -1088,7 +1169,10 @@ static int fix_pivots(gox_topo* t, int B, const double* p_spec, const double* q_
 static void upload_plans(gox_topo* t) {
   t->dsched.load(t->sc, t->yp, t->yi, t->yre, t->yim);
   t->dsched.load_streams(t->s32, t->s64);
-  for (int i = 0; i < 2; i++) t->dsched.load_dot(i, t->dot[i]);
+  for (int i = 0; i < 2; i++) {
+    t->dsched.load_dot(i, t->dot[i]);
+    for (int k = 0; k < 2; k++) DevSchedule::load_solo(t->dsched.solo[i][k], t->solo[i].p[k].get(), 32);
+  }
   t->uploaded = true;
 }
 
@@ -1422,6 +1506,14 @@ static void install_stream(gox_topo* t, int i, Stream&& s) {
   }
 }
 
+// Before a solve of B scenarios: the solo programs, where one may run them.  Not
+// at the first such solve: a topology that is used once does not pay for them.
+static void ensure_solo(gox_topo* t, int i, int B) {
+  if (B > 1216 || !t->dot_main[i] || t->solo[i].tried || !t->uploaded || ++t->small_solves[i] < 2) return;
+  make_solos(t->sc, i == 0 ? 4 : 8, t->solo[i]);
+  for (int k = 0; k < 2; k++) DevSchedule::load_solo(t->dsched.solo[i][k], t->solo[i].p[k].get(), 32);
+}
+
 template <typename T>
 static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st) {
   const int i = sizeof(T) == 4 ? 0 : 1;
@@ -1723,7 +1815,7 @@ static void run_iterations(gox_topo* t, BatchDev D, int max_iter, bool outage, c
     const int its = h[1], ran_out = (h[0] > 0 && its >= max_iter) ? 1 : 0;
     const int fills = h[0] > 0 ? its : its - 1;
     const int ns = t->dsched.has_bwd(sizeof(T) == 4 ? 0 : 1) ? 0 : 1;
-    const int nr = t->dsched.refactor_launches(sizeof(T) == 4 ? 0 : 1, D.G);
+    const int nr = t->dsched.refactor_launches(sizeof(T) == 4 ? 0 : 1, D.G, D.nb);
     t->launches += (int64_t)its * 4 + (int64_t)fills * (1 + nr + ns) + ran_out * 2;
     return;
   }
@@ -1774,7 +1866,7 @@ static void run_iterations(gox_topo* t, BatchDev D, int max_iter, bool outage, c
       ns = Iter<T>::solve_rest(t->dsched, D, st);
     }
     rec();
-    t->launches += 1 + t->dsched.refactor_launches(sizeof(T) == 4 ? 0 : 1, D.G) + ns;
+    t->launches += 1 + t->dsched.refactor_launches(sizeof(T) == 4 ? 0 : 1, D.G, D.nb) + ns;
     GOX_CK(cudaGetLastError());
   }
   if (it == max_iter) t->launches += Iter<T>::mismatch(S, D, max_iter, 1, outage, st);
@@ -2131,6 +2223,7 @@ static int batch_prepare(gox_topo* t, int B, const double* p_spec, const double*
   DevBatch& DB = t->batch;
   DB.ensure(S, G, precision, max_iter, want_hist);
   BatchDev D = DB.view(want_hist, outage, tol, t->piv_tol);
+  D.nb = B;
   // inputs -> interleaved layout
   const size_t tot = (size_t)G * n * 32;
   k_scatter_rows<<<grid1d(tot), 256, 0, st>>>(p_spec, B, n, n, D.psp, G);
@@ -3052,6 +3145,7 @@ static std::unique_ptr<gox_topo> clone_factored(const gox_topo* t) {
   for (int i = 0; i < 2; i++) {
     v->dot[i] = t->dot[i];
     v->dot_main[i] = t->dot_main[i];
+    v->solo[i] = t->solo[i];
   }
   v->factored = true;
   v->uploaded = false;
@@ -3113,7 +3207,11 @@ static int batch_split(gox_topo* t, int B, const double* p_spec, const double* q
   // 10,000-bus N-1 batch of 8,192: 4 parts 117-121 ms, 2 parts 122-124 ms
   // with host buffers; the 2,000-bus batch of 4,096 alike for 2, 4 and 8)
   const int want = t->split_parts > 0 ? t->split_parts : (B >= 8192 ? 4 : 2);
-  if (t->factored) ensure_dot_kind(t, precision == GOX_PRECISION_MIXED ? 0 : 1, (B + 31) / 32);
+  if (t->factored) {
+    const int i = precision == GOX_PRECISION_MIXED ? 0 : 1;
+    ensure_dot_kind(t, i, (B + 31) / 32);
+    ensure_solo(t, i, B);
+  }
   if (want < 2 || !t->factored || t->guess_mode != 0 || t->timing.on ||
       B < kSplitMinScenarios || precision != GOX_PRECISION_MIXED || !t->tune[0].done)
     return batch_any(t, B, p_spec, q_spec, vm0, va0, v_stride, o_slot, o_dre, o_dim, tol, max_iter,
@@ -3286,6 +3384,7 @@ int gox_topo_reset(gox_topo* t) {
   for (int i = 0; i < 2; i++) {
     t->dot[i] = DotPair();
     t->dot_main[i].reset();
+    t->solo[i] = SoloPair();
   }
   t->tune[0] = gox_topo::Tuning();
   t->tune[1] = gox_topo::Tuning();
@@ -3861,6 +3960,22 @@ int gox_topo_emulate_step(const gox_topo* t, const double* jac_vals, const doubl
       for (int x = 0; x < n && t->s32.has_bwd && p.with_subst; x++)
         if (differ(X[x], Xd[x])) throw std::runtime_error("the dot program's solution differs from the streams'");
     }
+    // ... and the solo programs, of both precisions and for one and many
+    for (int c = 0; c < 4; c++) {
+      SoloProgram p;
+      if (!build_solo_default(sc, c & 1 ? 8 : 4, (c & 2) != 0, p)) continue;
+      std::vector<double> lud(sc.n_slots, 0.0), Xd;
+      for (int x = 0; x < sc.n_slots; x++)
+        lud[x] = sc.slot_a[x] >= 0 ? packed[sc.a_csc[sc.slot_a[x]]] : 0.0;
+      bool singd = false;
+      const std::string ed = run_solo_host(sc, p, lud, b, Xd, singd);
+      if (!ed.empty()) throw std::runtime_error("solo program: " + ed);
+      auto differ = [](double x, double y) { return !(x == y) && !(std::isnan(x) && std::isnan(y)); };
+      for (int x = 0; x < sc.n_slots; x++)
+        if (differ(lu[x], lud[x])) throw std::runtime_error("the solo program's factor differs from the streams'");
+      for (int x = 0; x < n && t->s32.has_bwd; x++)
+        if (differ(X[x], Xd[x])) throw std::runtime_error("the solo program's solution differs from the streams'");
+    }
     bad = sing32;
     if (t->s32.has_bwd != t->s64.has_bwd) throw std::runtime_error("stream plans disagree");
     for (int x = 0; x < n && t->s32.has_bwd; x++)
@@ -4303,6 +4418,7 @@ int gox_ls_create(int32_t n, int32_t nnz, const int32_t* rows, const int32_t* co
     h->dsched.load(h->sc, dummy_p, dummy_i, dummy_x, dummy_x);
     h->dsched.load_streams(h->s32, h->s64);
     if (dot_fits(h->sc)) h->dsched.load_dot(1, DotPair{make_dot(h->sc, dot_default(h->sc, 8, 1)), nullptr});
+    if (auto p = make_solo(h->sc, 8, true)) DevSchedule::load_solo(h->dsched.solo[1][0], p.get(), 1);
     const SchedDev& S = h->dsched.d;
     h->jbuf.ensure((size_t)S.n_a * 32 * 8 + 8);
     h->lu.ensure((size_t)S.n_slots * 32 * 8 + 8);
@@ -4323,12 +4439,15 @@ static int ls_run(gox_ls* h, const double* vals, const double* rhs, double* x) {
   // pack duplicates, A order, replicate to all 32 lanes
   std::fill(h->packed.begin(), h->packed.end(), 0.0);
   for (size_t e = 0; e < h->rows.size(); e++) h->packed[h->csc.slot_of[e]] += vals[e];
-  // A values in the factor's layout (zeros at fill-in), replicated to 32 lanes
-  h->hostbuf.assign((size_t)S.n_slots * 32, 0.0);
+  // A values in the factor's layout (zeros at fill-in), replicated to 32 lanes;
+  // a solo program has one scenario's values only
+  const bool solo = h->dsched.pick_solo(1, 1) != nullptr;
+  const int lanes = solo ? 1 : 32;
+  h->hostbuf.assign((size_t)S.n_slots * lanes, 0.0);
   for (int x = 0; x < S.n_slots; x++) {
     const int a = h->sc.slot_a[x];
     if (a >= 0)
-      for (int l = 0; l < 32; l++) h->hostbuf[(size_t)x * 32 + l] = h->packed[h->sc.a_csc[a]];
+      for (int l = 0; l < lanes; l++) h->hostbuf[(size_t)x * lanes + l] = h->packed[h->sc.a_csc[a]];
   }
   GOX_CK(cudaMemcpy(h->lu.p, h->hostbuf.data(), h->hostbuf.size() * 8, cudaMemcpyHostToDevice));
   if (h->sc.n_off > 0) {
@@ -4337,13 +4456,14 @@ static int ls_run(gox_ls* h, const double* vals, const double* rhs, double* x) {
       for (int l = 0; l < 32; l++) ob[(size_t)x * 32 + l] = h->packed[h->sc.a_csc[h->sc.off_a[x]]];
     GOX_CK(cudaMemcpy(h->off.p, ob.data(), ob.size() * 8, cudaMemcpyHostToDevice));
   }
-  std::vector<double> b((size_t)n * 32);
+  std::vector<double> b((size_t)n * lanes);
   for (int k = 0; k < n; k++)
-    for (int l = 0; l < 32; l++) b[(size_t)k * 32 + l] = rhs[h->num.Pnum[k]];
+    for (int l = 0; l < lanes; l++) b[(size_t)k * lanes + l] = rhs[h->num.Pnum[k]];
   GOX_CK(cudaMemcpy(h->rhs.p, b.data(), b.size() * 8, cudaMemcpyHostToDevice));
   GOX_CK(cudaMemset(h->sing.p, 0, 128));
   BatchDev D{};
   D.G = 1;
+  D.nb = solo ? 1 : 0;
   D.jbuf = h->jbuf.p; D.lu = h->lu.p; D.off = h->off.p; D.rhs = h->rhs.p; D.sol = h->sol.p;
   D.sing = h->sing.as<int32_t>(); D.piv_flag = h->piv.as<int32_t>(); D.gact = h->gact.as<int32_t>();
   D.piv_tol = 0.0f;
@@ -4355,13 +4475,13 @@ static int ls_run(gox_ls* h, const double* vals, const double* rhs, double* x) {
   int32_t werr = 0;
   GOX_CK(cudaMemcpy(&werr, h->status.as<int32_t>() + 8, 4, cudaMemcpyDeviceToHost));
   if (werr) return GOX_E_DEVICE_WAIT;
-  std::vector<double> X((size_t)n * 32);
+  std::vector<double> X((size_t)n * lanes);
   int32_t sing = 0;
   GOX_CK(cudaMemcpy(X.data(), h->sol.p, X.size() * 8, cudaMemcpyDeviceToHost));
   GOX_CK(cudaMemcpy(&sing, h->sing.p, 4, cudaMemcpyDeviceToHost));
   bool finite = true;
   for (int k = 0; k < n; k++) {
-    double v = X[(size_t)k * 32];
+    double v = X[(size_t)k * lanes];
     x[h->sym.Q[k]] = v;
     if (!std::isfinite(v)) finite = false;
   }

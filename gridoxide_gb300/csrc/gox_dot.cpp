@@ -1,5 +1,6 @@
 // Compiler and checking interpreter of the dot-product programs.
 #include "gox_dot.hpp"
+#include "gox_sums.hpp"
 
 #include <algorithm>
 #include <cmath>
@@ -10,48 +11,6 @@
 namespace gox {
 
 namespace {
-
-// The sums of a schedule: per value its ordered terms.  Values are numbered
-// LU slots first, then y (row k at n_slots + k).
-struct Sums {
-  std::vector<int32_t> ptr, a, b;  // value -> terms
-  std::vector<int32_t> col;        // LU slot -> column
-};
-
-Sums make_sums(const Schedule& sc) {
-  Sums s;
-  const int n = sc.n_u, ns = sc.n_slots;
-  s.ptr.assign((size_t)ns + n + 1, 0);
-  s.col.assign(ns, 0);
-  for (int k = 0; k < n; k++) {
-    const int base = sc.c_base[k];
-    for (int d = 0; d < sc.c_ulen[k] + 1 + sc.c_llen[k]; d++) s.col[base + d] = k;
-    for (int e = sc.cu_ptr[k]; e < sc.cu_ptr[k + 1]; e++)
-      for (int t = sc.cu_dptr[e]; t < sc.cu_dptr[e + 1]; t++) s.ptr[base + sc.cu_dst[t] + 1]++;
-    if (sc.fuse_fwd) s.ptr[ns + k + 1] += sc.fw_ptr[k + 1] - sc.fw_ptr[k];
-  }
-  for (size_t v = 0; v + 1 < s.ptr.size(); v++) s.ptr[v + 1] += s.ptr[v];
-  s.a.assign(s.ptr.back(), 0);
-  s.b.assign(s.ptr.back(), 0);
-  std::vector<int32_t> at(s.ptr.begin(), s.ptr.end() - 1);
-  for (int k = 0; k < n; k++) {
-    const int base = sc.c_base[k];
-    for (int e = sc.cu_ptr[k]; e < sc.cu_ptr[k + 1]; e++) {
-      const int j = sc.cu_j[e], l0 = sc.c_base[j] + sc.c_ulen[j] + 1;
-      for (int t = sc.cu_dptr[e]; t < sc.cu_dptr[e + 1]; t++) {
-        const int v = base + sc.cu_dst[t];
-        s.a[at[v]] = l0 + (t - sc.cu_dptr[e]);
-        s.b[at[v]++] = base + (e - sc.cu_ptr[k]);
-      }
-    }
-    if (sc.fuse_fwd)
-      for (int t = sc.fw_ptr[k]; t < sc.fw_ptr[k + 1]; t++) {
-        s.a[at[ns + k]] = sc.fw_slot[t];
-        s.b[at[ns + k]++] = sc.fw_col[t];
-      }
-  }
-  return s;
-}
 
 // Rough cycles of n products on one warp (only their proportions matter:
 // they balance bins and warps)
@@ -263,81 +222,17 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
   // ---- bottom: parts of the elimination forest of at most cap * (total /
   // bins) cost, grown column by column (a column joins when everything it
   // depends on is in the bottom and the part it makes stays small enough)
-  std::vector<double> ccost(n, 0.0);
-  double total = 0;
-  for (int k = 0; k < n; k++) {
-    ccost[k] = 300.0 + 12.0 * len(k);
-    for (int e = sc.cu_ptr[k]; e < sc.cu_ptr[k + 1]; e++) ccost[k] += 40.0 + 8.0 * (sc.cu_dptr[e + 1] - sc.cu_dptr[e]);
-    if (subst) ccost[k] += 8.0 * nt(ns + k);
-    total += ccost[k];
-  }
-  std::vector<char> stage(n, 2);  // 0 bottom, 1 mid, 2 top
-  std::vector<int32_t> part(n), cta(n, -1);  // union-find parent; the mid column's CTA
-  std::vector<double> pcost(n, 0.0);
-  auto find = [&](int k) {
-    while (part[k] != k) k = part[k] = part[part[k]];
-    return k;
-  };
-  // columns into stage st: those whose dependences are in earlier stages or in a
-  // part of theirs, as long as their part is small enough
-  auto grow_parts = [&](char st, double cap) {
-    std::vector<int32_t> roots;
-    for (int k = 0; k < n; k++) {
-      if (stage[k] < st) continue;
-      bool ok = true;
-      roots.clear();
-      double c = ccost[k];
-      auto dep = [&](int j) {
-        if (stage[j] < st) return;
-        if (stage[j] > st) { ok = false; return; }
-        const int r = find(j);
-        if (std::find(roots.begin(), roots.end(), r) == roots.end()) {
-          roots.push_back(r);
-          c += pcost[r];
-        }
-      };
-      for (int e = sc.cu_ptr[k]; ok && e < sc.cu_ptr[k + 1]; e++) dep(sc.cu_j[e]);
-      if (subst)
-        for (int t = sc.fw_ptr[k]; ok && t < sc.fw_ptr[k + 1]; t++) dep(sc.fw_col[t]);
-      if (!ok || c > cap) continue;
-      stage[k] = st;
-      part[k] = k;
-      for (int r : roots) part[r] = k;
-      pcost[k] = c;
-    }
-  };
-  // a stage's parts to its workers, largest first onto the least loaded one
-  auto deal_parts = [&](char st, int workers) {
-    std::vector<std::vector<int32_t>> members(n), out(workers);
-    std::vector<int32_t> parts;
-    for (int k = 0; k < n; k++)
-      if (stage[k] == st) {
-        const int r = find(k);
-        members[r].push_back(k);
-        if (r == k) parts.push_back(k);
-      }
-    std::stable_sort(parts.begin(), parts.end(), [&](int x, int y) { return pcost[x] > pcost[y]; });
-    std::priority_queue<std::pair<double, int>, std::vector<std::pair<double, int>>, std::greater<>> q;
-    for (int b = 0; b < workers; b++) q.push({0.0, b});
-    for (int r : parts) {
-      auto [c, b] = q.top();
-      q.pop();
-      out[b].insert(out[b].end(), members[r].begin(), members[r].end());
-      q.push({c + pcost[r], b});
-    }
-    return out;
-  };
+  Parts parts(sc, S);
+  const std::vector<char>& stage = parts.stage;
+  std::vector<int32_t> cta(n, -1);  // the mid column's CTA
   std::vector<std::vector<int32_t>> bin, mid;
   if (plan.bins > 0) {
-    grow_parts(0, plan.cap * total / plan.bins);
-    bin = deal_parts(0, plan.bins);
+    parts.grow(0, plan.cap * parts.cost_from(0) / plan.bins);
+    bin = parts.deal(0, plan.bins);
   }
   if (plan.mid > 0) {
-    double rest = 0;
-    for (int k = 0; k < n; k++)
-      if (stage[k] > 0) rest += ccost[k];
-    grow_parts(1, plan.mid_cap * rest / plan.mid);
-    for (auto& m : deal_parts(1, plan.mid)) {
+    parts.grow(1, plan.mid_cap * parts.cost_from(1) / plan.mid);
+    for (auto& m : parts.deal(1, plan.mid)) {
       if (m.empty()) continue;
       std::sort(m.begin(), m.end());
       for (int k : m) cta[k] = (int)mid.size();
