@@ -3281,6 +3281,34 @@ static int batch_split(gox_topo* t, int B, const double* p_spec, const double* q
   return GOX_OK;
 }
 
+// Work that follows what the caller's stream holds, and that its later work
+// follows, on the thread's own stream (on: else the caller's itself).
+struct StreamDetour {
+  cudaStream_t caller, st;
+  cudaEvent_t ev = nullptr;
+  StreamDetour(cudaStream_t c, bool on) : caller(c), st(c) {
+    if (!on) return;
+    GOX_CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    st = thread_stream();
+    if (cudaEventRecord(ev, caller) != cudaSuccess || cudaStreamWaitEvent(st, ev, 0) != cudaSuccess) {
+      cudaGetLastError();
+      cudaEventDestroy(ev);
+      ev = nullptr;
+      st = caller;
+    }
+  }
+  ~StreamDetour() {
+    if (!ev) return;
+    if (cudaEventRecord(ev, st) != cudaSuccess || cudaStreamWaitEvent(caller, ev, 0) != cudaSuccess) {
+      cudaGetLastError();
+      cudaStreamSynchronize(st);
+    }
+    cudaEventDestroy(ev);
+  }
+  StreamDetour(const StreamDetour&) = delete;
+  StreamDetour& operator=(const StreamDetour&) = delete;
+};
+
 extern "C" {
 
 const char* gox_version(void) { return "gridoxide_gb300 0.1.0 (sm_103a)"; }
@@ -3419,9 +3447,15 @@ int gox_batch_solve_device(gox_topo* t, int32_t B, const double* p_spec, const d
   if (c <= 0) return c;
   if (int r = require_device()) return r;
   return guard_impl([&]() -> int {
-    cudaStream_t st = (cudaStream_t)stream;
-    AllocStreamScope alloc_scope(st);
     if (max_iter == 0) return GOX_E_INVALID;
+    // The default stream cannot be captured and orders the parts of a split solve
+    // after each other: a large batch runs on the thread's own stream, between an
+    // event of the caller's stream and one that it waits for (4,096 scenarios of
+    // 2,000 buses 16.3 -> 10.9 ms).  Smaller ones use neither graphs nor parts.
+    const bool legacy = stream == nullptr || (cudaStream_t)stream == cudaStreamLegacy;
+    StreamDetour detour((cudaStream_t)stream, legacy && B > 32 * (kGraphMinGroups - 1));
+    cudaStream_t st = detour.st;
+    AllocStreamScope alloc_scope(st);
     return batch_split(t, B, p_spec, q_spec, vm0, va0, v_stride, o_slot, o_dre, o_dim, tol,
                        max_iter, precision, vm_out, va_out, iterations, status, max_mismatch,
                        history, st, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
