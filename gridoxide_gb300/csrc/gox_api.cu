@@ -792,6 +792,28 @@ struct Iter {
       GOX_CK(cudaFuncSetAttribute(k_dot_topback<T>, a, 20));
     });
   }
+  template <bool OUTAGE, bool ZIP>
+  static void solo_newton_with(const SoloDev& P, const SchedDev& S, const BatchDev& D, int max_iter, cudaStream_t st) {
+    static std::once_flag once[64];
+    int dev = 0;
+    GOX_CK(cudaGetDevice(&dev));
+    std::call_once(once[dev & 63], [] {
+      GOX_CK(cudaFuncSetAttribute(k_solo_newton<T, OUTAGE, ZIP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  kSoloRingBytes + kSoloMaxBytes));
+    });
+    k_solo_newton<T, OUTAGE, ZIP><<<D.nb, 32 * kSoloWarps, P.bytes[2], st>>>(P, S, D, max_iter);
+    GOX_CK(cudaGetLastError());
+  }
+  static void solo_newton(const SoloDev& P, const SchedDev& S, const BatchDev& D, int max_iter, bool outage,
+                          cudaStream_t st) {
+    if (S.zip) {
+      if (outage) solo_newton_with<true, true>(P, S, D, max_iter, st);
+      else solo_newton_with<false, true>(P, S, D, max_iter, st);
+    } else {
+      if (outage) solo_newton_with<true, false>(P, S, D, max_iter, st);
+      else solo_newton_with<false, false>(P, S, D, max_iter, st);
+    }
+  }
   static void solo(const SoloDev& P, const SchedDev& S, const BatchDev& D, cudaStream_t st) {
     static std::once_flag once[64];
     int dev = 0;
@@ -1176,6 +1198,7 @@ static void upload_plans(gox_topo* t) {
   t->uploaded = true;
 }
 
+static constexpr int kSoloNewtonMax = 64;   // iterations of a loop in one launch
 static constexpr int kGraphMinGroups = 64;  // batches of >= 2,048 scenarios
 
 // The sink (node without dependents) of a graph captured from one stream
@@ -1806,6 +1829,16 @@ static void run_iterations(gox_topo* t, BatchDev D, int max_iter, bool outage, c
   const SchedDev& S = t->dsched.d;
   const bool timing = t->timing.on;
   const bool pivoting = sizeof(T) == 8 && t->pivot_pass;
+  // few scenarios with a program of one CTA: the whole loop in one launch (not
+  // for budgets that would keep a kernel running for long)
+  if (!timing && !pivoting && max_iter <= kSoloNewtonMax) {
+    const auto* x = t->dsched.pick_solo(sizeof(T) == 4 ? 0 : 1, D.nb);
+    if (x && x->d.ctas[0] == 0) {
+      Iter<T>::solo_newton(x->d, S, D, max_iter, outage, st);
+      t->launches++;
+      return;
+    }
+  }
   if (!timing && !pivoting && run_loop_graph<T>(t, D, max_iter, outage, st)) {
     // launches: per iteration 3 + 1 (decision) and, while running, fill,
     // refactor and the separate solve; the final mismatch when the budget ran out

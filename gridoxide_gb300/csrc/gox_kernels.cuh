@@ -96,6 +96,16 @@ struct BatchDev {
   int32_t* itp;                    // [1] iteration of the graph-captured loop (kernels given it < 0)
 };
 
+// a b + c d and a b - c d as one rounding of the second product and one of the
+// whole (written out: left to itself the compiler may round the first product
+// in one kernel and the second in another)
+__device__ __forceinline__ float dot2(float a, float b, float c, float d) { return fmaf(a, b, __fmul_rn(c, d)); }
+__device__ __forceinline__ double dot2(double a, double b, double c, double d) { return fma(a, b, __dmul_rn(c, d)); }
+__device__ __forceinline__ float dif2(float a, float b, float c, float d) { return fmaf(a, b, -__fmul_rn(c, d)); }
+__device__ __forceinline__ double dif2(double a, double b, double c, double d) { return fma(a, b, -__dmul_rn(c, d)); }
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return fma(a, b, c); }
+
 __device__ __forceinline__ size_t gidx(int g, int n, int e, int lane) {
   return ((size_t)g * (size_t)n + (size_t)e) * 32u + (size_t)lane;
 }
@@ -145,15 +155,9 @@ __device__ __forceinline__ double from_T(T v) {
 // K5 + K1a.  grid (ceil(N/8), G), 8 warps: warp -> bus, lane -> scenario.
 // mode 0: iteration `it`; mode 1: the update after the last iteration.
 template <typename T>
-__device__ __forceinline__ void update_body(const SchedDev& S, const BatchDev& D, int it, int mode,
-                                            int BX, int BY) {
-  if (it < 0) it = *D.itp;
-  const int g = BY;
-  const int lane = threadIdx.x & 31;
-  const int i = BX * 8 + (threadIdx.x >> 5);
+__device__ __forceinline__ void update_one(const SchedDev& S, const BatchDev& D, int it, int mode, int g, int i,
+                                           int lane) {
   const int N = S.n_bus;
-  // a block is 8 warps (a wider CTA's other warps take no part)
-  if (i >= N || (threadIdx.x >> 5) >= 8) return;
   const int s = g * 32 + lane;
   const bool upd = D.status[s] == ST_RUNNING && (it > 0 || mode == 1) && D.sing[s] == 0;
   const size_t x = gidx(g, N, i, lane);
@@ -203,18 +207,18 @@ __device__ __forceinline__ void update_body(const SchedDev& S, const BatchDev& D
   const bool tiny = it > 0 && (sizeof(T) == 4 ? ad < 0.0009765625f : fabs(dth) < 0.0009765625);
   if (tiny) {
     const double d2 = dth * dth;
-    const double cd = 1.0 + d2 * (-1.0 / 2 + d2 * (1.0 / 24));
-    const double sd = dth * (1.0 + d2 * (-1.0 / 6 + d2 * (1.0 / 120)));
+    const double cd = fma(d2, fma(d2, 1.0 / 24, -1.0 / 2), 1.0);
+    const double sd = dth * fma(d2, fma(d2, 1.0 / 120, -1.0 / 6), 1.0);
     const double c0 = D.cth[x], s0 = D.sth[x];
-    cs = c0 * cd - s0 * sd;
-    sn = s0 * cd + c0 * sd;
+    cs = dif2(c0, cd, s0, sd);
+    sn = dot2(c0, sd, s0, cd);
   } else if (small) {
     const double d2 = dth * dth;
-    const double cd = 1.0 + d2 * (-1.0 / 2 + d2 * (1.0 / 24 + d2 * (-1.0 / 720 + d2 * (1.0 / 40320))));
-    const double sd = dth * (1.0 + d2 * (-1.0 / 6 + d2 * (1.0 / 120 + d2 * (-1.0 / 5040))));
+    const double cd = fma(d2, fma(d2, fma(d2, fma(d2, 1.0 / 40320, -1.0 / 720), 1.0 / 24), -1.0 / 2), 1.0);
+    const double sd = dth * fma(d2, fma(d2, fma(d2, -1.0 / 5040, 1.0 / 120), -1.0 / 6), 1.0);
     const double c0 = D.cth[x], s0 = D.sth[x];
-    cs = c0 * cd - s0 * sd;
-    sn = s0 * cd + c0 * sd;
+    cs = dif2(c0, cd, s0, sd);
+    sn = dot2(c0, sd, s0, cd);
   } else {
     sincos(va, &sn, &cs);
   }
@@ -228,6 +232,15 @@ __device__ __forceinline__ void update_body(const SchedDev& S, const BatchDev& D
   // 1/|V| for the Jacobian fill, in the fill's precision (an FP64 division
   // costs far more than an FP32 one on this GPU)
   ((T*)D.ivT)[x] = (T)1 / to_T<T>(vm);
+}
+template <typename T>
+__device__ __forceinline__ void update_body(const SchedDev& S, const BatchDev& D, int it, int mode,
+                                            int BX, int BY) {
+  if (it < 0) it = *D.itp;
+  const int i = BX * 8 + (threadIdx.x >> 5);
+  // a block is 8 warps (a wider CTA's other warps take no part)
+  if (i >= S.n_bus || (threadIdx.x >> 5) >= 8) return;
+  update_one<T>(S, D, it, mode, BY, i, threadIdx.x & 31);
 }
 template <typename T>
 __global__ void __launch_bounds__(256) k_update(SchedDev S, BatchDev D, int it, int mode) {
@@ -302,6 +315,96 @@ __device__ __forceinline__ unsigned long long abs_bits(double v) {
   return b > 0x7ff0000000000000ull ? 0ull : b;  // NaN: skipped
 }
 
+template <typename T, bool OUTAGE, bool ZIP>
+__device__ __forceinline__ void inject_one(const SchedDev& S, const BatchDev& D, int g, int i, int lane, int s,
+                                           bool active, int obf, int obt, const double* st0,
+                                           unsigned long long& mx) {
+  const int N = S.n_bus;
+  T* rhs = (T*)D.rhs;
+  const double* __restrict__ e = D.e;
+  const double* __restrict__ f = D.f;
+  double ir = 0.0, ii = 0.0;
+  if (st0 != nullptr) {
+    ir = st0[4 * (size_t)N + i];
+    ii = st0[5 * (size_t)N + i];
+  } else {
+    int p = __ldg(S.yp + i);
+    const int pe = __ldg(S.yp + i + 1);
+    while (pe - p > 8) {
+      y_row<8>(S, e, f, g, N, lane, p, ir, ii);
+      p += 8;
+    }
+    switch (pe - p) {
+      case 1: y_row<1>(S, e, f, g, N, lane, p, ir, ii); break;
+      case 2: y_row<2>(S, e, f, g, N, lane, p, ir, ii); break;
+      case 3: y_row<3>(S, e, f, g, N, lane, p, ir, ii); break;
+      case 4: y_row<4>(S, e, f, g, N, lane, p, ir, ii); break;
+      case 5: y_row<5>(S, e, f, g, N, lane, p, ir, ii); break;
+      case 6: y_row<6>(S, e, f, g, N, lane, p, ir, ii); break;
+      case 7: y_row<7>(S, e, f, g, N, lane, p, ir, ii); break;
+      case 8: y_row<8>(S, e, f, g, N, lane, p, ir, ii); break;
+      default: break;
+    }
+  }
+  const size_t x = gidx(g, N, i, lane);
+  const double ei = e[x], fi = f[x];
+  if (OUTAGE && (i == obf || i == obt)) {
+    const size_t xf = gidx(g, N, obf, lane), xt = gidx(g, N, obt, lane);
+    const double ef = e[xf], ff = f[xf], et = e[xt], ft = f[xt];
+    const int c0 = (i == obf) ? 0 : 2;
+    const double ar = D.o_dre[4 * s + c0], ai = D.o_dim[4 * s + c0];
+    const double br = D.o_dre[4 * s + c0 + 1], bi = D.o_dim[4 * s + c0 + 1];
+    ir += ar * ef - ai * ff + br * et - bi * ft;
+    ii += ar * ff + ai * ef + br * ft + bi * et;
+  }
+  const int rp = __ldg(S.bus_rowP + i), rq = __ldg(S.bus_rowQ + i);
+  if constexpr (sizeof(T) == 4) {
+    // F = S_spec - V conj(I) in FP64 as two FMAs per component; the FP32
+    // Jacobian's P and Q are S_spec - F in FP32 (only the buses with a P
+    // row have Jacobian entries that use them; a PV bus's Q comes from
+    // the products, it has no Q row)
+    if (rp >= 0) {
+      const double psp = ZIP ? eff_inj(S.zip, N, i, 0, D.psp[x], D.vm[x]) : D.psp[x];
+      const double FP = fma(-fi, ii, fma(-ei, ir, psp));
+      const float fp = f32_rn(FP);
+      if (active) {
+        mx = max(mx, abs_bits(FP));
+        rhs[gidx(g, S.n_u, rp, lane)] = fp;
+      }
+      ((float*)D.pT)[x] = f32_rn(psp) - fp;
+      if (rq >= 0) {
+        const double qsp = ZIP ? eff_inj(S.zip, N, i, 1, D.qsp[x], D.vm[x]) : D.qsp[x];
+        const double FQ = fma(ei, ii, fma(-fi, ir, qsp));
+        const float fq = f32_rn(FQ);
+        if (active) {
+          mx = max(mx, abs_bits(FQ));
+          rhs[gidx(g, S.n_u, rq, lane)] = fq;
+        }
+        ((float*)D.qT)[x] = f32_rn(qsp) - fq;
+      } else {
+        ((float*)D.qT)[x] = f32_rn(dif2(fi, ir, ei, ii));
+      }
+    }
+  } else {
+    const double pc = dot2(ei, ir, fi, ii);
+    const double qc = dif2(fi, ir, ei, ii);
+    if (active) {
+      if (rp >= 0) {
+        const double F = (ZIP ? eff_inj(S.zip, N, i, 0, D.psp[x], D.vm[x]) : D.psp[x]) - pc;
+        mx = max(mx, abs_bits(F));
+        rhs[gidx(g, S.n_u, rp, lane)] = (T)F;
+      }
+      if (rq >= 0) {
+        const double F = (ZIP ? eff_inj(S.zip, N, i, 1, D.qsp[x], D.vm[x]) : D.qsp[x]) - qc;
+        mx = max(mx, abs_bits(F));
+        rhs[gidx(g, S.n_u, rq, lane)] = (T)F;
+      }
+    }
+    ((T*)D.pT)[x] = (T)pc;
+    ((T*)D.qT)[x] = (T)qc;
+  }
+  }
+
 template <typename T, bool OUTAGE, int BPW, bool ZIP>
 __device__ __forceinline__ void inject_body(const SchedDev& S, const BatchDev& D, int it, int BX,
                                             int BY) {
@@ -312,9 +415,6 @@ __device__ __forceinline__ void inject_body(const SchedDev& S, const BatchDev& D
   const int N = S.n_bus;
   __shared__ unsigned long long red[8][32];
   const bool active = D.status[s] == ST_RUNNING && !(it > 0 && D.sing[s] != 0);
-  T* rhs = (T*)D.rhs;
-  const double* __restrict__ e = D.e;
-  const double* __restrict__ f = D.f;
   int obf = -1, obt = -1;
   if (OUTAGE) { obf = D.o_bf[s]; obt = D.o_bt[s]; }
   unsigned long long mx = 0ull;
@@ -323,86 +423,7 @@ __device__ __forceinline__ void inject_body(const SchedDev& S, const BatchDev& D
   const int i0 = in_block ? (BX * 8 + warp) * BPW : N;
   const double* st0 = it == 0 ? D.st0 : nullptr;  // the shared start's currents
   for (int i = i0; i < min(N, i0 + BPW); i++) {
-    double ir = 0.0, ii = 0.0;
-    if (st0 != nullptr) {
-      ir = st0[4 * (size_t)N + i];
-      ii = st0[5 * (size_t)N + i];
-    } else {
-      int p = __ldg(S.yp + i);
-      const int pe = __ldg(S.yp + i + 1);
-      while (pe - p > 8) {
-        y_row<8>(S, e, f, g, N, lane, p, ir, ii);
-        p += 8;
-      }
-      switch (pe - p) {
-        case 1: y_row<1>(S, e, f, g, N, lane, p, ir, ii); break;
-        case 2: y_row<2>(S, e, f, g, N, lane, p, ir, ii); break;
-        case 3: y_row<3>(S, e, f, g, N, lane, p, ir, ii); break;
-        case 4: y_row<4>(S, e, f, g, N, lane, p, ir, ii); break;
-        case 5: y_row<5>(S, e, f, g, N, lane, p, ir, ii); break;
-        case 6: y_row<6>(S, e, f, g, N, lane, p, ir, ii); break;
-        case 7: y_row<7>(S, e, f, g, N, lane, p, ir, ii); break;
-        case 8: y_row<8>(S, e, f, g, N, lane, p, ir, ii); break;
-        default: break;
-      }
-    }
-    const size_t x = gidx(g, N, i, lane);
-    const double ei = e[x], fi = f[x];
-    if (OUTAGE && (i == obf || i == obt)) {
-      const size_t xf = gidx(g, N, obf, lane), xt = gidx(g, N, obt, lane);
-      const double ef = e[xf], ff = f[xf], et = e[xt], ft = f[xt];
-      const int c0 = (i == obf) ? 0 : 2;
-      const double ar = D.o_dre[4 * s + c0], ai = D.o_dim[4 * s + c0];
-      const double br = D.o_dre[4 * s + c0 + 1], bi = D.o_dim[4 * s + c0 + 1];
-      ir += ar * ef - ai * ff + br * et - bi * ft;
-      ii += ar * ff + ai * ef + br * ft + bi * et;
-    }
-    const int rp = __ldg(S.bus_rowP + i), rq = __ldg(S.bus_rowQ + i);
-    if constexpr (sizeof(T) == 4) {
-      // F = S_spec - V conj(I) in FP64 as two FMAs per component; the FP32
-      // Jacobian's P and Q are S_spec - F in FP32 (only the buses with a P
-      // row have Jacobian entries that use them; a PV bus's Q comes from
-      // the products, it has no Q row)
-      if (rp >= 0) {
-        const double psp = ZIP ? eff_inj(S.zip, N, i, 0, D.psp[x], D.vm[x]) : D.psp[x];
-        const double FP = fma(-fi, ii, fma(-ei, ir, psp));
-        const float fp = f32_rn(FP);
-        if (active) {
-          mx = max(mx, abs_bits(FP));
-          rhs[gidx(g, S.n_u, rp, lane)] = fp;
-        }
-        ((float*)D.pT)[x] = f32_rn(psp) - fp;
-        if (rq >= 0) {
-          const double qsp = ZIP ? eff_inj(S.zip, N, i, 1, D.qsp[x], D.vm[x]) : D.qsp[x];
-          const double FQ = fma(ei, ii, fma(-fi, ir, qsp));
-          const float fq = f32_rn(FQ);
-          if (active) {
-            mx = max(mx, abs_bits(FQ));
-            rhs[gidx(g, S.n_u, rq, lane)] = fq;
-          }
-          ((float*)D.qT)[x] = f32_rn(qsp) - fq;
-        } else {
-          ((float*)D.qT)[x] = f32_rn(fi * ir - ei * ii);
-        }
-      }
-    } else {
-      const double pc = ei * ir + fi * ii;
-      const double qc = fi * ir - ei * ii;
-      if (active) {
-        if (rp >= 0) {
-          const double F = (ZIP ? eff_inj(S.zip, N, i, 0, D.psp[x], D.vm[x]) : D.psp[x]) - pc;
-          mx = max(mx, abs_bits(F));
-          rhs[gidx(g, S.n_u, rp, lane)] = (T)F;
-        }
-        if (rq >= 0) {
-          const double F = (ZIP ? eff_inj(S.zip, N, i, 1, D.qsp[x], D.vm[x]) : D.qsp[x]) - qc;
-          mx = max(mx, abs_bits(F));
-          rhs[gidx(g, S.n_u, rq, lane)] = (T)F;
-        }
-      }
-      ((T*)D.pT)[x] = (T)pc;
-      ((T*)D.qT)[x] = (T)qc;
-    }
+    inject_one<T, OUTAGE, ZIP>(S, D, g, i, lane, s, active, obf, obt, st0, mx);
   }
   if (in_block) red[warp][lane] = mx;
   __syncthreads();
@@ -418,10 +439,8 @@ __global__ void __launch_bounds__(256) k_inject(SchedDev S, BatchDev D, int it) 
   inject_body<T, OUTAGE, BPW, ZIP>(S, D, it, blockIdx.x, blockIdx.y);
 }
 
-__device__ __forceinline__ void decide_body(const BatchDev& D, int it, int mode, int BX) {
-  if (it < 0) it = *D.itp;
-  const int g = BX, lane = threadIdx.x;
-  const int s = g * 32 + lane;
+// Scenario s after its mismatch (acc: the bits of max|F|): whether it goes on
+__device__ __forceinline__ bool decide_one(const BatchDev& D, int it, int mode, int s, unsigned long long acc) {
   bool running = D.status[s] == ST_RUNNING;
   if (running) {
     const int sg = D.sing[s];
@@ -432,7 +451,7 @@ __device__ __forceinline__ void decide_body(const BatchDev& D, int it, int mode,
       D.status[s] = ST_MAXITER;
       running = false;
     } else {
-      const double m = __longlong_as_double((long long)D.maxacc[s]);
+      const double m = __longlong_as_double((long long)acc);
       D.maxmis[s] = m;
       if (D.hist) D.hist[(size_t)s * D.max_iter + it] = m;
       D.iters[s] = it + 1;
@@ -443,6 +462,13 @@ __device__ __forceinline__ void decide_body(const BatchDev& D, int it, int mode,
       }
     }
   }
+  return running;
+}
+__device__ __forceinline__ void decide_body(const BatchDev& D, int it, int mode, int BX) {
+  if (it < 0) it = *D.itp;
+  const int g = BX, lane = threadIdx.x;
+  const int s = g * 32 + lane;
+  const bool running = decide_one(D, it, mode, s, D.maxacc[s]);
   D.maxacc[s] = 0ull;
   const unsigned any = __ballot_sync(0xffffffffu, running);
   if (lane == 0) {
@@ -486,6 +512,30 @@ __device__ __forceinline__ void fill_store(T* LU, T* OFF, int n_slots, int x, in
   else OFF[(size_t)(x - n_slots) * 32u + lane] = v;
 }
 
+// The four Jacobian entries of a task from its five values (a diagonal's or an
+// off-diagonal's)
+template <typename T>
+__device__ __forceinline__ void fill_entries(bool dg, const T* v, T G, T B, T& h, T& nn, T& m, T& l) {
+  if (dg) {
+    const T ei = v[0], fi = v[1], iv = v[2], P = v[3], Q = v[4];
+    const T vi2 = dot2(ei, ei, fi, fi);
+    const T vi = vi2 * iv;       // |V_i|^2 / |V_i|
+    h = fma_rn(-vi2, B, -Q);     // H_ii = -Q - |V_i|^2 B
+    nn = dot2(P, iv, vi, G);     // N_ii
+    m = fma_rn(-vi2, G, P);      // M_ii = P - |V_i|^2 G
+    l = dif2(Q, iv, vi, B);      // L_ii
+  } else {
+    const T ei = v[0], fi = v[1], ek = v[2], fk = v[3], ivk = v[4];
+    const T c = dot2(ei, ek, fi, fk);   // V_i V_k cos
+    const T sn = dif2(fi, ek, ei, fk);  // V_i V_k sin
+    const T a = dif2(G, sn, B, c);
+    const T b = dot2(G, c, B, sn);
+    h = a;          // H_ik
+    nn = b * ivk;   // N_ik
+    m = -b;         // M_ik
+    l = a * ivk;    // L_ik
+  }
+}
 template <typename T, bool OUTAGE>
 __device__ __forceinline__ void fill_body(const SchedDev& S, const BatchDev& D, int tw, int per_warp,
                                           int BX, int BY) {
@@ -577,25 +627,7 @@ __device__ __forceinline__ void fill_body(const SchedDev& S, const BatchDev& D, 
     for (int u = 0; u < U; u++) {
       if (ta + u >= t1) break;
       T h, nn, m, l;
-      if (bus[u].w != 0) {
-        const T ei = v[u][0], fi = v[u][1], iv = v[u][2], P = v[u][3], Q = v[u][4];
-        const T vi2 = ei * ei + fi * fi;
-        const T vi = vi2 * iv;  // |V_i|^2 / |V_i|
-        h = -Q - vi2 * B[u];       // H_ii
-        nn = P * iv + vi * G[u];   // N_ii
-        m = P - vi2 * G[u];        // M_ii
-        l = Q * iv - vi * B[u];    // L_ii
-      } else {
-        const T ei = v[u][0], fi = v[u][1], ek = v[u][2], fk = v[u][3], ivk = v[u][4];
-        const T c = ei * ek + fi * fk;   // V_i V_k cos
-        const T sn = fi * ek - ei * fk;  // V_i V_k sin
-        const T a = G[u] * sn - B[u] * c;
-        const T b = G[u] * c + B[u] * sn;
-        h = a;          // H_ik
-        nn = b * ivk;   // N_ik
-        m = -b;         // M_ik
-        l = a * ivk;    // L_ik
-      }
+      fill_entries<T>(bus[u].w != 0, v[u], G[u], B[u], h, nn, m, l);
       fill_store(LU, OFF, S.n_slots, dst[u].x, lane, h);
       fill_store(LU, OFF, S.n_slots, dst[u].y, lane, nn);
       fill_store(LU, OFF, S.n_slots, dst[u].z, lane, m);

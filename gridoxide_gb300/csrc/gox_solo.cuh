@@ -32,15 +32,14 @@ struct SoloDev {
   int stride;             // from a scenario's value to its next (32; 1: a batch of one by itself)
 };
 
-// One launch of a program: a CTA per part and scenario.
+// Scenario s's part in CTA `part` of a launch.
 template <typename T>
-__global__ void __launch_bounds__(32 * kSoloWarps)
-    k_solo(SoloDev P, SchedDev S, BatchDev D, int which) {
+__device__ __forceinline__ void solo_body(const SoloDev& P, const SchedDev& S, const BatchDev& D, int which, int part,
+                                          int s) {
   extern __shared__ __align__(16) unsigned char solo_smem[];
-  const int g = blockIdx.y >> 5, l = blockIdx.y & 31, s = blockIdx.y;
-  if (!D.gact[g]) return;
+  const int g = s >> 5, l = s & 31;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const SoloCta* C = P.cta[which] + blockIdx.x;
+  const SoloCta* C = P.cta[which] + part;
   uint4* ring = reinterpret_cast<uint4*>(solo_smem) + warp * kSoloDepth * kSoloQuads + lane;
   char* c = reinterpret_cast<char*>(solo_smem) + kSoloRingBytes;
   const uint4* gs = P.words + (size_t)C->stream[warp] * kSoloQuads + lane;
@@ -152,6 +151,95 @@ __global__ void __launch_bounds__(32 * kSoloWarps)
   }
   if (bad) D.sing[s] = 1;
   if (tiny) D.piv_flag[s] = 1;
+}
+
+// One launch of a program: a CTA per part and scenario.
+template <typename T>
+__global__ void __launch_bounds__(32 * kSoloWarps) k_solo(SoloDev P, SchedDev S, BatchDev D, int which) {
+  if (D.gact[blockIdx.y >> 5]) solo_body<T>(P, S, D, which, blockIdx.x, blockIdx.y);
+}
+
+// Task t's Jacobian entries of one scenario
+template <typename T, bool OUTAGE>
+__device__ __forceinline__ void solo_fill(const SchedDev& S, const BatchDev& D, int g, int lane, int s, int t) {
+  const int4 dst = __ldg(S.ft_dst + t), bus = __ldg(S.ft_bus + t);
+  T G, B;
+  if constexpr (sizeof(T) == 4) {
+    const float2 y = __ldg(S.ft_yf + t);
+    G = y.x;
+    B = y.y;
+  } else {
+    const double2 y = __ldg(S.ft_y + t);
+    G = y.x;
+    B = y.y;
+  }
+  const size_t gb = (size_t)g * S.n_bus * 32u + lane, xi = gb + (size_t)bus.x * 32u, xk = gb + (size_t)bus.y * 32u;
+  const bool dg = bus.w != 0;
+  const T *eT = (const T*)D.eT, *fT = (const T*)D.fT, *ivT = (const T*)D.ivT;
+  const T v[5] = {eT[xi], fT[xi], dg ? ivT[xi] : eT[xk], dg ? ((const T*)D.pT)[xi] : fT[xk],
+                  dg ? ((const T*)D.qT)[xi] : ivT[xk]};
+  if (OUTAGE && D.o_bf[s] >= 0) {
+    for (int c = 0; c < 4; c++)
+      if (D.o_slot[4 * s + c] == bus.z) {  // (the first of equal slots, as the batch kernel)
+        const double2 y = __ldg(S.ft_y + t);
+        G = (T)(y.x + D.o_dre[4 * s + c]);
+        B = (T)(y.y + D.o_dim[4 * s + c]);
+        break;
+      }
+  }
+  T h, nn, m, l;
+  fill_entries<T>(dg, v, G, B, h, nn, m, l);
+  T* LU = (T*)D.lu + (size_t)g * S.n_slots * 32u;
+  T* OFF = (T*)D.off + (size_t)g * S.n_off * 32u;
+  fill_store(LU, OFF, S.n_slots, dst.x, lane, h);
+  fill_store(LU, OFF, S.n_slots, dst.y, lane, nn);
+  fill_store(LU, OFF, S.n_slots, dst.z, lane, m);
+  fill_store(LU, OFF, S.n_slots, dst.w, lane, l);
+}
+
+// A scenario's whole Newton loop on its CTA (programs of one CTA): the
+// batch kernels' steps with a thread per bus, per Y entry and per slot, and
+// CTA barriers between them.  Seven launches, a copy and a wait on the host
+// per iteration took some 50 us of a small grid's iteration, as much as its
+// refactor.  Measured, whole solves: 118 buses FP64, one scenario .741 -> .565
+// ms (mixed .513 -> .347), 75 load cases of 300 buses .631 -> .542.
+template <typename T, bool OUTAGE, bool ZIP>
+__global__ void __launch_bounds__(32 * kSoloWarps, 4) k_solo_newton(SoloDev P, SchedDev S, BatchDev D, int max_iter) {
+  constexpr int NTH = 32 * kSoloWarps;
+  __shared__ unsigned long long red[kSoloWarps];
+  __shared__ int go;
+  const int s = blockIdx.x, g = s >> 5, l = s & 31, tid = threadIdx.x;
+  int obf = -1, obt = -1;
+  if (OUTAGE) {
+    obf = D.o_bf[s];
+    obt = D.o_bt[s];
+  }
+  for (int it = 0; it < max_iter; it++) {
+    for (int i = tid; i < S.n_bus; i += NTH) update_one<T>(S, D, it, 0, g, i, l);
+    const bool active = D.status[s] == ST_RUNNING && !(it > 0 && D.sing[s] != 0);
+    __syncthreads();
+    unsigned long long mx = 0ull;
+    for (int i = tid; i < S.n_bus; i += NTH)
+      inject_one<T, OUTAGE, ZIP>(S, D, g, i, l, s, active, obf, obt, it == 0 ? D.st0 : nullptr, mx);
+    for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if ((tid & 31) == 0) red[tid >> 5] = mx;
+    __syncthreads();
+    if (tid == 0) {
+      for (int w = 1; w < kSoloWarps; w++) mx = max(mx, red[w]);
+      go = decide_one(D, it, 0, s, active ? mx : 0ull);
+    }
+    __syncthreads();
+    if (!go) return;
+    for (int t = tid; t < S.n_ftask; t += NTH) solo_fill<T, OUTAGE>(S, D, g, l, s, t);
+    T* LU = (T*)D.lu + (size_t)g * S.n_slots * 32u + l;
+    for (int z = tid; z < S.n_fzero; z += NTH) LU[(size_t)__ldg(S.fz_slot + z) * 32u] = (T)0;
+    __syncthreads();
+    solo_body<T>(P, S, D, 2, 0, s);
+    __syncthreads();
+  }
+  for (int i = tid; i < S.n_bus; i += NTH) update_one<T>(S, D, max_iter, 1, g, i, l);
+  __syncthreads();
+  if (tid == 0) decide_one(D, max_iter, 1, s, 0ull);
 }
 
 }  // namespace gox

@@ -51,7 +51,7 @@ constexpr int kSoloQuads = 3 * 32;         // quads of a unit
 constexpr int kSoloWarps = 8;
 constexpr int kSoloDepth = 3;  // units of a warp in shared memory: the one run and the next two
 constexpr int kSoloRingBytes = kSoloWarps * kSoloDepth * kSoloQuads * 16;
-constexpr int kSoloMaxBytes = 227 * 1024 - kSoloRingBytes;  // a CTA's values
+constexpr int kSoloMaxBytes = 226 * 1024 - kSoloRingBytes;  // a CTA's values (1 KB is left for the kernel's own)
 
 // A CTA: its warps' streams (first unit of each), its values and what it stores
 // (positions in lists: SOLO_LU, SOLO_RHS or SOLO_SOL and the slot or row, a
