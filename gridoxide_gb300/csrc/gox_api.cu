@@ -346,9 +346,10 @@ struct DevSchedule {
   // solo programs beside the dot programs: the one for the fewest scenarios
   // first; max: the most scenarios it runs
   struct SoloOne {
-    int max = 0;
+    int max = 0, max_deep = 0;
     DevMem words, lists, ctas;
     SoloDev d{};
+    bool deep(int nb) const { return nb <= max_deep; }
   } solo[2][2];
   const SoloOne* pick_solo(int i, int nb) const {
     if (dot[i].on && nb > 0)
@@ -371,11 +372,12 @@ struct DevSchedule {
     for (int i = 0; i < 4; i++) {
       x.d.cta[i] = at;
       x.d.ctas[i] = (int)p->launch[i].size();
-      x.d.bytes[i] = kSoloRingBytes + p->max_values[i] * p->plan.elem;
+      x.d.bytes[i] = p->max_values[i] * p->plan.elem;
       at += p->launch[i].size();
     }
     x.d.stride = stride;
-    x.max = solo_scenarios(*p);
+    x.max = solo_scenarios(*p, kSoloDepth);
+    x.max_deep = solo_scenarios(*p, kSoloDeep);
   }
   // the plan's substitutions are part of its refactor
   bool has_bwd(int i) const { return dot[i].on ? dot[i].with_subst : st_bwd[i]; }
@@ -743,7 +745,7 @@ struct Iter {
   static void refactor(const DevSchedule& ds, const BatchDev& D, cudaStream_t st) {
     const int i = sizeof(T) == 4 ? 0 : 1;
     if (const auto* x = ds.pick_solo(i, D.nb)) {
-      solo(x->d, ds.d, D, st);
+      solo(*x, ds.d, D, st);
       return;
     }
     if (ds.dot[i].on) {
@@ -792,37 +794,35 @@ struct Iter {
       GOX_CK(cudaFuncSetAttribute(k_dot_topback<T>, a, 20));
     });
   }
-  template <bool OUTAGE, bool ZIP>
-  static void solo_newton_with(const SoloDev& P, const SchedDev& S, const BatchDev& D, int max_iter, cudaStream_t st) {
+  template <int DEPTH>
+  static void solo_attr() {
     static std::once_flag once[64];
     int dev = 0;
     GOX_CK(cudaGetDevice(&dev));
     std::call_once(once[dev & 63], [] {
-      GOX_CK(cudaFuncSetAttribute(k_solo_newton<T, OUTAGE, ZIP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  kSoloRingBytes + kSoloMaxBytes));
+      const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+      GOX_CK(cudaFuncSetAttribute(k_solo<T, DEPTH>, a, kSoloSmem));
+      GOX_CK(cudaFuncSetAttribute(k_solo_newton<T, false>, a, kSoloSmem));
+      GOX_CK(cudaFuncSetAttribute(k_solo_newton<T, true>, a, kSoloSmem));
     });
-    k_solo_newton<T, OUTAGE, ZIP><<<D.nb, 32 * kSoloWarps, P.bytes[2], st>>>(P, S, D, max_iter);
+  }
+  static void solo_newton(const SoloDev& P, const SchedDev& S, const BatchDev& D, int max_iter, cudaStream_t st) {
+    solo_attr<kSoloDepth>();
+    const int bytes = solo_ring_bytes(kSoloDepth) + P.bytes[2];
+    if (S.zip || D.o_bf) k_solo_newton<T, true><<<D.nb, 32 * kSoloWarps, bytes, st>>>(P, S, D, max_iter);
+    else k_solo_newton<T, false><<<D.nb, 32 * kSoloWarps, bytes, st>>>(P, S, D, max_iter);
     GOX_CK(cudaGetLastError());
   }
-  static void solo_newton(const SoloDev& P, const SchedDev& S, const BatchDev& D, int max_iter, bool outage,
-                          cudaStream_t st) {
-    if (S.zip) {
-      if (outage) solo_newton_with<true, true>(P, S, D, max_iter, st);
-      else solo_newton_with<false, true>(P, S, D, max_iter, st);
-    } else {
-      if (outage) solo_newton_with<true, false>(P, S, D, max_iter, st);
-      else solo_newton_with<false, false>(P, S, D, max_iter, st);
-    }
-  }
-  static void solo(const SoloDev& P, const SchedDev& S, const BatchDev& D, cudaStream_t st) {
-    static std::once_flag once[64];
-    int dev = 0;
-    GOX_CK(cudaGetDevice(&dev));
-    std::call_once(once[dev & 63], [] {
-      GOX_CK(cudaFuncSetAttribute(k_solo<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSoloRingBytes + kSoloMaxBytes));
-    });
+  template <int DEPTH>
+  static void solo_at(const SoloDev& P, const SchedDev& S, const BatchDev& D, cudaStream_t st) {
+    solo_attr<DEPTH>();
     for (int i = 0; i < 4; i++)
-      if (P.ctas[i] > 0) k_solo<T><<<dim3(P.ctas[i], D.nb), 32 * kSoloWarps, P.bytes[i], st>>>(P, S, D, i);
+      if (P.ctas[i] > 0)
+        k_solo<T, DEPTH><<<dim3(P.ctas[i], D.nb), 32 * kSoloWarps, solo_ring_bytes(DEPTH) + P.bytes[i], st>>>(P, S, D, i);
+  }
+  static void solo(const DevSchedule::SoloOne& x, const SchedDev& S, const BatchDev& D, cudaStream_t st) {
+    if (x.deep(D.nb)) solo_at<kSoloDeep>(x.d, S, D, st);
+    else solo_at<kSoloDepth>(x.d, S, D, st);
   }
   template <int WHICH>
   static void dot_bins(const DotDev& P, const SchedDev& S, const BatchDev& D, int n, int groups, cudaStream_t st) {
@@ -1834,7 +1834,7 @@ static void run_iterations(gox_topo* t, BatchDev D, int max_iter, bool outage, c
   if (!timing && !pivoting && max_iter <= kSoloNewtonMax) {
     const auto* x = t->dsched.pick_solo(sizeof(T) == 4 ? 0 : 1, D.nb);
     if (x && x->d.ctas[0] == 0) {
-      Iter<T>::solo_newton(x->d, S, D, max_iter, outage, st);
+      Iter<T>::solo_newton(x->d, S, D, max_iter, st);
       t->launches++;
       return;
     }

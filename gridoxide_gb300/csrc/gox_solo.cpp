@@ -49,12 +49,14 @@ bool build_solo_default(const Schedule& sc, int elem, bool wide, SoloProgram& ou
   return false;
 }
 
-int solo_scenarios(const SoloProgram& p) {
+int solo_scenarios(const SoloProgram& p, int depth) {
   int most = 1 << 20;
+  for (int v : p.max_values)
+    if (solo_ring_bytes(depth) + v * p.plan.elem > kSoloSmem) return 0;
   for (int i : {0, 2, 3}) {  // (the second launch's CTAs are many and short)
     const int ctas = (int)p.launch[i].size();
     if (ctas == 0) continue;
-    const int bytes = kSoloRingBytes + p.max_values[i] * p.plan.elem + 1024;
+    const int bytes = solo_ring_bytes(depth) + p.max_values[i] * p.plan.elem + 1024;
     most = std::min(most, 152 * std::min(8, (228 * 1024) / bytes) / ctas);
   }
   return most;

@@ -28,20 +28,21 @@ struct SoloDev {
   const uint4* words;
   const uint32_t* lists;
   const SoloCta* cta[4];
-  int ctas[4], bytes[4];  // per launch: CTAs, shared memory of one
+  int ctas[4], bytes[4];  // per launch: CTAs, bytes of a CTA's values
   int stride;             // from a scenario's value to its next (32; 1: a batch of one by itself)
 };
 
-// Scenario s's part in CTA `part` of a launch.
-template <typename T>
+// Scenario s's part in CTA `part` of a launch; DEPTH: units of a warp in shared
+// memory.
+template <typename T, int DEPTH>
 __device__ __forceinline__ void solo_body(const SoloDev& P, const SchedDev& S, const BatchDev& D, int which, int part,
                                           int s) {
   extern __shared__ __align__(16) unsigned char solo_smem[];
   const int g = s >> 5, l = s & 31;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const SoloCta* C = P.cta[which] + part;
-  uint4* ring = reinterpret_cast<uint4*>(solo_smem) + warp * kSoloDepth * kSoloQuads + lane;
-  char* c = reinterpret_cast<char*>(solo_smem) + kSoloRingBytes;
+  uint4* ring = reinterpret_cast<uint4*>(solo_smem) + warp * DEPTH * kSoloQuads + lane;
+  char* c = reinterpret_cast<char*>(solo_smem) + kSoloWarps * DEPTH * kSoloQuads * 16;
   const uint4* gs = P.words + (size_t)C->stream[warp] * kSoloQuads + lane;
   auto fetch = [&](int slot) {
 #pragma unroll
@@ -53,7 +54,7 @@ __device__ __forceinline__ void solo_body(const SoloDev& P, const SchedDev& S, c
     gs += kSoloQuads;
   };
 #pragma unroll
-  for (int i = 0; i < kSoloDepth; i++) fetch(i);
+  for (int i = 0; i < DEPTH; i++) fetch(i);
   const size_t stride = (size_t)P.stride;
   T* lu = (T*)D.lu + (size_t)g * S.n_slots * 32 + l;
   T* sol = (T*)D.sol + (size_t)g * S.n_u * 32 + l;
@@ -76,7 +77,7 @@ __device__ __forceinline__ void solo_body(const SoloDev& P, const SchedDev& S, c
   uint4 q0, q1, q2;
   // a unit's words: a lane reads only what it copied itself
   auto words = [&]() {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(kSoloDepth - 1) : "memory");
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(DEPTH - 1) : "memory");
     const uint4* u = ring + slot * kSoloQuads;
     q0 = u[0];
     q1 = u[32];
@@ -85,7 +86,7 @@ __device__ __forceinline__ void solo_body(const SoloDev& P, const SchedDev& S, c
   // on to the next unit's, in the shadow of this one's loads
   auto next = [&]() {
     fetch(slot);
-    slot = slot == kSoloDepth - 1 ? 0 : slot + 1;
+    slot = slot == DEPTH - 1 ? 0 : slot + 1;
     words();
   };
   // the products of the lane that the unit's longest sum has (in FP64 each one
@@ -154,14 +155,14 @@ __device__ __forceinline__ void solo_body(const SoloDev& P, const SchedDev& S, c
 }
 
 // One launch of a program: a CTA per part and scenario.
-template <typename T>
+template <typename T, int DEPTH>
 __global__ void __launch_bounds__(32 * kSoloWarps) k_solo(SoloDev P, SchedDev S, BatchDev D, int which) {
-  if (D.gact[blockIdx.y >> 5]) solo_body<T>(P, S, D, which, blockIdx.x, blockIdx.y);
+  if (D.gact[blockIdx.y >> 5]) solo_body<T, DEPTH>(P, S, D, which, blockIdx.x, blockIdx.y);
 }
 
-// Task t's Jacobian entries of one scenario
-template <typename T, bool OUTAGE>
-__device__ __forceinline__ void solo_fill(const SchedDev& S, const BatchDev& D, int g, int lane, int s, int t) {
+// Task t's Jacobian entries of one scenario (out: it has a branch out)
+template <typename T>
+__device__ __forceinline__ void solo_fill(const SchedDev& S, const BatchDev& D, int g, int lane, int s, bool out, int t) {
   const int4 dst = __ldg(S.ft_dst + t), bus = __ldg(S.ft_bus + t);
   T G, B;
   if constexpr (sizeof(T) == 4) {
@@ -178,7 +179,7 @@ __device__ __forceinline__ void solo_fill(const SchedDev& S, const BatchDev& D, 
   const T *eT = (const T*)D.eT, *fT = (const T*)D.fT, *ivT = (const T*)D.ivT;
   const T v[5] = {eT[xi], fT[xi], dg ? ivT[xi] : eT[xk], dg ? ((const T*)D.pT)[xi] : fT[xk],
                   dg ? ((const T*)D.qT)[xi] : ivT[xk]};
-  if (OUTAGE && D.o_bf[s] >= 0) {
+  if (out) {
     for (int c = 0; c < 4; c++)
       if (D.o_slot[4 * s + c] == bus.z) {  // (the first of equal slots, as the batch kernel)
         const double2 y = __ldg(S.ft_y + t);
@@ -203,14 +204,16 @@ __device__ __forceinline__ void solo_fill(const SchedDev& S, const BatchDev& D, 
 // per iteration took some 50 us of a small grid's iteration, as much as its
 // refactor.  Measured, whole solves: 118 buses FP64, one scenario .741 -> .565
 // ms (mixed .513 -> .347), 75 load cases of 300 buses .631 -> .542.
-template <typename T, bool OUTAGE, bool ZIP>
+// (kSoloDepth units: with kSoloDeep the 75 cases took .567 ms.)  EXTRA: the batch
+// has outages or voltage-dependent loads.
+template <typename T, bool EXTRA>
 __global__ void __launch_bounds__(32 * kSoloWarps, 4) k_solo_newton(SoloDev P, SchedDev S, BatchDev D, int max_iter) {
   constexpr int NTH = 32 * kSoloWarps;
   __shared__ unsigned long long red[kSoloWarps];
   __shared__ int go;
   const int s = blockIdx.x, g = s >> 5, l = s & 31, tid = threadIdx.x;
   int obf = -1, obt = -1;
-  if (OUTAGE) {
+  if (EXTRA && D.o_bf) {
     obf = D.o_bf[s];
     obt = D.o_bt[s];
   }
@@ -220,7 +223,7 @@ __global__ void __launch_bounds__(32 * kSoloWarps, 4) k_solo_newton(SoloDev P, S
     __syncthreads();
     unsigned long long mx = 0ull;
     for (int i = tid; i < S.n_bus; i += NTH)
-      inject_one<T, OUTAGE, ZIP>(S, D, g, i, l, s, active, obf, obt, it == 0 ? D.st0 : nullptr, mx);
+      inject_one<T, EXTRA, EXTRA>(S, D, g, i, l, s, active, obf, obt, it == 0 ? D.st0 : nullptr, mx);
     for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     if ((tid & 31) == 0) red[tid >> 5] = mx;
     __syncthreads();
@@ -230,11 +233,11 @@ __global__ void __launch_bounds__(32 * kSoloWarps, 4) k_solo_newton(SoloDev P, S
     }
     __syncthreads();
     if (!go) return;
-    for (int t = tid; t < S.n_ftask; t += NTH) solo_fill<T, OUTAGE>(S, D, g, l, s, t);
+    for (int t = tid; t < S.n_ftask; t += NTH) solo_fill<T>(S, D, g, l, s, EXTRA && obf >= 0, t);
     T* LU = (T*)D.lu + (size_t)g * S.n_slots * 32u + l;
     for (int z = tid; z < S.n_fzero; z += NTH) LU[(size_t)__ldg(S.fz_slot + z) * 32u] = (T)0;
     __syncthreads();
-    solo_body<T>(P, S, D, 2, 0, s);
+    solo_body<T, kSoloDepth>(P, S, D, 2, 0, s);
     __syncthreads();
   }
   for (int i = tid; i < S.n_bus; i += NTH) update_one<T>(S, D, max_iter, 1, g, i, l);

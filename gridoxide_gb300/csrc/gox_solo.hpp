@@ -49,9 +49,16 @@ enum : uint32_t {
 constexpr int kSoloTerms = 4;              // products of a unit, per lane
 constexpr int kSoloQuads = 3 * 32;         // quads of a unit
 constexpr int kSoloWarps = 8;
-constexpr int kSoloDepth = 3;  // units of a warp in shared memory: the one run and the next two
-constexpr int kSoloRingBytes = kSoloWarps * kSoloDepth * kSoloQuads * 16;
-constexpr int kSoloMaxBytes = 226 * 1024 - kSoloRingBytes;  // a CTA's values (1 KB is left for the kernel's own)
+// Units of a warp in shared memory, the one run and the next ones, while every
+// scenario's CTA finds a place with kSoloDeep, else kSoloDepth (a unit's words come from
+// the L2 and are wanted 300 to 500 cycles later; ms per refactor with 2 / 3 / 4 / 5
+// / 6 units: 2,000 buses FP32, 16 CTAs .53 / .39 / .324 / .310 / .316, 20,000 buses
+// .97 / .735 / .645 / .594 / .592; 600 scenarios of 118 buses FP64, which fit the
+// chip with 3 only, .119 with 3 and .197 with 5).
+constexpr int kSoloDepth = 3, kSoloDeep = 5;
+constexpr int solo_ring_bytes(int depth) { return kSoloWarps * depth * kSoloQuads * 16; }
+constexpr int kSoloSmem = 226 * 1024;  // of a CTA (1 KB is left for the kernel's own)
+constexpr int kSoloMaxBytes = kSoloSmem - solo_ring_bytes(kSoloDepth);  // a CTA's values
 
 // A CTA: its warps' streams (first unit of each), its values and what it stores
 // (positions in lists: SOLO_LU, SOLO_RHS or SOLO_SOL and the slot or row, a
@@ -86,8 +93,9 @@ bool build_solo(const Schedule& sc, const SoloPlan& plan, SoloProgram& out);
 // The program for a batch of one (wide) or for as many scenarios as possible:
 // the parts' CTAs that measured best, or as few as fit.
 bool build_solo_default(const Schedule& sc, int elem, bool wide, SoloProgram& out);
-// Scenarios whose CTAs find a place on the chip at once.
-int solo_scenarios(const SoloProgram& p);
+// Scenarios whose CTAs find a place on the chip at once, with `depth` units of a
+// warp in shared memory (0: its values leave no room for them).
+int solo_scenarios(const SoloProgram& p, int depth);
 
 // Host interpreter for one scenario in FP64, with the checks of run_dot_host:
 // indices in range, values final when read and not written in the tick (or, by
