@@ -695,12 +695,15 @@ static std::shared_ptr<const SoloProgram> make_solo(const Schedule& sc, int elem
 }
 // The solo programs of a schedule: one for the fewest scenarios and, where that
 // one has several CTAs, one for more.
+// A topology and its clones (a server's lanes) build them once between them.
 struct SoloPair {
+  std::mutex mu;
   bool tried = false;
   std::shared_ptr<const SoloProgram> p[2];
 };
 static void make_solos(const Schedule& sc, int elem, SoloPair& x) {
   x.tried = true;
+  if (sc.n_slots > 700000) return;  // (its rest does not fit: not worth the attempts)
   x.p[0] = make_solo(sc, elem, true);
   if (x.p[0] && x.p[0]->ctas() > 1) x.p[1] = make_solo(sc, elem, false);
   if (x.p[1] && x.p[1]->ctas() == x.p[0]->ctas()) x.p[1].reset();
@@ -975,7 +978,9 @@ struct gox_topo {
   // streams), and the one the tuner chose or found
   DotPair dot[2];
   std::shared_ptr<const DotProgram> dot_main[2];
-  SoloPair solo[2];            // beside them, from the topology's second solve of few scenarios on
+  // beside them, from the tuning or the second solve of few scenarios on
+  std::shared_ptr<SoloPair> solo[2] = {std::make_shared<SoloPair>(), std::make_shared<SoloPair>()};
+  bool solo_loaded[2] = {false, false};
   int small_solves[2] = {0, 0};
   DevSchedule dsched;
   DevBatch batch;
@@ -1175,7 +1180,7 @@ static int fix_pivots(gox_topo* t, int B, const double* p_spec, const double* q_
       for (int i = 0; i < 2; i++) {
         t->dot[i] = DotPair();
         t->dot_main[i].reset();
-        t->solo[i] = SoloPair();
+        t->solo[i] = std::make_shared<SoloPair>();
       }
       t->factored = true;
       t->uploaded = false;
@@ -1187,13 +1192,21 @@ static int fix_pivots(gox_topo* t, int B, const double* p_spec, const double* q_
   return -1;
 }
 
+// The solo programs to the device, where they are built (and not being built)
+static void load_solos(gox_topo* t, int i) {
+  std::unique_lock<std::mutex> lk(t->solo[i]->mu, std::try_to_lock);
+  t->solo_loaded[i] = lk && t->solo[i]->tried;
+  for (int k = 0; k < 2; k++)
+    DevSchedule::load_solo(t->dsched.solo[i][k], t->solo_loaded[i] ? t->solo[i]->p[k].get() : nullptr, 32);
+}
+
 // The schedule and the refactor plans to the device
 static void upload_plans(gox_topo* t) {
   t->dsched.load(t->sc, t->yp, t->yi, t->yre, t->yim);
   t->dsched.load_streams(t->s32, t->s64);
   for (int i = 0; i < 2; i++) {
     t->dsched.load_dot(i, t->dot[i]);
-    for (int k = 0; k < 2; k++) DevSchedule::load_solo(t->dsched.solo[i][k], t->solo[i].p[k].get(), 32);
+    load_solos(t, i);
   }
   t->uploaded = true;
 }
@@ -1530,11 +1543,20 @@ static void install_stream(gox_topo* t, int i, Stream&& s) {
 }
 
 // Before a solve of B scenarios: the solo programs, where one may run them.  Not
-// at the first such solve: a topology that is used once does not pay for them.
+// at a first such solve that does not tune: a topology that is used once does not
+// pay for them.  While a clone builds them, solves go on without.
+constexpr int kSoloMost = 1216;  // scenarios: no program runs more
 static void ensure_solo(gox_topo* t, int i, int B) {
-  if (B > 1216 || !t->dot_main[i] || t->solo[i].tried || !t->uploaded || ++t->small_solves[i] < 2) return;
-  make_solos(t->sc, i == 0 ? 4 : 8, t->solo[i]);
-  for (int k = 0; k < 2; k++) DevSchedule::load_solo(t->dsched.solo[i][k], t->solo[i].p[k].get(), 32);
+  if (B > kSoloMost || !t->dot_main[i] || t->solo_loaded[i] || !t->uploaded) return;
+  {
+    std::unique_lock<std::mutex> lk(t->solo[i]->mu, std::try_to_lock);
+    if (!lk) return;
+    if (!t->solo[i]->tried) {
+      if (++t->small_solves[i] < 2) return;
+      make_solos(t->sc, i == 0 ? 4 : 8, *t->solo[i]);
+    }
+  }
+  load_solos(t, i);
 }
 
 template <typename T>
@@ -1609,6 +1631,14 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st) {
     std::vector<std::thread> th;
     std::atomic<size_t> next{0};
     const unsigned nt = std::max(1u, std::min(8u, std::thread::hardware_concurrency()));
+    if (D.nb > 0 && D.nb <= kSoloMost)
+      th.emplace_back([&] {
+        std::unique_lock<std::mutex> lk(t->solo[i]->mu, std::try_to_lock);
+        try {
+          if (lk && !t->solo[i]->tried) make_solos(sc, elem, *t->solo[i]);
+        } catch (const std::exception&) {  // none
+        }
+      });
     for (unsigned w = 0; w < nt; w++)
       th.emplace_back([&] {
         for (size_t c; (c = next++) < cand.size() + dcand.size();) {
@@ -1711,6 +1741,7 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st) {
     const std::shared_ptr<const DotProgram> p = dbuilt[best - (int)cand.size()];
     entry = {p->plan.top_warps, kDotChunkWords, p->plan.mid, p->plan.bins};
     install_dot(t, i, p, D.G, dbuilt.back());
+    load_solos(t, i);
   } else {
     const StreamPlan& p = cand[best];
     entry = {p.nw, p.chunk_words, p.sync, p.wide_levels > 0 ? p.wide_min : 0};
@@ -3445,7 +3476,7 @@ int gox_topo_reset(gox_topo* t) {
   for (int i = 0; i < 2; i++) {
     t->dot[i] = DotPair();
     t->dot_main[i].reset();
-    t->solo[i] = SoloPair();
+    t->solo[i] = std::make_shared<SoloPair>();
   }
   t->tune[0] = gox_topo::Tuning();
   t->tune[1] = gox_topo::Tuning();

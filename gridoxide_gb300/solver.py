@@ -478,7 +478,9 @@ class Topology:
 
     def tuning(self, precision=GOX_PRECISION_MIXED) -> dict:
         """The refactor plan in `precision` and the autotuner's timed
-        candidates (gox_topo_tuning)."""
+        candidates, fastest first (gox_topo_tuning).  A dot program has 128
+        chunk_words; its wide_levels are its bins, its wide_phases its
+        mid-stage CTAs."""
         plan = np.zeros(9, np.int64)
         table = np.zeros((128, 7))
         rows = check(_lib.load().gox_topo_tuning(self._h, int(precision), _p(plan, _lib.i64p),

@@ -397,7 +397,10 @@ int gox_set_refactor_wide(int32_t min_width);
  * [3] stream-chunk words, [4] source (0 default, 1 timed by the autotuner,
  * 2 from its cache), [5] candidates timed, [6] 1 when the levels end in
  * per-warp progress flags, 0 in CTA barriers, [7] / [8] refactor levels /
- * backward phases the wide kernels run (plan must hold 9 entries).  With
+ * backward phases the wide kernels run (plan must hold 9 entries).  A dot
+ * program (the refactor as ordered sums) has 128 as its chunk words, no ring,
+ * [0] the warps of its tail's CTA, [7] its bins and [8] its mid-stage CTAs; it
+ * is the one for the batch size the topology was tuned with.  With
  * `table`, up to max_rows rows {warps, chunk words, ring rows, ms,
  * progress flags, wide levels, wide phases} of the timed candidates;
  * returns the rows written, or < 0.  Needs a fixed pivot order. */
