@@ -1419,9 +1419,9 @@ static void pivot_run(gox_topo* t, BatchDev& D, cudaStream_t st) {
 }
 
 // ---------------------------------------------------------------------------
-// Refactor autotuner.  The plan of a topology's refactor streams (warps per
-// CTA, stream-chunk words, hence ring rows) is chosen by timing the
-// candidate plans on the first batch the topology solves in a precision:
+// Refactor autotuner.  The plan of a topology's refactor (a dot program: bins,
+// mid-stage CTAs, the top's warps; or streams: warps per CTA, stream-chunk
+// words, hence ring rows) is chosen by timing the candidate plans on the first batch the topology solves in a precision:
 // after that batch's first Jacobian fill, each candidate's stream (compiled
 // on the host and checked by the host interpreter first) refactors the
 // first min(G, 152) groups of the image, twice, timed with CUDA events on

@@ -30,7 +30,7 @@ int units_of(int n) { return std::max(1, (n + kSoloTerms - 1) / kSoloTerms); }
 
 }  // namespace
 
-// The parts' CTAs, ms per refactor of one scenario with 0 / 4 / 8 / 16 / 32 / 64
+// The parts' CTAs, ms per refactor of one scenario (three units under way) with 0 / 4 / 8 / 16 / 32 / 64
 // (-: its values do not fit): 118 buses FP64 .104 / .126 / .117 / - / - / -, FP32
 // .049; 2,000 buses FP32 .540 / .397 / .380 / .367 / .360 / -, FP64 - / .769 /
 // .747 / .736 / - / -; 10,000 FP32 - / - / .637 / .592 / .562 / -; 20,000 FP32 - /

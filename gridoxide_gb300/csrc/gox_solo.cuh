@@ -15,8 +15,8 @@
 // Eight warps: with 16 the copies of the streams take the room of values (118
 // buses: the same time).
 // Refactor of one scenario with both substitutions, dot program -> solo, ms:
-// 118 buses FP64 0.156 -> 0.104; 2,000 buses FP32 0.67 -> 0.37, FP64 1.27 -> 0.74;
-// 20,000 buses FP32 1.52 -> 0.74.  152 scenarios of 2,000 buses FP32 0.69 -> 0.47;
+// 118 buses FP64 0.156 -> 0.104; 2,000 buses FP32 0.67 -> 0.31, FP64 1.27 -> 0.69;
+// 20,000 buses FP32 1.52 -> 0.59.  152 scenarios of 2,000 buses FP32 0.69 -> 0.47;
 // 600 of 118 buses FP64 0.19 -> 0.12.
 #pragma once
 #include "gox_kernels.cuh"
