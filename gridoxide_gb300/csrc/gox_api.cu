@@ -1552,7 +1552,8 @@ static void ensure_solo(gox_topo* t, int i, int B) {
     std::unique_lock<std::mutex> lk(t->solo[i]->mu, std::try_to_lock);
     if (!lk) return;
     if (!t->solo[i]->tried) {
-      if (++t->small_solves[i] < 2) return;
+      // (a variant, one of many of a Q-limit or island solve, only when used often)
+      if (++t->small_solves[i] < (t->tune_cache_only ? 16 : 2)) return;
       make_solos(t->sc, i == 0 ? 4 : 8, *t->solo[i]);
     }
   }
@@ -1570,21 +1571,28 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st) {
   const int elem = (int)sizeof(T);
   const std::array<int, 4> key = tune_key(t, i, D.G);
   {
-    std::lock_guard<std::mutex> lk(g_tune_mu);
-    tune_cache_load();
-    auto it = g_tune.find(key);
-    if (it == g_tune.end() && t->tune_cache_only) {
+    // (the lock is not held while a plan is compiled: other topologies go on)
+    bool cached = false;
+    std::array<int, 4> plan{};
+    {
+      std::lock_guard<std::mutex> lk(g_tune_mu);
+      tune_cache_load();
+      auto it = g_tune.find(key);
+      cached = it != g_tune.end();
+      if (cached) plan = it->second;
+    }
+    if (!cached && t->tune_cache_only) {
       // not timed: the program the measured rule gives
       if (fits) install_dot(t, i, make_dot(sc, dot_default(sc, elem, D.G)), D.G, nullptr);
       return;
     }
-    if (it != g_tune.end() && it->second[1] == kDotChunkWords) {
+    if (cached && plan[1] == kDotChunkWords) {
       // (timed on a batch of the key's smallest size, its mid stage can have more
       // CTAs than this batch allows: the most that it does)
       const DotPlan* found = nullptr;
       const std::vector<DotPlan> plans = dot_candidates(sc, elem, D.G);
       for (const DotPlan& p : plans)
-        if (p.top_warps == it->second[0] && p.bins == it->second[3] && p.mid <= it->second[2] &&
+        if (p.top_warps == plan[0] && p.bins == plan[3] && p.mid <= plan[2] &&
             (!found || p.mid > found->mid))
           found = &p;
       if (found && fits) {
@@ -1593,11 +1601,11 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st) {
         return;
       }
       if (t->tune_cache_only) return;
-    } else if (it != g_tune.end()) {
+    } else if (cached) {
       const Stream& cur = i == 0 ? t->s32 : t->s64;
       auto same = [&](const StreamPlan& p) {
-        return p.nw == it->second[0] && p.chunk_words == it->second[1] && p.sync == it->second[2] &&
-               (p.wide_levels > 0 ? p.wide_min : 0) == it->second[3];
+        return p.nw == plan[0] && p.chunk_words == plan[1] && p.sync == plan[2] &&
+               (p.wide_levels > 0 ? p.wide_min : 0) == plan[3];
       };
       if (same(cur.plan)) {
         TU.source = 2;
