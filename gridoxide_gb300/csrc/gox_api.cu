@@ -1212,6 +1212,7 @@ static void upload_plans(gox_topo* t) {
 }
 
 static constexpr int kSoloNewtonMax = 64;   // iterations of a loop in one launch
+static constexpr int kSoloMost = 1216;      // scenarios: no solo program runs more
 static constexpr int kGraphMinGroups = 64;  // batches of >= 2,048 scenarios
 
 // The sink (node without dependents) of a graph captured from one stream
@@ -1545,7 +1546,6 @@ static void install_stream(gox_topo* t, int i, Stream&& s) {
 // Before a solve of B scenarios: the solo programs, where one may run them.  Not
 // at a first such solve that does not tune: a topology that is used once does not
 // pay for them.  While a clone builds them, solves go on without.
-constexpr int kSoloMost = 1216;  // scenarios: no program runs more
 static void ensure_solo(gox_topo* t, int i, int B) {
   if (B > kSoloMost || !t->dot_main[i] || t->solo_loaded[i] || !t->uploaded) return;
   {
@@ -2295,7 +2295,9 @@ static int batch_prepare(gox_topo* t, int B, const double* p_spec, const double*
   DevBatch& DB = t->batch;
   DB.ensure(S, G, precision, max_iter, want_hist);
   BatchDev D = DB.view(want_hist, outage, tol, t->piv_tol);
-  D.nb = B;
+  // (left out where no solo program can run: a captured loop's key is the
+  // whole of D, and ragged batches of one group count share their graph)
+  if (B <= kSoloMost) D.nb = B;
   // inputs -> interleaved layout
   const size_t tot = (size_t)G * n * 32;
   k_scatter_rows<<<grid1d(tot), 256, 0, st>>>(p_spec, B, n, n, D.psp, G);

@@ -89,7 +89,7 @@ struct BatchDev {
   const double *o_dre, *o_dim;
   float piv_tol;                   // pivot-ratio threshold (mixed path)
   int32_t* err;                    // [0] set when a bounded device wait gave up
-  int nb;  // scenarios, where a program for few may run them (0: not)
+  int nb;  // scenarios, where a solo program may run them (0: more than any runs)
   // a start point that all scenarios share, per bus: cos, sin of its angle, e, f
   // and the current sum_k Y_ik V_k (k_shared_start); null: each has its own
   const double* st0;               // [6][n_bus]
