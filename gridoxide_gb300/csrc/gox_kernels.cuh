@@ -60,9 +60,8 @@ struct SchedDev {
 __device__ __forceinline__ double eff_inj(const double* zip, int nb, int i, int part, double s,
                                           double vm) {
   if (zip == nullptr) return s;
-  s += zip[(size_t)part * nb + i] * vm * vm;
-  s += zip[(size_t)(2 + part) * nb + i] * vm;
-  return s;
+  s = fma(__dmul_rn(zip[(size_t)part * nb + i], vm), vm, s);
+  return fma(zip[(size_t)(2 + part) * nb + i], vm, s);
 }
 
 struct BatchDev {
@@ -354,8 +353,8 @@ __device__ __forceinline__ void inject_one(const SchedDev& S, const BatchDev& D,
     const int c0 = (i == obf) ? 0 : 2;
     const double ar = D.o_dre[4 * s + c0], ai = D.o_dim[4 * s + c0];
     const double br = D.o_dre[4 * s + c0 + 1], bi = D.o_dim[4 * s + c0 + 1];
-    ir += ar * ef - ai * ff + br * et - bi * ft;
-    ii += ar * ff + ai * ef + br * ft + bi * et;
+    ir += fma(-bi, ft, fma(br, et, dif2(ar, ef, ai, ff)));
+    ii += fma(bi, et, fma(br, ft, dot2(ar, ff, ai, ef)));
   }
   const int rp = __ldg(S.bus_rowP + i), rq = __ldg(S.bus_rowQ + i);
   if constexpr (sizeof(T) == 4) {
@@ -403,7 +402,7 @@ __device__ __forceinline__ void inject_one(const SchedDev& S, const BatchDev& D,
     ((T*)D.pT)[x] = (T)pc;
     ((T*)D.qT)[x] = (T)qc;
   }
-  }
+}
 
 template <typename T, bool OUTAGE, int BPW, bool ZIP>
 __device__ __forceinline__ void inject_body(const SchedDev& S, const BatchDev& D, int it, int BX,
