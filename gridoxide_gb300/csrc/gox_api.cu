@@ -357,15 +357,20 @@ struct DevSchedule {
         if (nb <= x.max) return &x;
     return nullptr;
   }
-  // (null: none)
+  // (null, or no room for it: none)
   static void load_solo(SoloOne& x, const SoloProgram* p, int stride) {
     x.max = 0;
     if (!p) return;
-    upload(x.words, p->words);
-    upload(x.lists, p->lists);
     std::vector<SoloCta> all;
     for (const auto& l : p->launch) all.insert(all.end(), l.begin(), l.end());
-    upload(x.ctas, all);
+    try {
+      upload(x.words, p->words);
+      upload(x.lists, p->lists);
+      upload(x.ctas, all);
+    } catch (const std::bad_alloc&) {
+      for (DevMem* m : {&x.words, &x.lists, &x.ctas}) m->release();
+      return;
+    }
     x.d.words = x.words.as<uint4>();
     x.d.lists = x.lists.as<uint32_t>();
     const SoloCta* at = x.ctas.as<SoloCta>();
@@ -428,15 +433,21 @@ struct DevSchedule {
     d.n_prep2 = (int)p.prep2.size() / nt;
     d.n_midback = (int)p.midback.size() / kDotBackWarps;
   }
-  // (none: the streams)
-  void load_dot(int i, const DotPair& p) {
+  // (none, or no room for them: the streams); whether they are used
+  bool load_dot(int i, const DotPair& p) {
     DotPlanDev& x = dot[i];
-    x.on = p.few || p.many;
-    if (!x.on) return;
+    x.on = false;
+    if (!p.few && !p.many) return false;
     x.with_subst = (p.few ? p.few : p.many)->with_subst;
     x.few_groups = p.few_groups();
-    if (p.few) load_one(x.few, *p.few);
-    if (p.many) load_one(x.many, *p.many);
+    try {
+      if (p.few) load_one(x.few, *p.few);
+      if (p.many) load_one(x.many, *p.many);
+    } catch (const std::bad_alloc&) {
+      for (DevMem* m : {&x.few.words, &x.few.starts, &x.many.words, &x.many.starts}) m->release();
+      return false;
+    }
+    return x.on = true;
   }
 
   void load_streams(const Stream& s32, const Stream& s64) {
@@ -672,26 +683,38 @@ static void make_streams(const Schedule& sc, Stream& s32, Stream& s64) {
 }
 
 // A program through the checking host interpreter, as every stream: indices,
-// order of each sum, no value read before it is final.
+// order of each sum, no value read before it is final.  Null for a plan that
+// does not compile, or whose program does not pass (said on stderr): a topology
+// has its streams, which run in its place.
 static std::shared_ptr<const DotProgram> make_dot(const Schedule& sc, const DotPlan& plan) {
-  auto p = std::make_shared<DotProgram>();
-  build_dot(sc, plan, *p);
-  std::vector<double> lu(sc.n_slots, 1.0), rhs(sc.n_u, 0.0), X;
-  bool sing = false;
-  const std::string e = run_dot_host(sc, *p, lu, rhs, X, sing);
-  if (!e.empty()) throw std::runtime_error("dot program check: " + e);
-  return p;
+  try {
+    auto p = std::make_shared<DotProgram>();
+    build_dot(sc, plan, *p);
+    std::vector<double> lu(sc.n_slots, 1.0), rhs(sc.n_u, 0.0), X;
+    bool sing = false;
+    const std::string e = run_dot_host(sc, *p, lu, rhs, X, sing);
+    if (e.empty()) return p;
+    std::fprintf(stderr, "gridoxide_gb300: a dot program is not used: %s\n", e.c_str());
+  } catch (const std::exception& e) {
+    std::fprintf(stderr, "gridoxide_gb300: a dot program is not used: %s\n", e.what());
+  }
+  return nullptr;
 }
 
 // A solo program, checked likewise (null: there is none).
 static std::shared_ptr<const SoloProgram> make_solo(const Schedule& sc, int elem, bool wide) {
-  auto p = std::make_shared<SoloProgram>();
-  if (!build_solo_default(sc, elem, wide, *p)) return nullptr;
-  std::vector<double> lu(sc.n_slots, 1.0), rhs(sc.n_u, 0.0), X;
-  bool sing = false;
-  const std::string e = run_solo_host(sc, *p, lu, rhs, X, sing);
-  if (!e.empty()) throw std::runtime_error("solo program check: " + e);
-  return p;
+  try {
+    auto p = std::make_shared<SoloProgram>();
+    if (!build_solo_default(sc, elem, wide, *p)) return nullptr;
+    std::vector<double> lu(sc.n_slots, 1.0), rhs(sc.n_u, 0.0), X;
+    bool sing = false;
+    const std::string e = run_solo_host(sc, *p, lu, rhs, X, sing);
+    if (e.empty()) return p;
+    std::fprintf(stderr, "gridoxide_gb300: a solo program is not used: %s\n", e.c_str());
+  } catch (const std::exception& e) {
+    std::fprintf(stderr, "gridoxide_gb300: a solo program is not used: %s\n", e.what());
+  }
+  return nullptr;
 }
 // The solo programs of a schedule: one for the fewest scenarios and, where that
 // one has several CTAs, one for more.
@@ -978,6 +1001,7 @@ struct gox_topo {
   // streams), and the one the tuner chose or found
   DotPair dot[2];
   std::shared_ptr<const DotProgram> dot_main[2];
+  bool no_dot_other[2] = {false, false};  // the other kind did not compile: not tried again
   // beside them, from the tuning or the second solve of few scenarios on
   std::shared_ptr<SoloPair> solo[2] = {std::make_shared<SoloPair>(), std::make_shared<SoloPair>()};
   bool solo_loaded[2] = {false, false};
@@ -1180,6 +1204,7 @@ static int fix_pivots(gox_topo* t, int B, const double* p_spec, const double* q_
       for (int i = 0; i < 2; i++) {
         t->dot[i] = DotPair();
         t->dot_main[i].reset();
+        t->no_dot_other[i] = false;
         t->solo[i] = std::make_shared<SoloPair>();
       }
       t->factored = true;
@@ -1200,12 +1225,19 @@ static void load_solos(gox_topo* t, int i) {
     DevSchedule::load_solo(t->dsched.solo[i][k], t->solo_loaded[i] ? t->solo[i]->p[k].get() : nullptr, 32);
 }
 
+// The dot programs to the device (without room there: the streams)
+static void load_dots(gox_topo* t, int i) {
+  if (t->dsched.load_dot(i, t->dot[i])) return;
+  t->dot[i] = DotPair();
+  t->dot_main[i].reset();
+}
+
 // The schedule and the refactor plans to the device
 static void upload_plans(gox_topo* t) {
   t->dsched.load(t->sc, t->yp, t->yi, t->yre, t->yim);
   t->dsched.load_streams(t->s32, t->s64);
   for (int i = 0; i < 2; i++) {
-    t->dsched.load_dot(i, t->dot[i]);
+    load_dots(t, i);
     load_solos(t, i);
   }
   t->uploaded = true;
@@ -1509,7 +1541,7 @@ static void install_dot(gox_topo* t, int i, std::shared_ptr<const DotProgram> p,
   for (gox_topo* x = t; x; x = x->twin.get()) {  // and the split solves' twins
     x->dot[i] = few ? DotPair{p, other} : DotPair{other, p};
     x->dot_main[i] = p;
-    if (x->uploaded) x->dsched.load_dot(i, x->dot[i]);
+    if (x->uploaded) load_dots(x, i);
     drop_loops(x, i);
   }
 }
@@ -1521,12 +1553,14 @@ static DotPlan dot_other(const Schedule& sc, int elem, int groups) {
 // topology's plan was found in the cache and only its own kind is built.
 static void ensure_dot_kind(gox_topo* t, int i, int groups) {
   const std::shared_ptr<const DotProgram> p = t->dot_main[i];
-  if (!p || t->tune_cache_only || (t->dot[i].few && t->dot[i].many)) return;
+  if (!p || t->tune_cache_only || t->no_dot_other[i] || (t->dot[i].few && t->dot[i].many)) return;
   const int elem = i == 0 ? 4 : 8;
   const bool few = p == t->dot[i].few;
   if (few ? dot_few(p->plan, groups) : !dot_few(dot_default(t->sc, elem, 1), groups)) return;
   const int own = few ? 1 : 152;
-  install_dot(t, i, p, own, make_dot(t->sc, dot_other(t->sc, elem, own)));
+  const std::shared_ptr<const DotProgram> other = make_dot(t->sc, dot_other(t->sc, elem, own));
+  t->no_dot_other[i] = !other;
+  if (other) install_dot(t, i, p, own, other);
 }
 
 static void install_stream(gox_topo* t, int i, Stream&& s) {
@@ -1595,8 +1629,9 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st) {
         if (p.top_warps == plan[0] && p.bins == plan[3] && p.mid <= plan[2] &&
             (!found || p.mid > found->mid))
           found = &p;
-      if (found && fits) {
-        install_dot(t, i, make_dot(sc, *found), D.G, nullptr);
+      const std::shared_ptr<const DotProgram> p = found && fits ? make_dot(sc, *found) : nullptr;
+      if (p) {
+        install_dot(t, i, p, D.G, nullptr);
         TU.source = 2;
         return;
       }
@@ -1642,22 +1677,13 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st) {
     if (D.nb > 0 && D.nb <= kSoloMost)
       th.emplace_back([&] {
         std::unique_lock<std::mutex> lk(t->solo[i]->mu, std::try_to_lock);
-        try {
-          if (lk && !t->solo[i]->tried) make_solos(sc, elem, *t->solo[i]);
-        } catch (const std::exception&) {  // none
-        }
+        if (lk && !t->solo[i]->tried) make_solos(sc, elem, *t->solo[i]);
       });
     for (unsigned w = 0; w < nt; w++)
       th.emplace_back([&] {
         for (size_t c; (c = next++) < cand.size() + dcand.size();) {
-          if (c < cand.size()) {
-            ok[c] = compile_checked(sc, cand[c], built[c]);
-          } else {
-            try {
-              dbuilt[c - cand.size()] = make_dot(sc, dcand[c - cand.size()]);
-            } catch (const std::exception&) {  // not a candidate
-            }
-          }
+          if (c < cand.size()) ok[c] = compile_checked(sc, cand[c], built[c]);
+          else dbuilt[c - cand.size()] = make_dot(sc, dcand[c - cand.size()]);
         }
       });
     for (auto& x : th) x.join();
@@ -1699,7 +1725,11 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st) {
     if (c >= cand.size()) {
       const DotProgram* p = dbuilt[c - cand.size()].get();
       if (!p) continue;
-      DevSchedule::load_one(dev, *p);
+      try {
+        DevSchedule::load_one(dev, *p);
+      } catch (const std::bad_alloc&) {  // not a candidate
+        continue;
+      }
       const float ms = time_plan([&] { Iter<T>::dot(dev.d, t->dsched.d, D, Gt, st); });
       if (ms < 0.0f) continue;
       TU.table.push_back({(double)p->plan.top_warps, (double)kDotChunkWords, 0.0, (double)ms, 0.0,
@@ -3486,6 +3516,7 @@ int gox_topo_reset(gox_topo* t) {
   for (int i = 0; i < 2; i++) {
     t->dot[i] = DotPair();
     t->dot_main[i].reset();
+    t->no_dot_other[i] = false;
     t->solo[i] = std::make_shared<SoloPair>();
   }
   t->tune[0] = gox_topo::Tuning();
