@@ -139,9 +139,8 @@ struct Writer {
     flush();
     room(1);
     raw(DOT_END, 0u, 0u, 0u);
-    // a warp loads up to three chunks past the one it is in
     while (w.size() % (4 * kDotChunk)) w.push_back(0);
-    w.insert(w.end(), 4 * kDotChunk * 3, 0u);
+    w.insert(w.end(), 4 * kDotChunk * kDotAhead, 0u);
   }
 };
 
@@ -873,7 +872,7 @@ std::string run_dot_host(const Schedule& sc, const DotProgram& P, std::vector<do
   auto step = [&](Warp& A, int w, bool top) -> bool {
     if (!A.waits && A.bars > 0 && --A.bars > 0) return true;
     for (;;) {
-      if (A.pos >= nq) return fail("a stream runs past the program");
+      if ((A.pos / kDotChunk + 1 + kDotAhead) * kDotChunk > nq) return fail("a stream runs past the program");
       const uint32_t* h = &P.words[A.pos * 4];
       const uint32_t op = h[0] & 15u;
       if (!((may >> op) & 1u)) return fail("a unit in the wrong launch");

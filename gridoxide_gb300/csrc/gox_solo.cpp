@@ -510,8 +510,7 @@ bool build_solo(const Schedule& sc, const SoloPlan& plan, SoloProgram& P) {
     backward(m, t);
     streams(t, 0, 3);
   }
-  // a warp loads up to three units past the one it is in
-  P.words.insert(P.words.end(), 4 * kSoloQuads * 4, 0u);
+  P.words.insert(P.words.end(), (size_t)kSoloAhead * kSoloQuads * 4, 0u);
   return *std::max_element(P.max_values, P.max_values + 4) <= max_values;
 }
 
@@ -584,7 +583,7 @@ std::string run_solo_host(const Schedule& sc, const SoloProgram& P, std::vector<
     if (w.bars > 0 && --w.bars > 0) return true;
     if (w.ended) return true;
     for (;;) {
-      if (w.at + 3 >= nu) return fail("a stream runs past the program");
+      if (w.at + kSoloAhead >= nu) return fail("a stream runs past the program");
       const uint32_t* u = &P.words[w.at * kSoloQuads * 4];
       auto word = [&](int l, int i) { return u[((i / 4) * 32 + l) * 4 + i % 4]; };
       const uint32_t f = word(0, 11);

@@ -56,6 +56,8 @@ constexpr int kSoloWarps = 8;
 // .97 / .735 / .645 / .594 / .592; 600 scenarios of 118 buses FP64, which fit the
 // chip with 3 only, .119 with 3 and .197 with 5).
 constexpr int kSoloDepth = 3, kSoloDeep = 5;
+constexpr int kSoloAhead = kSoloDeep - 1;  // units that are read past the one run (a program ends in as many)
+static_assert(kSoloDeep >= kSoloDepth, "the deeper ring is the one that reads further");
 constexpr int solo_ring_bytes(int depth) { return kSoloWarps * depth * kSoloQuads * 16; }
 constexpr int kSoloSmem = 226 * 1024;  // of a CTA (1 KB is left for the kernel's own)
 constexpr int kSoloMaxBytes = kSoloSmem - solo_ring_bytes(kSoloDepth);  // a CTA's values
