@@ -1581,7 +1581,7 @@ static void install_stream(gox_topo* t, int i, Stream&& s) {
 // at a first such solve that does not tune: a topology that is used once does not
 // pay for them.  While a clone builds them, solves go on without.
 static void ensure_solo(gox_topo* t, int i, int B) {
-  if (B > kSoloMost || !t->dot_main[i] || t->solo_loaded[i] || !t->uploaded) return;
+  if (!t->dot_main[i] || t->solo_loaded[i] || !t->uploaded || B > solo_most(t->sc, i == 0 ? 4 : 8)) return;
   {
     std::unique_lock<std::mutex> lk(t->solo[i]->mu, std::try_to_lock);
     if (!lk) return;
@@ -1674,7 +1674,7 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st) {
     std::vector<std::thread> th;
     std::atomic<size_t> next{0};
     const unsigned nt = std::max(1u, std::min(8u, std::thread::hardware_concurrency()));
-    if (D.nb > 0 && D.nb <= kSoloMost)
+    if (D.nb > 0 && D.nb <= solo_most(sc, elem))
       th.emplace_back([&] {
         std::unique_lock<std::mutex> lk(t->solo[i]->mu, std::try_to_lock);
         if (lk && !t->solo[i]->tried) make_solos(sc, elem, *t->solo[i]);

@@ -26,6 +26,11 @@ struct Vec {
 // A CTA's ticks
 using Ticks = std::vector<std::vector<Vec>>;
 
+// A schedule that solo programs can be compiled from
+bool solo_possible(const Schedule& sc) {
+  return sc.fuse_fwd && sc.n_u > 0 && (int64_t)sc.n_slots + sc.n_u < (1 << 28);
+}
+
 int units_of(int n) { return std::max(1, (n + kSoloTerms - 1) / kSoloTerms); }
 
 }  // namespace
@@ -35,7 +40,11 @@ int units_of(int n) { return std::max(1, (n + kSoloTerms - 1) / kSoloTerms); }
 // .049; 2,000 buses FP32 .540 / .397 / .380 / .367 / .360 / -, FP64 - / .769 /
 // .747 / .736 / - / -; 10,000 FP32 - / - / .637 / .592 / .562 / -; 20,000 FP32 - /
 // - / - / .905 / .735 / .819.
+static bool build_solo(const Schedule& sc, const Sums& S, const SoloPlan& plan, SoloProgram& P);
 bool build_solo_default(const Schedule& sc, int elem, bool wide, SoloProgram& out) {
+  out = SoloProgram();
+  if (!solo_possible(sc)) return false;
+  const Sums S = make_sums(sc);
   SoloPlan p;
   p.elem = elem;
   // (the values of the parts together, some twice)
@@ -44,9 +53,18 @@ bool build_solo_default(const Schedule& sc, int elem, bool wide, SoloProgram& ou
   for (int ctas : {0, 4, 8, 16, 32, 64}) {
     if (ctas < best || (ctas > 0 && ctas < share)) continue;
     p.ctas = ctas;
-    if (build_solo(sc, p, out)) return true;
+    if (build_solo(sc, S, p, out)) return true;
   }
   return false;
+}
+
+int solo_most(const Schedule& sc, int elem) {
+  if (!solo_possible(sc)) return 0;
+  // one CTA: places by its values; several: an SM has eight places at most, the
+  // parts have four CTAs at least
+  const int64_t bytes = solo_ring_bytes(kSoloDepth) + ((int64_t)sc.n_slots + sc.n_u + 1) * elem;
+  const int64_t one = bytes <= kSoloSmem ? 152 * std::min<int64_t>(8, (228 * 1024) / (bytes + 1024)) : 0;
+  return (int)std::max<int64_t>(one, 152 * 8 / 4);
 }
 
 int solo_scenarios(const SoloProgram& p, int depth) {
@@ -64,12 +82,15 @@ int solo_scenarios(const SoloProgram& p, int depth) {
 
 bool build_solo(const Schedule& sc, const SoloPlan& plan, SoloProgram& P) {
   P = SoloProgram();
+  return solo_possible(sc) && build_solo(sc, make_sums(sc), plan, P);
+}
+
+static bool build_solo(const Schedule& sc, const Sums& S, const SoloPlan& plan, SoloProgram& P) {
+  P = SoloProgram();
   P.plan = plan;
-  if (!sc.fuse_fwd || sc.n_u == 0 || (int64_t)sc.n_slots + sc.n_u >= (1 << 28)) return false;
   const int max_values = kSoloMaxBytes / plan.elem;
   const int n = sc.n_u, ns = sc.n_slots, zero = ns + n;
   if (plan.ctas == 0 && zero + 1 > max_values) return false;
-  const Sums S = make_sums(sc);
   auto nt = [&](int v) { return S.ptr[v + 1] - S.ptr[v]; };
   Parts parts(sc, S);
   std::vector<int32_t> cta(n, -1);
@@ -84,8 +105,68 @@ bool build_solo(const Schedule& sc, const SoloPlan& plan, SoloProgram& P) {
     }
   }
   const std::vector<char>& stage = parts.stage;
-  std::vector<int32_t> taken(ns + n, 0), stop(S.ptr.begin() + 1, S.ptr.end()), done(ns + n, -1), from(ns + n, 0);
   auto second = [&](int v, int t) { return v >= ns ? ns + S.b[t] : S.b[t]; };
+  // The values that the parts' and the rest's CTAs use, before anything is
+  // scheduled: a plan they do not fit is left here (20,000 buses FP64, where none
+  // fits: 1,480 ms on one core -> 40; 50,000 buses FP32 3,900 -> 95).
+  {
+    std::vector<int32_t> by(zero, -1), begin(S.ptr.begin(), S.ptr.end() - 1);  // begin: past what the second launch ran
+    if (!mid.empty())
+      for (int k = 0; k < n; k++) {
+        if (stage[k] != 2) continue;
+        auto leading = [&](int v) {
+          for (int& t = begin[v]; t < S.ptr[v + 1]; t++)
+            if (stage[S.col[S.a[t]]] > 1 || (v >= ns ? stage[S.b[t]] > 1 : begin[S.b[t]] < S.ptr[S.b[t] + 1])) break;
+        };
+        for (int v = sc.c_base[k]; v <= sc.c_base[k] + sc.c_ulen[k] + sc.c_llen[k]; v++) leading(v);
+        leading(ns + k);
+      }
+    int32_t id = 0;
+    int64_t used = 0;
+    auto use = [&](int v) {
+      used += by[v] != id;
+      by[v] = id;
+    };
+    auto sum = [&](int v, bool always) {
+      if (always || begin[v] < S.ptr[v + 1]) use(v);
+      for (int t = begin[v]; t < S.ptr[v + 1]; t++) {
+        use(S.a[t]);
+        use(second(v, t));
+      }
+    };
+    auto column = [&](int k) {
+      const int d = sc.c_base[k] + sc.c_ulen[k];
+      for (int v = sc.c_base[k]; v <= d + sc.c_llen[k]; v++) sum(v, v >= d);
+      sum(ns + k, false);
+    };
+    auto row = [&](int k) {
+      use(ns + k);
+      use(sc.diag_slot[k]);
+      for (int t = sc.bw_ptr[k]; t < sc.bw_ptr[k + 1]; t++) {
+        use(sc.bw_slot[t]);
+        use(ns + sc.bw_col[t]);
+      }
+    };
+    auto fits = [&]() {
+      const bool ok = used + 1 <= max_values;
+      id++;
+      used = 0;
+      return ok;
+    };
+    for (const auto& m : mid) {
+      for (int k : m) column(k);
+      if (!fits()) return false;
+      for (int k : m) row(k);
+      if (!fits()) return false;
+    }
+    for (int k = 0; k < n; k++)
+      if (stage[k] == 2) {
+        column(k);
+        row(k);
+      }
+    if (!fits()) return false;
+  }
+  std::vector<int32_t> taken(ns + n, 0), stop(S.ptr.begin() + 1, S.ptr.end()), done(ns + n, -1), from(ns + n, 0);
 
   // ---- a CTA's forward ticks: nodes (a leading part of a sum, a sum, a column's
   // pivot and L entries), each in a tick after the ticks of what it reads

@@ -95,6 +95,9 @@ bool build_solo(const Schedule& sc, const SoloPlan& plan, SoloProgram& out);
 // The program for a batch of one (wide) or for as many scenarios as possible:
 // the parts' CTAs that measured best, or as few as fit.
 bool build_solo_default(const Schedule& sc, int elem, bool wide, SoloProgram& out);
+// Scenarios that a program of the schedule could run at most, by the sizes alone
+// (more: none is compiled for them).
+int solo_most(const Schedule& sc, int elem);
 // Scenarios whose CTAs find a place on the chip at once, with `depth` units of a
 // warp in shared memory (0: its values leave no room for them).
 int solo_scenarios(const SoloProgram& p, int depth);
