@@ -727,9 +727,12 @@ struct SoloPair {
 static void make_solos(const Schedule& sc, int elem, SoloPair& x) {
   x.tried = true;
   if (sc.n_slots > 700000) return;  // (its rest does not fit: not worth the attempts)
+  std::thread more;  // (from 1,000 unknowns on the first one has several CTAs)
+  if (sc.n_u >= 1000) more = std::thread([&] { x.p[1] = make_solo(sc, elem, false); });
   x.p[0] = make_solo(sc, elem, true);
-  if (x.p[0] && x.p[0]->ctas() > 1) x.p[1] = make_solo(sc, elem, false);
-  if (x.p[1] && x.p[1]->ctas() == x.p[0]->ctas()) x.p[1].reset();
+  if (more.joinable()) more.join();
+  else if (x.p[0] && x.p[0]->ctas() > 1) x.p[1] = make_solo(sc, elem, false);
+  if (x.p[1] && (!x.p[0] || x.p[1]->ctas() == x.p[0]->ctas())) x.p[1].reset();
 }
 
 struct Timing {
@@ -1577,9 +1580,13 @@ static void install_stream(gox_topo* t, int i, Stream&& s) {
   }
 }
 
-// Before a solve of B scenarios: the solo programs, where one may run them.  Not
-// at a first such solve that does not tune: a topology that is used once does not
-// pay for them.  While a clone builds them, solves go on without.
+// Before a solve of B scenarios: the solo programs, where one may run them.  They
+// are compiled beside the tuning of a topology's first solve, or its cached plan,
+// where that solve is of few scenarios; else once as many such solves have gone
+// without them as have lost about what compiling takes (ms, against what a solve
+// loses: 118 buses FP64 1.7 / .5, 300 3.7 / .4, 2,000 FP64 69 / 1.9, 10,000 360 / 2.5,
+// 20,000 760 / 5.7, on one thread).  While a clone compiles them, solves go on
+// without.
 static void ensure_solo(gox_topo* t, int i, int B) {
   if (!t->dot_main[i] || t->solo_loaded[i] || !t->uploaded || B > solo_most(t->sc, i == 0 ? 4 : 8)) return;
   {
@@ -1587,15 +1594,17 @@ static void ensure_solo(gox_topo* t, int i, int B) {
     if (!lk) return;
     if (!t->solo[i]->tried) {
       // (a variant, one of many of a Q-limit or island solve, only when used often)
-      if (++t->small_solves[i] < (t->tune_cache_only ? 16 : 2)) return;
+      const int wait = std::min(2 + t->sc.n_slots / 2500, 64);
+      if (++t->small_solves[i] < (t->tune_cache_only ? std::max(16, wait) : wait)) return;
       make_solos(t->sc, i == 0 ? 4 : 8, *t->solo[i]);
     }
   }
   load_solos(t, i);
 }
 
+// (solos: the solve may run solo programs)
 template <typename T>
-static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st) {
+static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st, bool solos) {
   const int i = sizeof(T) == 4 ? 0 : 1;
   gox_topo::Tuning& TU = t->tune[i];
   TU.done = true;
@@ -1604,6 +1613,11 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st) {
   const bool fits = dot_fits(sc);
   const int elem = (int)sizeof(T);
   const std::array<int, 4> key = tune_key(t, i, D.G);
+  solos = solos && D.nb > 0 && D.nb <= solo_most(sc, elem);
+  auto build_solos = [&] {
+    std::unique_lock<std::mutex> lk(t->solo[i]->mu, std::try_to_lock);
+    if (lk && !t->solo[i]->tried) make_solos(sc, elem, *t->solo[i]);
+  };
   {
     // (the lock is not held while a plan is compiled: other topologies go on)
     bool cached = false;
@@ -1629,7 +1643,13 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st) {
         if (p.top_warps == plan[0] && p.bins == plan[3] && p.mid <= plan[2] &&
             (!found || p.mid > found->mid))
           found = &p;
-      const std::shared_ptr<const DotProgram> p = found && fits ? make_dot(sc, *found) : nullptr;
+      std::shared_ptr<const DotProgram> p;
+      if (found && fits) {
+        std::thread beside;
+        if (solos) beside = std::thread(build_solos);
+        p = make_dot(sc, *found);
+        if (beside.joinable()) beside.join();
+      }
       if (p) {
         install_dot(t, i, p, D.G, nullptr);
         TU.source = 2;
@@ -1674,11 +1694,7 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st) {
     std::vector<std::thread> th;
     std::atomic<size_t> next{0};
     const unsigned nt = std::max(1u, std::min(8u, std::thread::hardware_concurrency()));
-    if (D.nb > 0 && D.nb <= solo_most(sc, elem))
-      th.emplace_back([&] {
-        std::unique_lock<std::mutex> lk(t->solo[i]->mu, std::try_to_lock);
-        if (lk && !t->solo[i]->tried) make_solos(sc, elem, *t->solo[i]);
-      });
+    if (solos) th.emplace_back(build_solos);
     for (unsigned w = 0; w < nt; w++)
       th.emplace_back([&] {
         for (size_t c; (c = next++) < cand.size() + dcand.size();) {
@@ -1779,7 +1795,7 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st) {
     const std::shared_ptr<const DotProgram> p = dbuilt[best - (int)cand.size()];
     entry = {p->plan.top_warps, kDotChunkWords, p->plan.mid, p->plan.bins};
     install_dot(t, i, p, D.G, dbuilt.back());
-    load_solos(t, i);
+    if (solos) load_solos(t, i);
   } else {
     const StreamPlan& p = cand[best];
     entry = {p.nw, p.chunk_words, p.sync, p.wide_levels > 0 ? p.wide_min : 0};
@@ -1954,7 +1970,7 @@ static void run_iterations(gox_topo* t, BatchDev D, int max_iter, bool outage, c
     }
     Iter<T>::fill(S, D, outage, st);
     if (!pivoting && !t->tune[sizeof(T) == 4 ? 0 : 1].done) {
-      autotune<T>(t, D, st);
+      autotune<T>(t, D, st, true);
       tuned_now = true;
     }
     rec();
@@ -2752,7 +2768,7 @@ static void run_multi(const std::vector<gox_topo*>& ts, std::vector<BatchRun>& r
     bool retuned = false;
     for (int j : act)
       if (!ts[j]->tune[i].done) {
-        autotune<T>(ts[j], runs[j].D, st);
+        autotune<T>(ts[j], runs[j].D, st, false);
         retuned = true;
       }
     if (retuned) {
