@@ -14,11 +14,14 @@
 #include <cstdlib>
 #include <climits>
 #include <cstring>
+#include <exception>
+#include <initializer_list>
 #include <memory>
 #include <mutex>
 #include <new>
 #include <stdexcept>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -663,23 +666,45 @@ static std::atomic<int> g_refactor_sync{0};
 // kernels (0: none; gox_set_refactor_wide).
 static std::atomic<int> g_refactor_wide{0};
 
+// Host work side by side: the last of `fs` on this thread, the others on threads
+// of their own; an exception of any of them leaves when all have ended.
+static void side_by_side(std::initializer_list<std::function<void()>> fs) {
+  std::vector<std::exception_ptr> failed(fs.size());
+  std::vector<std::thread> th;
+  th.reserve(fs.size());
+  auto run = [&](size_t k) {
+    try {
+      fs.begin()[k]();
+    } catch (...) {
+      failed[k] = std::current_exception();
+    }
+  };
+  size_t k = 0;
+  try {
+    for (; k + 1 < fs.size(); k++) th.emplace_back(run, k);
+  } catch (const std::system_error&) {  // no more threads: the rest here
+  }
+  for (; k < fs.size(); k++) run(k);
+  for (auto& x : th) x.join();
+  for (auto& e : failed)
+    if (e) std::rethrow_exception(e);
+}
+
 // Compiles the refactor streams of a schedule for both precisions.
 static void make_streams(const Schedule& sc, Stream& s32, Stream& s64) {
-  std::string why;
   const int sync = g_refactor_sync.load(), wide = g_refactor_wide.load();
-  if (!choose_stream(sc, 4, kRefactorSmem, s32, why, sync, wide))
-    throw std::runtime_error("refactor schedule (FP32): " + why);
-  if (!choose_stream(sc, 8, kRefactorSmem, s64, why, sync, wide))
-    throw std::runtime_error("refactor schedule (FP64): " + why);
-  // every stream runs once through the checking host interpreter before a
-  // GPU sees it (indices, copies waited for, no cross-warp conflicts)
-  std::vector<double> lu(sc.n_slots, 1.0), rhs(sc.n_u, 0.0), X;
-  bool sing = false;
-  for (const Stream* s : {&s32, &s64}) {
-    std::fill(lu.begin(), lu.end(), 1.0);
-    const std::string e = run_stream_host(sc, *s, lu, rhs, X, sing);
+  auto make = [&](int elem, Stream& s) {
+    std::string why;
+    if (!choose_stream(sc, elem, kRefactorSmem, s, why, sync, wide))
+      throw std::runtime_error((elem == 4 ? "refactor schedule (FP32): " : "refactor schedule (FP64): ") + why);
+    // every stream runs once through the checking host interpreter before a
+    // GPU sees it (indices, copies waited for, no cross-warp conflicts)
+    std::vector<double> lu(sc.n_slots, 1.0), rhs(sc.n_u, 0.0), X;
+    bool sing = false;
+    const std::string e = run_stream_host(sc, s, lu, rhs, X, sing);
     if (!e.empty()) throw std::runtime_error("refactor stream check: " + e);
-  }
+  };
+  side_by_side({[&] { make(4, s32); }, [&] { make(8, s64); }});
 }
 
 // A program through the checking host interpreter, as every stream: indices,
@@ -727,11 +752,12 @@ struct SoloPair {
 static void make_solos(const Schedule& sc, int elem, SoloPair& x) {
   x.tried = true;
   if (sc.n_slots > 700000) return;  // (its rest does not fit: not worth the attempts)
-  std::thread more;  // (from 1,000 unknowns on the first one has several CTAs)
-  if (sc.n_u >= 1000) more = std::thread([&] { x.p[1] = make_solo(sc, elem, false); });
-  x.p[0] = make_solo(sc, elem, true);
-  if (more.joinable()) more.join();
-  else if (x.p[0] && x.p[0]->ctas() > 1) x.p[1] = make_solo(sc, elem, false);
+  if (sc.n_u >= 1000) {  // (the first one has several CTAs)
+    side_by_side({[&] { x.p[1] = make_solo(sc, elem, false); }, [&] { x.p[0] = make_solo(sc, elem, true); }});
+  } else {
+    x.p[0] = make_solo(sc, elem, true);
+    if (x.p[0] && x.p[0]->ctas() > 1) x.p[1] = make_solo(sc, elem, false);
+  }
   if (x.p[1] && (!x.p[0] || x.p[1]->ctas() == x.p[0]->ctas())) x.p[1].reset();
 }
 
@@ -1645,10 +1671,8 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st, bool solos
           found = &p;
       std::shared_ptr<const DotProgram> p;
       if (found && fits) {
-        std::thread beside;
-        if (solos) beside = std::thread(build_solos);
-        p = make_dot(sc, *found);
-        if (beside.joinable()) beside.join();
+        if (solos) side_by_side({build_solos, [&] { p = make_dot(sc, *found); }});
+        else p = make_dot(sc, *found);
       }
       if (p) {
         install_dot(t, i, p, D.G, nullptr);
@@ -1693,7 +1717,11 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st, bool solos
   {
     std::vector<std::thread> th;
     std::atomic<size_t> next{0};
-    const unsigned nt = std::max(1u, std::min(8u, std::thread::hardware_concurrency()));
+    // (with 8 threads, and one thread for the streams of both precisions, the dot plans
+    // had made a topology's first solve 6 to 20 % longer; ms, streams only / with the dot
+    // plans / with 16 threads and two: 300 buses 102 / 124 / 98, 1,500 459 / 549 / 410,
+    // 10,000 2,642 / 2,998 / 2,067)
+    const unsigned nt = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
     if (solos) th.emplace_back(build_solos);
     for (unsigned w = 0; w < nt; w++)
       th.emplace_back([&] {
@@ -2095,12 +2123,16 @@ static void guess_build(gox_topo* t, const double* p0, const double* q0) {
   }
   if (klu_factor(G.csc, packed.data(), G.sym, 0.001, G.num) != 0) return;
   build_schedule(nullptr, G.csc, G.sym, G.num, G.sc);
-  make_streams(G.sc, G.s32, G.s64);
+  DotPair dots;
+  auto dot = [&](int groups) {
+    return dot_fits(G.sc) ? make_dot(G.sc, dot_default(G.sc, 8, groups)) : std::shared_ptr<const DotProgram>();
+  };
+  side_by_side({[&] { dots.few = dot(1); }, [&] { dots.many = dot(152); }, [&] { make_streams(G.sc, G.s32, G.s64); }});
   std::vector<int32_t> dummy_p(1, 0), dummy_i;
   std::vector<double> dummy_x;
   G.dsched.load(G.sc, dummy_p, dummy_i, dummy_x, dummy_x);
   G.dsched.load_streams(G.s32, G.s64);
-  if (dot_fits(G.sc)) G.dsched.load_dot(1, DotPair{make_dot(G.sc, dot_default(G.sc, 8, 1)), make_dot(G.sc, dot_default(G.sc, 8, 152))});
+  G.dsched.load_dot(1, dots);
   // value recipe per LU slot, then per off-diagonal entry
   const int ns = G.sc.n_slots, no = G.sc.n_off;
   std::vector<int32_t> rec((size_t)(ns + no) * 4);
@@ -4567,13 +4599,17 @@ int gox_ls_create(int32_t n, int32_t nnz, const int32_t* rows, const int32_t* co
     for (int e = 0; e < nnz; e++) h->packed[h->csc.slot_of[e]] += vals[e];
     if (klu_factor(h->csc, h->packed.data(), h->sym, 0.001, h->num) != 0) return GOX_SINGULAR;
     build_schedule(nullptr, h->csc, h->sym, h->num, h->sc);
-    make_streams(h->sc, h->s32, h->s64);
+    std::shared_ptr<const DotProgram> dot;
+    std::shared_ptr<const SoloProgram> solo;
+    side_by_side({[&] { solo = make_solo(h->sc, 8, true); },
+                  [&] { if (dot_fits(h->sc)) dot = make_dot(h->sc, dot_default(h->sc, 8, 1)); },
+                  [&] { make_streams(h->sc, h->s32, h->s64); }});
     std::vector<int32_t> dummy_p(1, 0), dummy_i;
     std::vector<double> dummy_x;
     h->dsched.load(h->sc, dummy_p, dummy_i, dummy_x, dummy_x);
     h->dsched.load_streams(h->s32, h->s64);
-    if (dot_fits(h->sc)) h->dsched.load_dot(1, DotPair{make_dot(h->sc, dot_default(h->sc, 8, 1)), nullptr});
-    if (auto p = make_solo(h->sc, 8, true)) DevSchedule::load_solo(h->dsched.solo[1][0], p.get(), 1);
+    h->dsched.load_dot(1, DotPair{dot, nullptr});
+    DevSchedule::load_solo(h->dsched.solo[1][0], solo.get(), 1);
     const SchedDev& S = h->dsched.d;
     h->jbuf.ensure((size_t)S.n_a * 32 * 8 + 8);
     h->lu.ensure((size_t)S.n_slots * 32 * 8 + 8);
