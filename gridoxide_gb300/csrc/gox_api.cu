@@ -1607,19 +1607,18 @@ static void install_stream(gox_topo* t, int i, Stream&& s) {
 }
 
 // Before a solve of B scenarios: the solo programs, where one may run them.  They
-// are compiled beside the tuning of a topology's first solve, or its cached plan,
-// where that solve is of few scenarios; else once as many such solves have gone
-// without them as have lost about what compiling takes (ms, against what a solve
-// loses: 118 buses FP64 1.7 / .5, 300 3.7 / .4, 2,000 FP64 69 / 1.9, 10,000 360 / 2.5,
-// 20,000 760 / 5.7, on one thread).  While a clone compiles them, solves go on
-// without.
+// are compiled beside the plan of a topology's first solve, of whatever size (that
+// solve takes as long with them; compiled in a later one they were 1.7 ms among
+// solves of 1 ms, 118 buses FP64; 69 / 3.8, 2,000 FP64; 360 / 5, 10,000; 750 / 10, 20,000).
+// A variant, or a topology tuned in a call over many, compiles them once as many
+// small solves have gone without them as have lost about that.  While a clone
+// compiles them, solves go on without.
 static void ensure_solo(gox_topo* t, int i, int B) {
   if (!t->dot_main[i] || t->solo_loaded[i] || !t->uploaded || B > solo_most(t->sc, i == 0 ? 4 : 8)) return;
   {
     std::unique_lock<std::mutex> lk(t->solo[i]->mu, std::try_to_lock);
     if (!lk) return;
     if (!t->solo[i]->tried) {
-      // (a variant, one of many of a Q-limit or island solve, only when used often)
       const int wait = std::min(2 + t->sc.n_slots / 2500, 64);
       if (++t->small_solves[i] < (t->tune_cache_only ? std::max(16, wait) : wait)) return;
       make_solos(t->sc, i == 0 ? 4 : 8, *t->solo[i]);
@@ -1628,7 +1627,7 @@ static void ensure_solo(gox_topo* t, int i, int B) {
   load_solos(t, i);
 }
 
-// (solos: the solve may run solo programs)
+// (solos: the call is one that solo programs may run)
 template <typename T>
 static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st, bool solos) {
   const int i = sizeof(T) == 4 ? 0 : 1;
@@ -1639,7 +1638,6 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st, bool solos
   const bool fits = dot_fits(sc);
   const int elem = (int)sizeof(T);
   const std::array<int, 4> key = tune_key(t, i, D.G);
-  solos = solos && D.nb > 0 && D.nb <= solo_most(sc, elem);
   auto build_solos = [&] {
     std::unique_lock<std::mutex> lk(t->solo[i]->mu, std::try_to_lock);
     if (lk && !t->solo[i]->tried) make_solos(sc, elem, *t->solo[i]);
@@ -1823,7 +1821,7 @@ static void autotune(gox_topo* t, const BatchDev& D, cudaStream_t st, bool solos
     const std::shared_ptr<const DotProgram> p = dbuilt[best - (int)cand.size()];
     entry = {p->plan.top_warps, kDotChunkWords, p->plan.mid, p->plan.bins};
     install_dot(t, i, p, D.G, dbuilt.back());
-    if (solos) load_solos(t, i);
+    if (solos && D.nb > 0 && D.nb <= solo_most(sc, elem)) load_solos(t, i);
   } else {
     const StreamPlan& p = cand[best];
     entry = {p.nw, p.chunk_words, p.sync, p.wide_levels > 0 ? p.wide_min : 0};
