@@ -35,9 +35,8 @@ struct Writer {
     idle = 0;
   }
   // a sum's products [0, n) as units of up to 8
-  int sum(uint32_t op, uint32_t y, uint32_t z, const int32_t* a, const int32_t* b, int n) {
+  void sum(uint32_t op, uint32_t y, uint32_t z, const int32_t* a, const int32_t* b, int n) {
     flush();
-    int units = 0;
     bool cin = false;
     do {
       const int m = std::min(n, kDotTerms);
@@ -53,9 +52,7 @@ struct Writer {
       b += m;
       n -= m;
       cin = true;
-      units++;
     } while (n > 0);
-    return units;
   }
   // four sums of m products each (the last ones repeated to make four: the
   // same sum twice stores the same value twice)
@@ -238,14 +235,11 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
       mid.push_back(std::move(m));
     }
   }
-  for (int k = 0; k < n; k++) {
-    P.bottom_cols += stage[k] == 0;
-    P.mid_cols += stage[k] == 1;
-  }
+  const int bottom_cols = (int)std::count(stage.begin(), stage.end(), 0);
   auto emit_sum = [&](Writer& W, uint32_t op, int v, uint32_t z, int t0, int t1) {
     const bool y = v >= ns;
-    P.units += W.sum(op | (y && t0 == S.ptr[v] ? DOT_FIRST : 0u), (uint32_t)(y ? v - ns : v), z, S.a.data() + t0,
-                     S.b.data() + t0, t1 - t0);
+    W.sum(op | (y && t0 == S.ptr[v] ? DOT_FIRST : 0u), (uint32_t)(y ? v - ns : v), z, S.a.data() + t0,
+          S.b.data() + t0, t1 - t0);
   };
   // independent sums of one warp (products [t0, t1) of value v): the short ones
   // by fours, those of one length together, the long ones one by one
@@ -263,12 +257,8 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
         const auto& l = by[kind][m];
         for (size_t i = 0; i < l.size(); i += 4) {
           const int cnt = (int)std::min<size_t>(4, l.size() - i);
-          if (cnt == 1) {
-            emit_sum(W, kind ? DOT_Y : DOT_U, l[i].v, 0, l[i].t0, l[i].t0 + m);
-          } else {
-            W.pack(S, &l[i], cnt, m, kind > 0, kind == 2, ns);
-            P.units++;
-          }
+          if (cnt == 1) emit_sum(W, kind ? DOT_Y : DOT_U, l[i].v, 0, l[i].t0, l[i].t0 + m);
+          else W.pack(S, &l[i], cnt, m, kind > 0, kind == 2, ns);
         }
       }
   };
@@ -312,20 +302,17 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
       Writer W;
       for (size_t d = 0; d < at.size(); d++) {
         emit_group(W, at[d]);
-        for (int k : fins[d]) {
-          W.fin(sc.diag_slot[k], sc.c_llen[k]);
-          P.units++;
-        }
+        for (int k : fins[d]) W.fin(sc.diag_slot[k], sc.c_llen[k]);
       }
       append(P, P.bottom, W);
     }
   }
   // ---- prep: per later column, the leading products of each sum whose values
   // the bottom (or the prep of this same column) finishes
-  if (P.bottom_cols > 0) {
+  if (bottom_cols > 0) {
     std::vector<int32_t> prep_depth(ns + n, 0);
     std::vector<std::vector<Part>> at;  // the stream's sums, by depth among its columns' U entries
-    int left_cols = n - (int)P.bottom_cols, in_stream = 0;
+    int left_cols = n - bottom_cols, in_stream = 0;
     // (two columns fill the packs better; four leave too few warps in flight:
     // 2,000 buses, 256 bins, 128 groups FP32 0.305 / 0.276 / 0.285 ms for 1 / 2 / 4)
     const int per_stream = left_cols >= 256 ? 2 : 1;
@@ -344,7 +331,6 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
         at[d].push_back({v, S.ptr[v], t});
         prep_depth[v] = d + 1;
         taken[v] = t - S.ptr[v];
-        P.prep_terms += taken[v];
       };
       for (int d = 0; d < len(k); d++) prefix(base + d);
       if (subst) prefix(ns + k);
@@ -427,7 +413,6 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
       prev = add_node({0, v, t, q, r, 0, sum_cost(q - t)});
       prev_tick = r;
       t = q;
-      P.parts++;
     }
     from[v] = t;
     return prev;
@@ -493,7 +478,6 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
     std::vector<std::vector<double>>& load_of = out.load;
     int tick = 0;
     auto emit = [&](int w, uint32_t op, int v, uint32_t z, int t0, int t1) {
-      P.top_terms += t1 - t0;
       plan_of.back().push_back({w, op, v, z, t0, t1});
     };
 
@@ -594,8 +578,8 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
     return out;
   };
   auto row = [&](Writer& w, int k) {
-    P.units += w.sum(DOT_B, (uint32_t)k, (uint32_t)sc.diag_slot[k], sc.bw_slot.data() + sc.bw_ptr[k],
-                     sc.bw_col.data() + sc.bw_ptr[k], sc.bw_ptr[k + 1] - sc.bw_ptr[k]);
+    w.sum(DOT_B, (uint32_t)k, (uint32_t)sc.diag_slot[k], sc.bw_slot.data() + sc.bw_ptr[k],
+          sc.bw_col.data() + sc.bw_ptr[k], sc.bw_ptr[k + 1] - sc.bw_ptr[k]);
   };
   // ---- a CTA's backward rows, level by level
   std::vector<int32_t> lev(n, 0);
@@ -717,7 +701,6 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
           for (size_t q = i; q < std::min(need.size(), i + 12); q++)
             (need[q] >= ns ? touch[at][w].second : touch[at][w].first).push_back(need[q] >= ns ? need[q] - ns : need[q]);
           load[w] += 60.0 + 8.0 * 12;
-          P.touched += std::min<size_t>(12, need.size() - i);
         }
       }
     }
@@ -739,10 +722,7 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
       }
       for (int w = 0; w < NT; w++) emit_group(W[w], group[w]);
       for (const Do& d : plan_of[t])
-        if (d.op == DOT_FIN) {
-          W[d.w].fin(sc.diag_slot[d.v], sc.c_llen[d.v]);
-          P.units++;
-        }
+        if (d.op == DOT_FIN) W[d.w].fin(sc.diag_slot[d.v], sc.c_llen[d.v]);
       if (!touch[t].empty())
         for (int w = 0; w < NT; w++) {
           auto& x = touch[t][w];
@@ -778,7 +758,6 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
             if (stage[S.col[a]] > 1 || (v >= ns ? stage[b] > 1 : stop[b] < S.ptr[b + 1])) break;
           }
           any |= stop[v] > t0;
-          P.prep_terms += stop[v] - t0;
         };
         for (int d = 0; d < len(k); d++) prefix(base + d);
         if (subst) prefix(ns + k);
@@ -789,17 +768,9 @@ void build_dot(const Schedule& sc, const DotPlan& plan, DotProgram& P) {
       }
       if (!cols.empty()) streams(schedule(cols, true), NT, P.prep2);
     }
-  {
-    Ticks t = schedule(top, false);
-    P.ticks = (int)t.plan.size();
-    streams(std::move(t), NT, P.top);
-  }
+  streams(schedule(top, false), NT, P.top);
   if (!subst) return;
-  {
-    Ticks t = backward(top);
-    P.back_ticks = (int)t.plan.size();
-    streams(std::move(t), kDotBackWarps, P.tback);
-  }
+  streams(backward(top), kDotBackWarps, P.tback);
   for (auto& m : mid) streams(backward(m), kDotBackWarps, P.midback);
   for (int b = 0; b < plan.bins; b++) {
     if (bin[b].empty()) continue;

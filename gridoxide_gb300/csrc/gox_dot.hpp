@@ -89,8 +89,6 @@ struct DotProgram {
   std::vector<uint32_t> words;                   // all streams, 4 words per quad
   std::vector<int32_t> bottom, prep, mid, prep2, top, tback, midback, back;  // per bin / warp: first quad of its stream
   bool with_subst = false;                       // forward and backward substitution included
-  int ticks = 0, back_ticks = 0;
-  int64_t units = 0, parts = 0, bottom_cols = 0, mid_cols = 0, top_terms = 0, prep_terms = 0, touched = 0;
 };
 
 // Programs address a group's values by 32-bit byte offsets: a matrix with more

@@ -515,7 +515,6 @@ static bool build_solo(const Schedule& sc, const Sums& S, const SoloPlan& plan, 
             word(l, 11) = f;
             if (l >= (int)v->lane.size()) continue;
             const Lane& s = v->lane[l];
-            P.lanes++;
             word(l, 0) = off(div ? ns + s.v : s.v);
             if (last)
               word(l, 9) = (s.info & ~SOLO_SRC) |
@@ -526,10 +525,8 @@ static bool build_solo(const Schedule& sc, const Sums& S, const SoloPlan& plan, 
               if (e >= s.t1) break;
               word(l, 1 + 2 * i) = off(div ? sc.bw_slot[e] : S.a[e]);
               word(l, 2 + 2 * i) = off(div ? ns + sc.bw_col[e] : second(s.v, e));
-              P.products++;
             }
           }
-          P.units++;
         }
       }
       if (t + 1 < ticks.size())
@@ -583,7 +580,6 @@ static bool build_solo(const Schedule& sc, const Sums& S, const SoloPlan& plan, 
     Ticks t = forward(top, false);
     const size_t back = t.size();
     backward(top, t);
-    P.ticks = (int)t.size();
     streams(t, back, 2);
   }
   for (auto& m : mid) {

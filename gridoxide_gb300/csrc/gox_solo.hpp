@@ -84,8 +84,6 @@ struct SoloProgram {
   // with its backward rows, the parts' backward rows
   std::vector<SoloCta> launch[4];
   int max_values[4] = {0, 0, 0, 0};  // of a CTA, the zero included
-  int ticks = 0;
-  int64_t units = 0, lanes = 0, products = 0;
   int ctas() const { return std::max<int>(1, (int)launch[0].size()); }
 };
 
