@@ -96,8 +96,13 @@ bool build_solo_default(const Schedule& sc, int elem, bool wide, SoloProgram& ou
 // Scenarios that a program of the schedule could run at most, by the sizes alone
 // (more: none is compiled for them).
 int solo_most(const Schedule& sc, int elem);
-// Scenarios whose CTAs find a place on the chip at once, with `depth` units of a
-// warp in shared memory (0: its values leave no room for them).
+// Scenarios whose CTAs find a place on the chip at once by their shared memory,
+// with `depth` units of a warp in it (0: its values leave no room for them).
+// Registers are not counted: of k_solo_newton's CTAs (64 a thread) four fit on an SM,
+// of k_solo's (40, FP64 47) six and five, so that of a grid of up to 60 buses more
+// are let in than run at once.  They are still faster than the dot program (ms,
+// 640 to 760 scenarios here / 800 there: 20 buses mixed .374 / .465, FP64 .48 / .53;
+// 700 / 1,000: 50 buses .49 / .55, .66 / .68).
 int solo_scenarios(const SoloProgram& p, int depth);
 
 // Host interpreter for one scenario in FP64, with the checks of run_dot_host:

@@ -391,7 +391,8 @@ class Topology:
         p/q/vm_out/va_out float64 [B, N]; vm0/va0 float64 [N] or [B, N];
         iters/status int32 [B]; max_mis float64 [B]; outage = (slots int32
         [B,4], dre, dim float64 [B,4]) or None; history float64 [B, max_iter]
-        or None.  Work is enqueued on `stream` (a torch.cuda.Stream or None)."""
+        or None.  The work is in the order of `stream` (a torch.cuda.Stream or
+        None, the default stream)."""
         L = _lib.load()
         B, n = p_spec.shape
         stride = n if vm0.dim() == 2 else 0

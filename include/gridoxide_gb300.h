@@ -153,10 +153,15 @@ int gox_batch_solve(gox_topo *t, int32_t B, const double *p_spec, const double *
                     double *va_out, int32_t *iterations, int32_t *status, double *max_mismatch,
                     double *history);
 
-/* As gox_batch_solve, with every array in device memory and the work
- * enqueued on `stream` (a cudaStream_t, NULL = legacy default stream).
- * Synchronizes with the stream once per Newton iteration to read the
- * running-scenario count. */
+/* As gox_batch_solve, with every array in device memory and the work in the
+ * order of `stream` (a cudaStream_t, NULL = legacy default stream): after what
+ * the stream holds, before what is enqueued on it later.  Batches of more than
+ * 2,016 scenarios on the legacy default stream run on a stream of the calling
+ * thread, between an event of the caller's stream and one that it waits for.
+ * The call waits for the Newton loop: once per iteration to read the
+ * running-scenario count, or once where the loop is one launch (a captured
+ * loop; few scenarios of a small grid).  The outputs may still be being written
+ * when it returns. */
 int gox_batch_solve_device(gox_topo *t, int32_t B, const double *p_spec, const double *q_spec,
                            const double *vm0, const double *va0, int32_t v_stride,
                            const int32_t *out_slot, const double *out_dre,
@@ -460,7 +465,8 @@ int gox_topo_set_zip(gox_topo *t, const double *zi_re, const double *zi_im, cons
                      const double *zc_im);
 
 /* Newton loop as a captured CUDA graph (default on): from the second solve
- * of a configuration (same batch buffers, precision, budget, outage use)
+ * of a configuration (same groups of 32 scenarios, batch buffers, precision,
+ * budget, outage use)
  * the whole loop is one graph launch with conditional while / if nodes and
  * the iteration on the device, instead of host-driven launches with one
  * synchronization per iteration; results are the same bit for bit.  Only

@@ -61,6 +61,7 @@ int main() {
 def test_interpreters_refuse_a_read_past_the_words(gox, tmp_path):
     from gridoxide_gb300 import build as gb
     objs = []
+    os.makedirs(gb.OBJ, exist_ok=True)
     for s in ("gox_symbolic.cpp", "gox_engine.cpp", "gox_dot.cpp", "gox_solo.cpp"):
         o = os.path.join(gb.OBJ, s + ".o")
         objs.append(o if os.path.exists(o) else gb._compile(s, gb._nvcc(), []))

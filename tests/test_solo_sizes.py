@@ -66,6 +66,7 @@ def _pattern(path, n, seed):
 def test_solo_programs_only_where_they_run(gox, tmp_path):
     from gridoxide_gb300 import build as gb
     objs = []
+    os.makedirs(gb.OBJ, exist_ok=True)
     for s in ("gox_symbolic.cpp", "gox_engine.cpp", "gox_dot.cpp", "gox_solo.cpp"):
         o = os.path.join(gb.OBJ, s + ".o")
         objs.append(o if os.path.exists(o) else gb._compile(s, gb._nvcc(), []))
