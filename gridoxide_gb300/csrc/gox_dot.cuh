@@ -227,7 +227,7 @@ __device__ __forceinline__ void dot_run(const uint4* __restrict__ gs, uint4* win
   bool bad = false, tiny = false;
   T v = (T)0;
   gs += lane;
-  static_assert(kDotAhead == 2, "two chunks in shared memory and one in registers");
+  static_assert(kDotAhead >= 2, "two chunks in shared memory and one in registers");
   win[lane] = __ldg(gs);
   win[32 + lane] = __ldg(gs + 32);
   uint4 pre = __ldg(gs + 64);

@@ -68,7 +68,7 @@ constexpr int kDotBackWarps = 16;  // warps of the top's backward CTA
 // products of a chain's row (two rows in registers)
 constexpr int dot_chain_terms(int elem) { return elem == 4 ? 10 : 8; }
 constexpr int kDotChunk = 32;   // quads of a chunk: one 16-byte load per lane
-constexpr int kDotAhead = 2;    // chunks that are read past the one run (a stream ends in as many)
+constexpr int kDotAhead = 3;    // chunks that a stream ends in (two are read past the one run)
 constexpr int kDotMaxMid = 14;  // mid barriers of one tick (ids 1..14)
 
 struct DotPlan {
